@@ -17,10 +17,8 @@
 // SM are resident. Partials land in scratch and a small second kernel adds the K splits and applies the
 // epilogue (bias, residual, or SiLU(gate)*up).
 //
-// Prompt rows (M > 256) are cut into blocks of 128 on grid.z. Whenever one problem needs no K split, the epilogue warps
-// apply bias, post norm, residual and soft cap themselves and store the result: no partials, no second kernel. Gate and up
-// projections without a K split are paired: a weight tile is 64 gate rows over 64 up rows, and the epilogue warps that
-// hold the up half hand it to the others through shared memory, which store act(gate) * up.
+// Whenever one problem needs no K split, the epilogue warps apply bias, post norm, residual and soft cap themselves and store
+// the result: no partials, no second kernel. More than 128 rows go to the CTA-pair kernel (gemm_tc_pair.cu).
 //
 // Every wait is bounded: a wait that runs out sets bit 2 of the context's device status word, the
 // CTA stops issuing work, frees its TMEM and returns.
@@ -28,11 +26,18 @@
 
 #include "common.cuh"
 #include "gemm_tc.cuh"
+#include "gemm_tc_pair.cuh"
 #include "tc_ptx.cuh"
 
 namespace {
 
 using namespace tc;
+
+// From here on a tile of gemm_tc_f16_kernel cannot stack the hi and lo rows in one MMA, and the CTA-pair kernel is faster
+// (111 against 155 + 21 us with the epilogue kernel at 2 x 14336 x 4096 gate | up weights and 256 rows, 638 against
+// 1005 us at 2048 rows). At 128 rows it is
+// slower: 42 + 7 against 35 + 9 us at 4096 x 14336, 21 + 7 against 18 + 8 at 4096 x 4096.
+constexpr uint32_t PAIR_MIN_ROWS = 129;
 
 struct TcArgs {
     float* partial;            // [k_splits][M][n_total]
@@ -42,14 +47,10 @@ struct TcArgs {
     uint32_t tile_begin[4];    // first tile of each problem, tile_begin[problems] = total
     uint32_t problems;
     uint32_t kblocks_per_split, kblocks_total;
-    uint32_t use_lo;           // 1: activations carry a lo part (second MMA)
     uint32_t stages;
-    uint32_t m_block;          // activation rows per grid.z block
     uint32_t fmt_bits;         // operand type bits of the instruction descriptor (0: f16, see idesc_bf16())
     // direct != 0: one problem, no K split; the result is finished and stored by the epilogue warps
     uint32_t direct, n_out;
-    uint32_t paired;  // direct gate|up: problems 0 and 1 share every tile, 64 rows each
-    int act;
     float* out;
     const float* bias;
     const float* residual;
@@ -68,11 +69,9 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_f16_kernel(const __grid_consta
     unsigned char* smem = smem_unaligned + ((1024u - (smem_u32(smem_unaligned) & 1023u)) & 1023u);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t tile = blockIdx.x, ksplit = blockIdx.y;
-    const uint32_t m_base = blockIdx.z * a.m_block;
-    const uint32_t m_live = min(a.m_block, a.M - m_base);
     const uint32_t a_bytes = BLOCK_N * BLOCK_K * 2;                 // 16 KB
     const uint32_t b_bytes = a.M_pad * BLOCK_K * 2;                 // per hi / lo part
-    const uint32_t stage_bytes = a_bytes + (a.use_lo ? 2u : 1u) * b_bytes;
+    const uint32_t stage_bytes = a_bytes + 2u * b_bytes;
     unsigned char* stage_base = smem;                                // stages * stage_bytes, 1024-aligned each
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + a.stages * stage_bytes);
     uint64_t* full = bars;
@@ -81,18 +80,17 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_f16_kernel(const __grid_consta
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * a.stages + 1);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
-    // hi and lo activation tiles are contiguous rows of one operand: up to M_pad = 128 a single MMA of width
-    // 2 * M_pad takes the weight tile against both (the weight operand passes the tensor core once); the two
-    // halves of the accumulator are added in the epilogue.
-    const bool stacked = a.use_lo && a.M_pad <= 128u;
-    const uint32_t acc_cols = stacked ? 2u * a.M_pad : a.M_pad;
+    // hi and lo activation tiles are contiguous rows of one operand: a single MMA of width 2 * M_pad takes the weight tile
+    // against both (the weight operand passes the tensor core once); the two halves of the accumulator are added in the
+    // epilogue.
+    const uint32_t acc_cols = 2u * a.M_pad;
     uint32_t tmem_cols = 32;
     while (tmem_cols < acc_cols) tmem_cols <<= 1;
 
     uint32_t problem = 0;
     while (problem + 1 < a.problems && tile >= a.tile_begin[problem + 1]) ++problem;
     const CUtensorMap* tmW = problem == 0 ? &tmW0 : (problem == 1 ? &tmW1 : &tmW2);
-    const uint32_t row0 = a.paired ? tile * (BLOCK_N / 2) : (tile - a.tile_begin[problem]) * BLOCK_N;
+    const uint32_t row0 = (tile - a.tile_begin[problem]) * BLOCK_N;
     const uint32_t kb0 = ksplit * a.kblocks_per_split;
     uint32_t kb1 = kb0 + a.kblocks_per_split;
     if (kb1 > a.kblocks_total) kb1 = a.kblocks_total;
@@ -122,15 +120,13 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_f16_kernel(const __grid_consta
             for (uint32_t i = 0; i < pre; ++i) {
                 mbar_expect_tx(&full[i], stage_bytes);
                 tma_load_2d(stage_base + i * stage_bytes, tmW, &full[i], (int)((kb0 + i) * BLOCK_K), (int)row0);
-                if (a.paired)
-                    tma_load_2d(stage_base + i * stage_bytes + a_bytes / 2, &tmW1, &full[i], (int)((kb0 + i) * BLOCK_K), (int)row0);
             }
             pdl_wait();
             for (uint32_t i = 0; i < pre; ++i) {
                 unsigned char* st = stage_base + i * stage_bytes;
                 const int kx = (int)((kb0 + i) * BLOCK_K);
-                tma_load_2d(st + a_bytes, &tmXh, &full[i], kx, (int)m_base);
-                if (a.use_lo) tma_load_2d(st + a_bytes + b_bytes, &tmXl, &full[i], kx, (int)m_base);
+                tma_load_2d(st + a_bytes, &tmXh, &full[i], kx, 0);
+                tma_load_2d(st + a_bytes + b_bytes, &tmXl, &full[i], kx, 0);
             }
             for (uint32_t i = pre; i < n_kb; ++i) {
                 const uint32_t s = i % a.stages, round = i / a.stages;
@@ -140,9 +136,8 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_f16_kernel(const __grid_consta
                 mbar_expect_tx(&full[s], stage_bytes);
                 const int kx = (int)((kb0 + i) * BLOCK_K);
                 tma_load_2d(st, tmW, &full[s], kx, (int)row0);
-                if (a.paired) tma_load_2d(st + a_bytes / 2, &tmW1, &full[s], kx, (int)row0);
-                tma_load_2d(st + a_bytes, &tmXh, &full[s], kx, (int)m_base);
-                if (a.use_lo) tma_load_2d(st + a_bytes + b_bytes, &tmXl, &full[s], kx, (int)m_base);
+                tma_load_2d(st + a_bytes, &tmXh, &full[s], kx, 0);
+                tma_load_2d(st + a_bytes + b_bytes, &tmXl, &full[s], kx, 0);
             }
         }
     } else if (warp == 1) {
@@ -160,7 +155,6 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_f16_kernel(const __grid_consta
                 for (uint32_t k = 0; k < BLOCK_K / UMMA_K; ++k) {
                     const uint64_t da = make_desc_sw128(sa + k * UMMA_K * 2);
                     umma_f16(tmem_base, da, make_desc_sw128(sb + k * UMMA_K * 2), idesc, (i | k) != 0u);
-                    if (a.use_lo && !stacked) umma_f16(tmem_base, da, make_desc_sw128(sb + b_bytes + k * UMMA_K * 2), idesc, 1u);
                 }
                 umma_commit(&empty[s]);  // frees the stage once these MMAs have read it
             }
@@ -177,37 +171,7 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_f16_kernel(const __grid_consta
         ok = __all_sync(0xffffffffu, ok);  // tcgen05.ld is warp-collective
         tc_fence_after();
         const uint32_t n_glob = tile * BLOCK_N + lane_group * 32 + lane;
-        if (a.paired) {
-            // lanes 0..63 of the accumulator hold gate rows, 64..127 the up rows of the same outputs; the ring is free
-            float* xs = reinterpret_cast<float*>(smem);  // [M_pad][64]
-            const uint32_t r = (lane_group & 1u) * 32u + lane;
-            const uint32_t n = tile * (BLOCK_N / 2) + r;
-            for (uint32_t half = 0; half < 2; ++half) {
-                if (half == 1) asm volatile("bar.sync 1, 128;" ::: "memory");
-                if ((lane_group >= 2u) != (half == 0)) continue;  // up warps first, then gate warps
-                for (uint32_t c = 0; c < a.M_pad; c += 8) {
-                    float v[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) v[j] = 0.0f;
-                    if (ok) {
-                        tmem_ld8(tmem_base + ((lane_group * 32u) << 16) + c, v);
-                        if (stacked) {
-                            float w[8];
-                            tmem_ld8(tmem_base + ((lane_group * 32u) << 16) + a.M_pad + c, w);
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) v[j] += w[j];
-                        }
-                    }
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        if (half == 0) xs[(c + j) * 64u + r] = v[j];
-                        else if (n < a.n_out && c + j < m_live)
-                            a.out[(size_t)(m_base + c + j) * a.n_out + n] = m40_act(a.act, v[j]) * xs[(c + j) * 64u + r];
-                    }
-                }
-            }
-        }
-        float* dst = a.partial + ((size_t)ksplit * a.M + m_base) * a.n_total + n_glob;
+        float* dst = a.partial + (size_t)ksplit * a.M * a.n_total + n_glob;
         const bool n_ok = n_glob < a.n_out;  // direct mode: one problem, so the padded column is the output column
         float bias = 0.0f, pw = 1.0f, pb = 0.0f;
         if (a.direct && n_ok) {
@@ -215,16 +179,14 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_f16_kernel(const __grid_consta
             if (a.post_w) pw = a.post_w[n_glob];
             if (a.post_b) pb = a.post_b[n_glob];
         }
-        for (uint32_t c = a.paired ? a.M_pad : 0u; c < a.M_pad; c += 8) {
+        for (uint32_t c = 0; c < a.M_pad; c += 8) {
             float v[8];
             if (ok) {
                 tmem_ld8(tmem_base + ((lane_group * 32u) << 16) + c, v);
-                if (stacked) {
-                    float w[8];
-                    tmem_ld8(tmem_base + ((lane_group * 32u) << 16) + a.M_pad + c, w);
+                float w[8];
+                tmem_ld8(tmem_base + ((lane_group * 32u) << 16) + a.M_pad + c, w);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) v[j] += w[j];
-                }
+                for (int j = 0; j < 8; ++j) v[j] += w[j];
             } else {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) v[j] = 0.0f;
@@ -233,18 +195,18 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_f16_kernel(const __grid_consta
                 float res[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {  // unconditional loads (clamped), so that the eight go out together
-                    const uint32_t m = m_base + min(c + j, m_live - 1u);
+                    const uint32_t m = min(c + j, a.M - 1u);
                     res[j] = a.residual ? a.residual[(size_t)m * a.n_out + (n_ok ? n_glob : 0u)] : 0.0f;
                 }
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    if (n_ok && c + j < m_live)
-                        a.out[(size_t)(m_base + c + j) * a.n_out + n_glob] = m40_tail(a.tail, v[j], bias, pw, pb, res[j]);
+                    if (n_ok && c + j < a.M)
+                        a.out[(size_t)(c + j) * a.n_out + n_glob] = m40_tail(a.tail, v[j], bias, pw, pb, res[j]);
                 continue;
             }
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-                if (c + j < m_live) dst[(size_t)(c + j) * a.n_total] = v[j];
+                if (c + j < a.M) dst[(size_t)(c + j) * a.n_total] = v[j];
         }
     }
     if (*abort_flag && threadIdx.x == 64) atomicOr(a.status, 4u);
@@ -606,38 +568,23 @@ int m40_gemm_tc_f16(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind
         for (int p = 0; p < 3; ++p)
             if (N[p] % 128 != 0 || N[p] % (int)rope->head_dim != 0) return -2;
     }
-    const uint32_t m_block = M > 256 ? 128u : (uint32_t)M;
-    const uint32_t m_blocks = ((uint32_t)M + m_block - 1) / m_block;
-    const uint32_t M_pad = (m_block + 15) / 16 * 16;
+    const uint32_t M_pad = ((uint32_t)M + 15) / 16 * 16;
     TcArgs a = {};
-    a.m_block = m_block;
     a.fmt_bits = bf16 ? idesc_bf16() : 0u;
     a.M = (uint32_t)M;
     a.M_pad = M_pad;
     a.K = (uint32_t)K;
     a.problems = (uint32_t)problems;
-    // hi-only f16 activations miss the parity tolerance for outputs near zero (error ~3e-4 * |x| * sqrt(K) * |w|),
-    // so the lo part is always carried; above ~128 rows this makes the kernel tensor-bound instead of HBM-bound.
-    a.use_lo = 1u;
     uint32_t tiles = 0;
-    // Gate|up of prompt rows in paired tiles when those alone fill the machine: no K split, and none of the M x 2N partials
-    // (up to 256 rows the separate tiles and their epilogue kernel measured faster).
-    a.paired = ext && mode == 1 && problems == 2 && N[0] == N[1] && M > 256 &&
-                       (uint32_t)((N[0] + BLOCK_N / 2 - 1) / (BLOCK_N / 2)) * m_blocks >= (uint32_t)ctx->sm_count
-                   ? 1u : 0u;
-    for (int p = 0; p < (a.paired ? 0 : problems); ++p) {
+    for (int p = 0; p < problems; ++p) {
         a.tile_begin[p] = tiles;
         tiles += (uint32_t)((N[p] + BLOCK_N - 1) / BLOCK_N);
     }
-    for (int p = a.paired ? 4 : problems; p < 4; ++p) a.tile_begin[p] = tiles;
-    if (a.paired) {
-        tiles = (uint32_t)((N[0] + BLOCK_N / 2 - 1) / (BLOCK_N / 2));
-        a.tile_begin[1] = a.tile_begin[2] = a.tile_begin[3] = tiles;
-    }
+    for (int p = problems; p < 4; ++p) a.tile_begin[p] = tiles;
     a.n_total = tiles * BLOCK_N;
     a.kblocks_total = (uint32_t)((K + BLOCK_K - 1) / BLOCK_K);
     // stages from the shared-memory budget; two CTAs per SM when the stage is small
-    const uint32_t stage_bytes = BLOCK_N * BLOCK_K * 2 + (a.use_lo ? 2u : 1u) * M_pad * BLOCK_K * 2;
+    const uint32_t stage_bytes = BLOCK_N * BLOCK_K * 2 + 2u * M_pad * BLOCK_K * 2;
     uint32_t stages = (100u * 1024u) / stage_bytes;
     if (stages > 8) stages = 8;
     if (stages < 2) stages = 2;
@@ -645,14 +592,25 @@ int m40_gemm_tc_f16(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind
     const size_t smem = (size_t)stages * stage_bytes + (2 * stages + 1) * 8 + 16 + 1024;
     const uint32_t ctas_per_sm = smem <= 110u * 1024u ? 2u : 1u;
     // K splits: fill about one wave of resident CTAs, keep at least 4 k-blocks per split
-    uint32_t ks = ((uint32_t)ctx->sm_count * ctas_per_sm) / (tiles * m_blocks);
-    if (ks < 1 || a.paired) ks = 1;
+    uint32_t ks = ((uint32_t)ctx->sm_count * ctas_per_sm) / tiles;
+    if (ks < 1) ks = 1;
     const uint32_t ks_max = a.kblocks_total / 4 ? a.kblocks_total / 4 : 1;
     if (ks > ks_max) ks = ks_max;
     if (ks > 16) ks = 16;
     a.kblocks_per_split = (a.kblocks_total + ks - 1) / ks;
     ks = (a.kblocks_total + a.kblocks_per_split - 1) / a.kblocks_per_split;
-    const bool direct = ext && ks == 1 && !rope && (a.paired || (problems == 1 && mode == 0));
+    // Many rows go to the CTA-pair kernel, which finishes the result itself unless K is split.
+    M40PairPlan plan = {};
+    const bool gate_up_pairs = mode == 1 && problems == 2 && N[0] == N[1];
+    const bool finishes = !rope && (gate_up_pairs || (problems == 1 && mode == 0));
+    const bool pairs = (uint32_t)M >= PAIR_MIN_ROWS;
+    if (pairs && !m40_pair_plan(ctx, (uint32_t)M, a.kblocks_total, (uint32_t)problems, N, gate_up_pairs, !finishes, &plan)) return -2;
+    if (pairs) {
+        ks = plan.k_splits;
+        a.n_total = plan.tiles * M40_PAIR_ROWS;
+        for (int p = 0; p < 4; ++p) a.tile_begin[p] = plan.tile_begin[p] * (M40_PAIR_ROWS / BLOCK_N);
+    }
+    const bool direct = pairs ? finishes && ks == 1 : ext && ks == 1 && !rope && problems == 1 && mode == 0;
 
     // scratch: [hi][lo] activation copies, then the partials
     const size_t act_elems = (size_t)M * K;
@@ -661,17 +619,19 @@ int m40_gemm_tc_f16(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind
     unsigned char* scratch = (unsigned char*)m40_ensure_scratch(ctx, stream_kind, 2 * act_bytes + part_bytes);
     if (!scratch) return -2;
     __half* xh = (__half*)scratch;
-    __half* xl = a.use_lo ? (__half*)(scratch + act_bytes) : nullptr;
+    __half* xl = (__half*)(scratch + act_bytes);
     a.partial = (float*)(scratch + 2 * act_bytes);
     a.status = ctx->d_status;
 
     CUtensorMap mW[3], mXh, mXl;
     for (int p = 0; p < 3; ++p) {
         const int q = p < problems ? p : 0;
-        if (!make_map_f16(&mW[p], W[q], (uint64_t)N[q], (uint64_t)K, a.paired ? BLOCK_N / 2 : BLOCK_N, bf16)) return -2;
+        const uint32_t w_box = pairs && gate_up_pairs ? BLOCK_N / 2 : BLOCK_N;
+        if (!make_map_f16(&mW[p], W[q], (uint64_t)N[q], (uint64_t)K, w_box, bf16)) return -2;
     }
-    if (!make_map_f16(&mXh, xh, (uint64_t)M, (uint64_t)K, M_pad, bf16)) return -2;
-    if (!make_map_f16(&mXl, a.use_lo ? xl : xh, (uint64_t)M, (uint64_t)K, M_pad, bf16)) return -2;
+    const uint32_t x_box = pairs ? plan.width / 2 : M_pad;
+    if (!make_map_f16(&mXh, xh, (uint64_t)M, (uint64_t)K, x_box, bf16)) return -2;
+    if (!make_map_f16(&mXl, xl, (uint64_t)M, (uint64_t)K, x_box, bf16)) return -2;
 
     if (ext) {
         SplitRowsArgs sa = {};
@@ -713,22 +673,44 @@ int m40_gemm_tc_f16(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind
         a.out = out[0];
         a.bias = bias ? bias[0] : nullptr;
         a.residual = residual ? residual[0] : nullptr;
-        a.post_w = ext->post_w;
-        a.post_b = ext->post_b;
-        a.act = ext->act;
+        a.post_w = ext ? ext->post_w : nullptr;
+        a.post_b = ext ? ext->post_b : nullptr;
     }
-    static unsigned long long configured = 0ull;
-    const unsigned long long bit = 1ull << (ctx->device_id & 63);
-    if (!(configured & bit)) {
-        if (cudaFuncSetAttribute(gemm_tc_f16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
-            return -2;
-        configured |= bit;
+    if (pairs) {
+        M40PairCall c = {};
+        for (int p = 0; p < 3; ++p) c.w[p] = mW[p];
+        c.xh = mXh;
+        c.xl = mXl;
+        c.M = (uint32_t)M;
+        c.kblocks = a.kblocks_total;
+        c.problems = (uint32_t)problems;
+        c.fmt_bits = a.fmt_bits;
+        c.paired = gate_up_pairs ? 1u : 0u;
+        c.partial = direct ? nullptr : a.partial;
+        c.out = a.out;
+        c.n_out = a.n_out;
+        c.bias = a.bias;
+        c.residual = a.residual;
+        c.post_w = a.post_w;
+        c.post_b = a.post_b;
+        c.act = ext ? ext->act : 0;
+        c.tail = a.tail;
+        if (m40_pair_launch(ctx, s, c, plan) != 0) return -2;
+        if (direct) return 0;
+    } else {
+        static unsigned long long configured = 0ull;
+        const unsigned long long bit = 1ull << (ctx->device_id & 63);
+        if (!(configured & bit)) {
+            if (cudaFuncSetAttribute(gemm_tc_f16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
+                return -2;
+            configured |= bit;
+        }
+        dim3 grid(tiles, ks);
+        m40_launch_dependent(gemm_tc_f16_kernel, grid, dim3(192), smem, s, mW[0], mW[1], mW[2], mXh, mXl, a);
+        M40_COUNT_LAUNCH(ctx);
+        if (cudaGetLastError() != cudaSuccess) return -2;
+        if (direct) return 0;
     }
-    dim3 grid(tiles, ks, m_blocks);
-    m40_launch_dependent(gemm_tc_f16_kernel, grid, dim3(192), smem, s, mW[0], mW[1], mW[2], mXh, mXl, a);
-    M40_COUNT_LAUNCH(ctx);
-    if (cudaGetLastError() != cudaSuccess) return -2;
-    if (direct) return 0;
 
     EpiArgs e = {};
     if (ext) {

@@ -86,6 +86,22 @@ def test_linear_gated(nat, rows, n, k, act, fn):
         close(got, fn(h @ w.T.astype(np.float64)) * (h @ w2.T.astype(np.float64)), 3e-6 if exact else 6e-5, f"exact={exact}")
 
 
+@pytest.mark.parametrize("rows", [129, 256, 257, 511, 1030])
+@pytest.mark.parametrize("n,k", [(255, 1000), (257, 64), (640, 2120)])
+@pytest.mark.parametrize("wdt", [N.DT_BF16, N.DT_F16])
+def test_linear_many_rows(nat, rows, n, k, wdt):
+    """Edges of the 256 x 256 tiles and of the partial sums over K. Activations keep 2^-17 (bf16 hi + lo) or 2^-22 (f16) of
+    their value; outputs are near 1, the largest of them near 5."""
+    rng = np.random.default_rng(rows + n)
+    x, w, w2 = rng.standard_normal((rows, k)).astype(np.float32), rounded(rng, wdt, n, k), rounded(rng, wdt, n, k)
+    bias, res = rng.standard_normal(n), rng.standard_normal((rows, n))
+    tol = 8e-6 if wdt == N.DT_BF16 else 2e-6
+    y = x.astype(np.float64) @ w.T.astype(np.float64)
+    close(run_linear(nat, x, w, wdt, rows, bias=bias, residual=res), y + bias + res, tol, "plain")
+    close(run_linear(nat, x, w, wdt, rows, w2=w2, act=N.ACT_GELU_ERF), S.gelu_erf(y) * (x.astype(np.float64) @ w2.T.astype(np.float64)),
+          2 * tol, "gated")
+
+
 @pytest.mark.parametrize("rows", [1, 5, 64, 300])
 def test_linear_row_pitch(nat, rows):
     rng = np.random.default_rng(rows)
