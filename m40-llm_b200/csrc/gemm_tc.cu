@@ -141,24 +141,23 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_f16_kernel(const __grid_consta
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc = make_idesc(acc_cols) | a.fmt_bits;
-            bool ok = true;
-            for (uint32_t i = 0; i < n_kb && ok; ++i) {
-                const uint32_t s = i % a.stages, round = i / a.stages;
-                if (!mbar_wait(&full[s], round & 1u)) { *abort_flag = 1; ok = false; break; }
-                tc_fence_after();
-                const uint32_t sa = smem_u32(stage_base + s * stage_bytes);
-                const uint32_t sb = sa + a_bytes;
+        // ---------------- MMA issuer: the warp walks the loop converged (see elect_one()), one lane issues
+        const uint32_t idesc = make_idesc(acc_cols) | a.fmt_bits;
+        uint32_t s = 0, phase = 0;
+        for (uint32_t i = 0; i < n_kb; ++i) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&full[s], phase))) { *abort_flag = 1; break; }
+            tc_fence_after();
+            const uint32_t sa = smem_u32(stage_base + s * stage_bytes);
+            const uint32_t sb = sa + a_bytes;
+            if (elect_one()) {
 #pragma unroll
-                for (uint32_t k = 0; k < BLOCK_K / UMMA_K; ++k) {
-                    const uint64_t da = make_desc_sw128(sa + k * UMMA_K * 2);
-                    umma_f16(tmem_base, da, make_desc_sw128(sb + k * UMMA_K * 2), idesc, (i | k) != 0u);
-                }
-                umma_commit(&empty[s]);  // frees the stage once these MMAs have read it
+                for (uint32_t k = 0; k < BLOCK_K / UMMA_K; ++k)
+                    umma_f16(tmem_base, make_desc_sw128(sa + k * UMMA_K * 2), make_desc_sw128(sb + k * UMMA_K * 2), idesc, i | k);
+                umma_commit(&empty[s]);                 // frees the stage once these MMAs have read it
+                if (i + 1 == n_kb) umma_commit(accum);  // accumulator complete
             }
-            if (ok) umma_commit(accum);  // accumulator complete
+            __syncwarp();
+            if (++s == a.stages) s = 0, phase ^= 1u;
         }
     } else {
         // ---------------- epilogue: warps 2..5 own TMEM lanes 32*(warp % 4) .. +31

@@ -130,20 +130,22 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_grouped_kernel(const __grid_co
                     mbar_wait(&full[i % a.stages], (i / a.stages) & 1u);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = make_idesc(acc_cols) | a.fmt_bits;
-            bool ok = true;
-            for (uint32_t i = 0; i < a.kblocks && ok; ++i) {
-                const uint32_t s = i % a.stages;
-                if (!mbar_wait(&full[s], (i / a.stages) & 1u)) { *abort_flag = 1; ok = false; break; }
-                tc_fence_after();
-                const uint32_t sa = smem_u32(smem + s * stage_bytes), sb = sa + a_bytes;
+        // the warp walks the loop converged (see elect_one()), one lane issues
+        const uint32_t idesc = make_idesc(acc_cols) | a.fmt_bits;
+        uint32_t s = 0, phase = 0;
+        for (uint32_t i = 0; i < a.kblocks; ++i) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&full[s], phase))) { *abort_flag = 1; break; }
+            tc_fence_after();
+            const uint32_t sa = smem_u32(smem + s * stage_bytes), sb = sa + a_bytes;
+            if (elect_one()) {
 #pragma unroll
                 for (uint32_t k = 0; k < BLOCK_K / UMMA_K; ++k)
-                    umma_f16(tmem_base, make_desc_sw128(sa + k * UMMA_K * 2), make_desc_sw128(sb + k * UMMA_K * 2), idesc, (i | k) != 0u);
+                    umma_f16(tmem_base, make_desc_sw128(sa + k * UMMA_K * 2), make_desc_sw128(sb + k * UMMA_K * 2), idesc, i | k);
                 umma_commit(&empty[s]);
+                if (i + 1 == a.kblocks) umma_commit(accum);
             }
-            if (ok) umma_commit(accum);
+            __syncwarp();
+            if (++s == a.stages) s = 0, phase ^= 1u;
         }
     } else {
         const uint32_t lane_group = warp & 3u, row_of_tile = lane_group * 32u + lane;  // weight row of the tile

@@ -147,7 +147,9 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t ran
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
     return r;
 }
-// True in one lane of a converged warp.
+// True in one lane of a converged warp. The loop of an MMA-issuing warp is walked by all lanes and one elected lane issues: with
+// the whole loop inside "lane == 0" the operands of every tcgen05.mma are moved from per-thread to uniform registers again
+// (1357 against 1050 cycles per eight instructions of 128 cycles each in gemm_tc_pair.cu).
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
