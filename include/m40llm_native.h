@@ -571,6 +571,12 @@ typedef struct {
     const uint32_t* seg_host; /* the same on the host, or null: calls that would pick a form per segment then take one for all */
 } M40llmStepRows;
 
+/* Causal attention of a step's rows over a dense f16 cache (head size 64 or 128) that already holds their keys and values: q and
+ * out f32 [rows][q_heads][head_dim], softmax scaled by 1/sqrt(head_dim). For portions of prompts: a segment's rows share every
+ * read of the cache. Returns 1 for a cache it does not take, -1 / -2 for bad arguments. Decode stream. */
+int m40llm_attention_step_rows_async(M40llmCudaContext* ctx, const M40llmKVCache* kv, const void* d_q_f32, uint32_t q_heads,
+                                     const M40llmStepRows* rows, void* d_out_f32);
+
 /* Dense cache with separate key and value sizes and f16 or f32 elements; v_dim 0 keeps one array only (latents, for
  * m40llm_attention_latent_async). f16 with k_dim == v_dim is exactly m40llm_kvcache_create; any other combination with
  * values is served by m40llm_attention_rotary_async only (the entry points above

@@ -301,6 +301,35 @@ int m40_attention_prefill(M40llmCudaContext* ctx, const M40PrefillCall& c) {
 
 extern "C" {
 
+int m40llm_attention_step_rows_async(M40llmCudaContext* ctx, const M40llmKVCache* kv, const void* d_q_f32, uint32_t q_heads,
+                                     const M40llmStepRows* rows, void* d_out_f32) {
+    if (!ctx || !kv || !d_q_f32 || !rows || !rows->seg || !d_out_f32) return -1;
+    if (rows->rows == 0 || rows->segments == 0 || rows->max_segment_rows == 0 || q_heads == 0 || kv->num_heads == 0 ||
+        q_heads % kv->num_heads != 0)
+        return -2;
+    if (kv->compressed || !kv->d_k || !kv->d_v) return 1;
+    if (m40_ensure_device(ctx) != 0) return -1;
+    M40PrefillCall p = {};
+    p.K = kv->d_k;
+    p.V = kv->d_v;
+    p.q = (const float*)d_q_f32;
+    p.out = (float*)d_out_f32;
+    p.seg = rows->seg;
+    p.segments = rows->segments;
+    p.max_segment_rows = rows->max_segment_rows;
+    p.rows = rows->rows;
+    p.hd = p.q_dim = p.v_dim = kv->head_dim;
+    p.q_heads = q_heads;
+    p.kv_heads = kv->num_heads;
+    p.q_ld = p.out_ld = q_heads * kv->head_dim;
+    p.slot_mul = rows->slot_mul;
+    p.slot_add = rows->slot_add;
+    p.slots = kv->max_batch_size;
+    p.max_seq_len = kv->max_seq_len;
+    p.scale = attn_inv_sqrt(kv->head_dim);
+    return m40_attention_prefill(ctx, p);
+}
+
 int m40llm_attention_prefill_f32_gqa_varlen_async(M40llmCudaContext* ctx, const void* d_q_f32, const void* d_k_f32,
                                                   const void* d_v_f32, const uint32_t* d_q_offsets,
                                                   const uint32_t* d_kv_offsets, const uint32_t* d_q_lens,

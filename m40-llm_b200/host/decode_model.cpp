@@ -17,7 +17,7 @@ DecodeModel::DecodeModel(M40llmCudaContext* ctx, const ModelConfig& cfg, const s
     // the caller owns the cache; the store is only the table of sequences
     store_.reset(new SequenceStore(ctx, sequences, 0xffffffffu, M40LLM_DT_F16));
     for (size_t l = 0; l < layers.size(); ++l)
-        layers_.emplace_back(new LlamaLayer(cfg, layers[l], kv, (uint32_t)l));
+        layers_.emplace_back(new LlamaLayer(cfg, layers[l], kv, (uint32_t)l, (uint32_t)layers.size()));
     flat_layers_ = (uint32_t)layers.size();
     ok_ = allocate() == 0;
 }

@@ -62,8 +62,8 @@ protected:
 
 class LlamaLayer : public ModelLayer {
 public:
-    LlamaLayer(const ModelConfig& cfg, const LayerWeights& w, M40llmKVCache* kv, uint32_t index)
-        : cfg_(cfg), w_(w), kv_(kv), index_(index) {}
+    LlamaLayer(const ModelConfig& cfg, const LayerWeights& w, M40llmKVCache* kv, uint32_t index, uint32_t layers)
+        : cfg_(cfg), w_(w), kv_(kv), index_(index), layers_(layers) {}
     BufferNeeds needs() const override;
     int enqueue(M40llmCudaContext* ctx, const StepBatch& batch, StepBuffers& b) override;
 
@@ -71,7 +71,7 @@ private:
     ModelConfig cfg_;
     LayerWeights w_;
     M40llmKVCache* kv_;
-    uint32_t index_;
+    uint32_t index_, layers_;  // slot of (sequence, layer) = sequence * layers + index
 };
 
 enum class MixerKind : uint32_t { RotaryAttention = 1, DeltaRule = 2, LatentAttention = 3, RgLru = 4 };

@@ -74,6 +74,37 @@ def test_greedy_decode_matches_oracle(nat, O, pkg, H, qh, kvh, hd, F, q80, n_lay
     nat.free_all()
 
 
+@pytest.mark.parametrize("hd,parts", [(64, [(70, 16), (65, 17)]), (128, [(33, 100)]), (64, [(40, 1), (20, 64)]), (32, [(20, 30)])])
+def test_prompt_portions_match_single_tokens(nat, O, pkg, hd, parts):
+    """Prompts in portions (a segment of 16 rows or more takes the prompt attention, a lone row keeps all on the decode form) give
+    the logits of the same tokens one by one; both round probabilities to f16 (relative 2^-11 a token) and share the cache."""
+    rng = np.random.default_rng(hd + len(parts))
+    H, qh, kvh, F, n_layers, vocab = 256, 8, 2, 512, 2, 500
+    layers = [make_weights(O, rng, H, qh, kvh, hd, F, False, False) for _ in range(n_layers)]
+    emb = (rng.standard_normal((vocab, H)) * 0.5).astype(np.float16)
+    lm = (rng.standard_normal((vocab, H)) * 0.02).astype(np.float16)
+    out_norm = (1 + 0.05 * rng.standard_normal(H)).astype(np.float32)
+    host, seqs = pkg.host, len(parts)
+    kv = nat.kv_dense(200, 2 * seqs * n_layers, kvh, hd)
+    head = host.ModelHead(nat.buf(emb).ptr, nat.buf(out_norm).ptr, nat.buf(lm).ptr, vocab)
+    model = host.DecodeModel(nat.ctx, host.LayerCfg(H, qh, kvh, hd, F, 0, 1e-5, 1e4, 1.0), [_host_weights(pkg, nat, w, False) for w in layers],
+                             head, kv, 2 * seqs, max_rows=160)
+    tokens = [rng.integers(0, vocab, sum(p)).astype(np.uint32) for p in parts]
+    at = [0] * seqs
+    a, b = [model.acquire() for _ in parts], [model.acquire() for _ in parts]
+    for step in range(2):
+        entries = [(a[i], tokens[i][at[i]:at[i] + p[step]]) for i, p in enumerate(parts)]
+        at = [x + p[step] for x, p in zip(at, parts)]
+        got = model.step(entries, np.cumsum([p[step] for p in parts]) - 1)["logits"]
+    for i, t in enumerate(tokens):
+        for k, tok in enumerate(t):
+            last = model.step([(b[i], [tok])], [0] if k + 1 == len(t) else [], want_logits=k + 1 == len(t))["logits"]
+        assert_close(got[i], last[0], what=f"sequence {i}")
+    model.close()
+    nat.lib.m40llm_kvcache_destroy(kv)
+    nat.free_all()
+
+
 def test_argmax_and_embedding_rules(nat):
     L = nat.lib
     x = np.array([[1.0, 5.0, 5.0, np.nan, -np.inf], [np.nan, np.nan, np.nan, np.nan, np.nan],
