@@ -12,10 +12,13 @@
 // accumulation (q split into f16 hi + lo so that the scores keep f32-level accuracy, P rounded to f16), and the
 // softmax is online, base 2, in registers. Every kv row is read once per 64 q rows instead of once per q row.
 //
+// Segments of more than 64 rows take the tcgen05 kernel of attention_prefill_tc.cu where alignment allows; this one serves the rest.
+//
 // The same kernel also reads K and V straight from a dense f16 cache (CACHE): a prompt portion whose rows are already
 // appended attends everything its sequence holds, and the output may be turned back and gated before it is stored.
 #include "attention.cuh"
 #include "attention_mma.cuh"
+#include "attention_prefill_tc.cuh"
 #include "common.cuh"
 #include "stack_math.cuh"
 
@@ -285,6 +288,11 @@ int m40_attention_prefill(M40llmCudaContext* ctx, const M40PrefillCall& c) {
     if ((c.hd != 64 && c.hd != 128) || !c.K || !c.V || !c.seg) return 1;
     if (c.q_dim > c.hd || c.v_dim > c.hd || ((c.q_dim | c.v_dim | c.q_ld | c.out_ld) & 1u)) return 1;
     if ((((uintptr_t)c.q) & 7u) != 0u || (((uintptr_t)c.out) & 7u) != 0u) return 1;
+    M40PrefillTcArgs ta = {};
+    ta.c = c;
+    ta.status = ctx->d_status;
+    const int rc = m40_attention_prefill_tc(ctx, ctx->decode_stream, ta, (uint64_t)c.slots * c.kv_heads * c.max_seq_len);
+    if (rc <= 0) return rc;
     if (!prefill_configure(ctx->device_id)) return -4;
     const PrefillCache pc = {c, ctx->d_status};
     const dim3 grid((c.max_segment_rows + PF_TILE - 1) / PF_TILE, c.q_heads, c.segments);
@@ -378,8 +386,27 @@ int m40llm_attention_prefill_f32_gqa_varlen_async(M40llmCudaContext* ctx, const 
         prefill_pack_kv_kernel<<<blocks ? blocks : 1u, 256, 0, s>>>((const float*)d_k_f32, (const float*)d_v_f32, kh, vh, n8);
         M40_COUNT_LAUNCH(ctx);
     }
-    dim3 grid((max_q + PF_TILE - 1) / PF_TILE, q_heads, batch_size);
     const float inv_sqrt = attn_inv_sqrt(head_dim);
+    M40PrefillTcArgs ta = {};
+    ta.c.K = kh;
+    ta.c.V = vh;
+    ta.c.q = (const float*)d_q_f32;
+    ta.c.out = (float*)d_out_f32;
+    ta.c.segments = batch_size;
+    ta.c.max_segment_rows = max_q;
+    ta.c.hd = ta.c.q_dim = ta.c.v_dim = head_dim;
+    ta.c.q_heads = q_heads;
+    ta.c.kv_heads = kv_heads;
+    ta.c.q_ld = ta.c.out_ld = q_heads * head_dim;
+    ta.c.scale = inv_sqrt;
+    ta.q_offsets = d_q_offsets;
+    ta.kv_offsets = d_kv_offsets;
+    ta.q_lens = d_q_lens;
+    ta.kv_lens = d_kv_lens;
+    ta.status = ctx->d_status;
+    rc = m40_attention_prefill_tc(ctx, s, ta, total_kv);
+    if (rc <= 0) return rc;
+    dim3 grid((max_q + PF_TILE - 1) / PF_TILE, q_heads, batch_size);
     const size_t smem = (size_t)2 * 2 * PF_TILE * head_dim * sizeof(__half);
     if (!prefill_configure(ctx->device_id)) return -4;
     if (head_dim == 128)

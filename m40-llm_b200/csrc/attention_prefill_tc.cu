@@ -1,0 +1,376 @@
+// Prompt attention on the 5th-generation tensor cores: CTA = 128 query rows of one (sequence, q head), keys in tiles of 128.
+//
+//   scores   S[128 q rows][128 keys] = Qhi K^T + Qlo K^T   A = queries (f16 hi and lo, shared memory), B = the key tile, K-major;
+//   softmax  thread = query row = accumulator lane, so a row needs no exchange. A row's reference moves only when its maximum has
+//            grown by 2^8 or more (weights stay in f16 range below that): the accumulated output is rarely rescaled;
+//   values   O[128][HD] += P V                              A = the weights in tensor memory (f16, over the scores they came from),
+//                                                           B = the value tile, MN-major.
+//
+// Warps 0..3 are the query rows, warp 4 loads K and V by TMA (two stages each), warp 5 issues the MMAs: S(j + 1) runs while the
+// rows work on S(j). A 128 x 128 tile of HD 128 is 24 MMAs (1536 cycles at the tensor rate) beside 1024 cycles of exponentials per
+// scheduler; one set of rows per SM leaves part of either idle. Four packed prompts of 509 to 2048 tokens, 32 / 8 heads of 128:
+// 264 us, against 438 us with mma.sync fragments (attention_prefill.cu), which stay for short segments.
+// Rows behind a sequence's last key are whatever the cache holds there; the issuing warp clears them in the value tile, since
+// zero weights do not cancel a NaN.
+//
+// Every wait is bounded: a wait that runs out raises status bit 4; nothing waits any more from then on, copies in flight are drained
+// and tensor memory is freed.
+#include "attention.cuh"
+#include "attention_mma.cuh"
+#include "attention_prefill_tc.cuh"
+#include "gemm_tc.cuh"
+#include "stack_math.cuh"
+#include "tc_ptx.cuh"
+
+namespace {
+
+using namespace tc;
+using attn_mma::fast_exp2;
+using attn_mma::LOG2E;
+using attn_mma::pack_h2;
+using attn_mma::split_h2;
+
+constexpr uint32_t ROWS = 128, KEYS = 128, CHUNK = 128 * 128;  // a chunk: 128 rows of 64 f16
+constexpr uint32_t IDESC_B_MN = 1u << 16;
+
+template <int HD>
+struct Smem {
+    static constexpr uint32_t CH = HD / 64, TILE = CH * CHUNK;
+    static constexpr uint32_t Q_HI = 0, Q_LO = TILE, K0 = 2 * TILE, V0 = 4 * TILE, END = 6 * TILE;
+    // staged output: per warp 32 rows of HD + 4 floats, over the dead tiles
+    static constexpr uint32_t OUT_ROW = HD + 4;
+    static_assert(4 * 32 * OUT_ROW * 4 <= END, "output staging");
+    // one CTA per SM: 512 columns of tensor memory are all there is
+    static constexpr uint32_t BYTES = (END < 116 * 1024 ? 116 * 1024 : END) + 1024;
+};
+
+// MN-major, 128-byte-swizzled operand: 64-element chunks along MN are lbo bytes apart, groups of 8 along K 1024 bytes.
+__device__ __forceinline__ uint64_t make_desc_mn(uint32_t smem_addr, uint32_t lbo) {
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)(lbo >> 4) << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+
+template <int HD, bool CACHE>
+__global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                                                            M40PrefillTcArgs a) {
+    using L = Smem<HD>;
+    extern __shared__ unsigned char smem_unaligned[];
+    unsigned char* smem = smem_unaligned + ((1024u - (smem_u32(smem_unaligned) & 1023u)) & 1023u);
+    __shared__ uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], o_done[2], p_ready[2], q_ready;
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile uint32_t abort_flag;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    // the last q tiles of a sequence see the most keys: they are scheduled first
+    const uint32_t b = blockIdx.z, qh = blockIdx.y, r0 = (gridDim.x - 1u - blockIdx.x) * ROWS;
+    const M40PrefillCall& pc = a.c;
+    if (CACHE) {
+        pdl_wait();
+        pdl_trigger();
+    }
+    const uint32_t q_len = CACHE ? pc.seg[4 * b + 1] : a.q_lens[b];
+    const uint32_t kv_len = CACHE ? pc.seg[4 * b + 3] + q_len : a.kv_lens[b];
+    if (r0 >= q_len || q_len == 0 || kv_len == 0 || q_len > kv_len) return;
+    const uint32_t kvh = qh / (pc.q_heads / pc.kv_heads);
+    const uint32_t slot = CACHE ? pc.seg[4 * b + 2] * pc.slot_mul + pc.slot_add : 0u;
+    if (CACHE && (slot >= pc.slots || kv_len > pc.max_seq_len || (uint64_t)pc.seg[4 * b] + q_len > pc.rows)) {
+        if (threadIdx.x == 0) atomicOr(a.status, 1u);
+        return;
+    }
+    const size_t q_row0 = (size_t)(CACHE ? pc.seg[4 * b] : a.q_offsets[b]) + r0;
+    const int kv_row = (int)(CACHE ? (slot * pc.kv_heads + kvh) * pc.max_seq_len : a.kv_offsets[b]);
+    const int kv_col = CACHE ? 0 : (int)(kvh * HD);
+    const uint32_t shift = kv_len - q_len;                              // q row i sees keys 0 .. shift + i
+    const uint32_t kv_end = shift + min(r0 + ROWS, q_len);
+    const uint32_t n_tiles = (kv_end + KEYS - 1) / KEYS;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&k_full[i], 1);
+            mbar_init(&k_empty[i], 1);
+            mbar_init(&v_full[i], 1);
+            mbar_init(&v_empty[i], 1);
+            mbar_init(&s_full[i], 1);
+            // A row waits for a value product now and then only, by parity. Two barriers in turn keep that unambiguous: s_full of
+            // tile j says that product j - 2 is done, and product j + 1 cannot be before the row has handed over tile j.
+            mbar_init(&o_done[i], 1);
+            // S(j + 1) is there before all rows have handed over tile j: a fast warp's next arrival needs a barrier of its own
+            mbar_init(&p_ready[i], 128);
+        }
+        mbar_init(&q_ready, 128);
+        abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 5) tmem_alloc(&tmem_slot, 512);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_s = tmem_slot, tmem_o = tmem_s + 2 * KEYS;
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+        if (abort_flag) return false;
+        if (mbar_wait(bar, parity)) return true;
+        abort_flag = 1;
+        atomicOr(a.status, 4u);
+        return false;
+    };
+
+    if (warp == 4) {
+        if (lane == 0) {
+            uint32_t j = 0;
+            for (; j < n_tiles; ++j) {
+                const uint32_t s = j & 1u, round = j >> 1;
+                const int row = kv_row + (int)(j * KEYS);
+                if (round > 0 && !wait(&k_empty[s], (round - 1u) & 1u)) break;
+                mbar_expect_tx(&k_full[s], L::TILE);
+                for (uint32_t c = 0; c < L::CH; ++c)
+                    tma_load_2d(smem + L::K0 + s * L::TILE + c * CHUNK, &tmK, &k_full[s], kv_col + (int)(c * 64u), row);
+                if (round > 0 && !wait(&v_empty[s], (round - 1u) & 1u)) {
+                    mbar_wait(&k_full[s], round & 1u);
+                    break;
+                }
+                mbar_expect_tx(&v_full[s], L::TILE);
+                for (uint32_t c = 0; c < L::CH; ++c)
+                    tma_load_2d(smem + L::V0 + s * L::TILE + c * CHUNK, &tmV, &v_full[s], kv_col + (int)(c * 64u), row);
+            }
+            if (abort_flag)  // copies in flight land (bounded) before the CTA goes away
+                for (uint32_t i = j > 2 ? j - 2 : 0u; i < j; ++i) {
+                    mbar_wait(&k_full[i & 1u], (i >> 1) & 1u);
+                    mbar_wait(&v_full[i & 1u], (i >> 1) & 1u);
+                }
+        }
+        __syncwarp();
+    } else if (warp == 5) {
+        // the warp walks the loop converged (see elect_one()), one lane issues
+        const uint32_t idesc_s = make_idesc(KEYS), idesc_o = make_idesc(HD) | IDESC_B_MN;
+        const uint32_t q_at = smem_u32(smem), k_at = smem_u32(smem + L::K0), v_at = smem_u32(smem + L::V0);
+        auto scores = [&](uint32_t j) {
+            const uint32_t s = j & 1u;
+            if (!__all_sync(0xffffffffu, wait(&k_full[s], (j >> 1) & 1u))) return false;
+            tc_fence_after();
+            if (elect_one()) {
+#pragma unroll
+                for (uint32_t k = 0; k < HD / UMMA_K; ++k) {
+                    const uint32_t at = (k >> 2) * CHUNK + (k & 3u) * 32u;
+                    const uint64_t dk = make_desc_sw128(k_at + s * L::TILE + at);
+                    umma_f16(tmem_s + s * KEYS, make_desc_sw128(q_at + L::Q_HI + at), dk, idesc_s, k);
+                    umma_f16(tmem_s + s * KEYS, make_desc_sw128(q_at + L::Q_LO + at), dk, idesc_s, 1u);
+                }
+                umma_commit(&k_empty[s]);
+                umma_commit(&s_full[s]);
+            }
+            __syncwarp();
+            return true;
+        };
+        bool ok = __all_sync(0xffffffffu, wait(&q_ready, 0));
+        ok = ok && scores(0);
+        if (ok && n_tiles > 1) ok = scores(1);
+        for (uint32_t j = 0; j < n_tiles && ok; ++j) {
+            const uint32_t s = j & 1u;
+            ok = __all_sync(0xffffffffu, wait(&v_full[s], (j >> 1) & 1u));
+            if (!ok) break;
+            if ((j + 1) * KEYS > kv_end) {
+                const uint32_t first = kv_end - j * KEYS;
+                for (uint32_t i = first * 8u + lane; i < KEYS * 8u; i += 32u)
+                    for (uint32_t c = 0; c < L::CH; ++c)
+                        *reinterpret_cast<uint4*>(smem + L::V0 + s * L::TILE + c * CHUNK + i * 16u) = make_uint4(0u, 0u, 0u, 0u);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+            }
+            ok = __all_sync(0xffffffffu, wait(&p_ready[s], (j >> 1) & 1u));
+            if (!ok) break;
+            tc_fence_after();
+            if (elect_one()) {
+#pragma unroll
+                for (uint32_t k = 0; k < KEYS / UMMA_K; ++k)
+                    umma_f16_ts(tmem_o, tmem_s + s * KEYS + k * 8u, make_desc_mn(v_at + s * L::TILE + k * 2048u, CHUNK), idesc_o, j | k);
+                umma_commit(&v_empty[s]);
+                umma_commit(&o_done[s]);
+            }
+            __syncwarp();
+            if (j + 2 < n_tiles) ok = scores(j + 2);  // into the buffer whose weights the MMAs above read first
+        }
+    } else {
+        const uint32_t tid = threadIdx.x, row = r0 + tid;
+        const uint32_t lane_addr = (warp * 32u) << 16;
+        // ---- the queries, scaled to base 2, as f16 hi and lo
+        {
+            const float qs = pc.scale * LOG2E;
+            constexpr uint32_t PIECES = HD / 8;
+#pragma unroll 4
+            for (uint32_t i = tid; i < ROWS * PIECES; i += 128u) {
+                const uint32_t r = i / PIECES, p = i % PIECES;
+                float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), x1 = x0;
+                if (r0 + r < q_len && p * 8u < pc.q_dim) {
+                    const float4* q = reinterpret_cast<const float4*>(pc.q + (q_row0 + r) * pc.q_ld + qh * pc.q_dim + p * 8u);
+                    x0 = q[0], x1 = q[1];
+                }
+                uint32_t hi[4], lo[4];
+                split_h2(x0.x * qs, x0.y * qs, &hi[0], &lo[0]);
+                split_h2(x0.z * qs, x0.w * qs, &hi[1], &lo[1]);
+                split_h2(x1.x * qs, x1.y * qs, &hi[2], &lo[2]);
+                split_h2(x1.z * qs, x1.w * qs, &hi[3], &lo[3]);
+                unsigned char* dst = smem + (p >> 3) * CHUNK + r * 128u + (((p & 7u) ^ (r & 7u)) << 4);
+                *reinterpret_cast<uint4*>(dst + L::Q_HI) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4*>(dst + L::Q_LO) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            mbar_arrive(&q_ready);
+        }
+        const uint32_t lim = shift + min(row, q_len - 1u);  // last key this row sees
+        float ref = -INFINITY, l = 0.0f;
+        if (CACHE && pc.sink) {  // a sink is a key whose score is known from the start and whose value is zero
+            ref = pc.sink[qh] * LOG2E;
+            l = 1.0f;
+        }
+        bool ok = true;
+        for (uint32_t j = 0; j < n_tiles && ok; ++j) {
+            const uint32_t base = j * KEYS, s_at = tmem_s + (j & 1u) * KEYS + lane_addr;
+            ok = __all_sync(0xffffffffu, wait(&s_full[j & 1u], (j >> 1) & 1u));  // tensor-memory loads are warp-collective
+            if (!ok) break;
+            tc_fence_after();
+            uint32_t raw[KEYS];
+            tmem_ld_x64(s_at, raw);
+            tmem_ld_x64(s_at + 64u, raw + 64);
+            tmem_ld_wait();
+            float s[KEYS];
+#pragma unroll
+            for (uint32_t i = 0; i < KEYS; ++i) s[i] = __uint_as_float(raw[i]);
+            if (base + KEYS - 1u > shift + min(r0 + warp * 32u, q_len - 1u)) {  // some row of the warp does not see all of the tile
+#pragma unroll
+                for (uint32_t i = 0; i < KEYS; ++i)
+                    if (base + i > lim) s[i] = -INFINITY;
+            }
+            float mx[4] = {s[0], s[1], s[2], s[3]};
+#pragma unroll
+            for (uint32_t i = 4; i < KEYS; ++i) mx[i & 3u] = fmaxf(mx[i & 3u], s[i]);
+            const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+            const bool grow = top > ref + 8.0f;  // also a first finite maximum: the reference is -inf
+            float corr = 1.0f;
+            if (grow) {
+                corr = fast_exp2(ref - top);
+                ref = top;
+                l *= corr;
+            }
+            if (j > 0 && __any_sync(0xffffffffu, grow)) {
+                ok = __all_sync(0xffffffffu, wait(&o_done[(j - 1u) & 1u], ((j - 1u) >> 1) & 1u));
+                tc_fence_after();
+#pragma unroll
+                for (uint32_t c = 0; c < HD; c += 16) {
+                    uint32_t r[16];
+                    tmem_ld_x16(tmem_o + lane_addr + c, r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * corr);
+                    tmem_st_x16(tmem_o + lane_addr + c, r);
+                }
+            }
+            const float use = ref == -INFINITY ? 0.0f : ref;
+            float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (uint32_t c = 0; c < KEYS / 2; c += 16) {
+                uint32_t p[16];
+#pragma unroll
+                for (uint32_t i = 0; i < 16; ++i) {
+                    const float p0 = fast_exp2(s[2 * (c + i)] - use), p1 = fast_exp2(s[2 * (c + i) + 1] - use);
+                    sum[i & 3u] += p0 + p1;
+                    p[i] = pack_h2(p0, p1);
+                }
+                tmem_st_x16(s_at + c, p);
+            }
+            l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+            tmem_st_wait();
+            tc_fence_before();
+            mbar_arrive(&p_ready[j & 1u]);
+        }
+        ok = ok && __all_sync(0xffffffffu, wait(&o_done[(n_tiles - 1u) & 1u], ((n_tiles - 1u) >> 1) & 1u));
+        if (ok) {
+            tc_fence_after();
+            float o[HD];
+            {
+                uint32_t r[HD];
+                tmem_ld_x64(tmem_o + lane_addr, r);
+                if (HD == 128) tmem_ld_x64(tmem_o + lane_addr + 64u, r + HD - 64);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < HD; ++i) o[i] = __uint_as_float(r[i]);
+            }
+            float inv = 1.0f / (l > 0.0f ? l : 1.0f);
+            if (CACHE && pc.turn_back) {
+                const float4* t = reinterpret_cast<const float4*>(pc.turn_back + (q_row0 - r0 + min(row, q_len - 1u)) * (HD / 2));
+#pragma unroll
+                for (int i = 0; i < HD / 4; ++i) {
+                    const float4 cs = t[i];
+                    const float u0 = o[2 * i], v0 = o[2 * i + HD / 2], u1 = o[2 * i + 1], v1 = o[2 * i + 1 + HD / 2];
+                    o[2 * i] = u0 * cs.x + v0 * cs.y;
+                    o[2 * i + HD / 2] = v0 * cs.x - u0 * cs.y;
+                    o[2 * i + 1] = u1 * cs.z + v1 * cs.w;
+                    o[2 * i + 1 + HD / 2] = v1 * cs.z - u1 * cs.w;
+                }
+            }
+            if (CACHE && pc.gate && row < q_len) inv *= m40_sigmoid(pc.gate[(q_row0 + tid) * pc.gate_ld + qh]);
+            // rows leave through shared memory (every tile has been read), whole lines at a time
+            float* stage = reinterpret_cast<float*>(smem) + warp * 32u * L::OUT_ROW;
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+#pragma unroll
+            for (int i = 0; i < HD; i += 4)
+                *reinterpret_cast<float4*>(stage + lane * L::OUT_ROW + i) =
+                    make_float4(o[i] * inv, o[i + 1] * inv, o[i + 2] * inv, o[i + 3] * inv);
+            __syncwarp();
+            constexpr uint32_t PER = HD / 4;  // float4 per row
+            for (uint32_t i = lane; i < 32u * PER; i += 32u) {
+                const uint32_t r = i / PER, c = (i % PER) * 4u;
+                if (r0 + warp * 32u + r < q_len && c < pc.v_dim)
+                    *reinterpret_cast<float4*>(pc.out + (q_row0 + warp * 32u + r) * pc.out_ld + qh * pc.v_dim + c) =
+                        *reinterpret_cast<const float4*>(stage + r * L::OUT_ROW + c);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 5) {
+        tc_fence_after();
+        tmem_dealloc(tmem_slot, 512);
+    }
+}
+
+template <int HD, bool CACHE>
+int launch(M40llmCudaContext* ctx, cudaStream_t s, const CUtensorMap& mk, const CUtensorMap& mv, const M40PrefillTcArgs& a) {
+    static unsigned long long configured = 0ull;
+    const unsigned long long bit = 1ull << (ctx->device_id & 63);
+    if (!(configured & bit)) {
+        if (cudaFuncSetAttribute(prefill_tc_kernel<HD, CACHE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem<HD>::BYTES) !=
+            cudaSuccess)
+            return -4;
+        configured |= bit;
+    }
+    const dim3 grid((a.c.max_segment_rows + ROWS - 1) / ROWS, a.c.q_heads, a.c.segments);
+    cudaError_t e;
+    if (CACHE) {
+        e = m40_launch_dependent(prefill_tc_kernel<HD, CACHE>, grid, dim3(192), Smem<HD>::BYTES, s, mk, mv, a);
+    } else {
+        prefill_tc_kernel<HD, CACHE><<<grid, 192, Smem<HD>::BYTES, s>>>(mk, mv, a);
+        e = cudaSuccess;
+    }
+    M40_COUNT_LAUNCH(ctx);
+    return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
+
+}  // namespace
+
+int m40_attention_prefill_tc(M40llmCudaContext* ctx, cudaStream_t s, const M40PrefillTcArgs& a, uint64_t kv_rows) {
+    const M40PrefillCall& c = a.c;
+    const bool cache = c.seg != nullptr;
+    if (c.hd != 64 && c.hd != 128) return 1;
+    if (c.max_segment_rows < M40_PREFILL_TC_MIN_ROWS) return 1;
+    if (((((uintptr_t)c.q) | ((uintptr_t)c.out) | ((uintptr_t)c.K) | ((uintptr_t)c.V) | ((uintptr_t)c.turn_back)) & 15u) != 0u) return 1;
+    if (c.q_dim % 8 != 0 || c.v_dim % 4 != 0 || c.q_ld % 4 != 0 || c.out_ld % 4 != 0 || kv_rows >= 0x7fffffffull) return 1;
+    CUtensorMap mk, mv;
+    const uint64_t cols = cache ? c.hd : (uint64_t)c.kv_heads * c.hd;
+    if (!m40_tc_map(&mk, c.K, kv_rows, cols, KEYS, false) || !m40_tc_map(&mv, c.V, kv_rows, cols, KEYS, false)) return 1;
+    if (c.hd == 128) return cache ? launch<128, true>(ctx, s, mk, mv, a) : launch<128, false>(ctx, s, mk, mv, a);
+    return cache ? launch<64, true>(ctx, s, mk, mv, a) : launch<64, false>(ctx, s, mk, mv, a);
+}

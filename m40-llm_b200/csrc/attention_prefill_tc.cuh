@@ -1,0 +1,18 @@
+// Prompt attention on tcgen05; see attention_prefill_tc.cu.
+#pragma once
+#include "attention.cuh"
+
+// Segments shorter than this stay on the mma.sync kernel: they fill one of its 64-row tiles and half of a 128-row tile here.
+constexpr uint32_t M40_PREFILL_TC_MIN_ROWS = 65;
+
+struct M40PrefillTcArgs {
+    M40PrefillCall c;  // c.seg null: packed K, V [rows][kv_heads][hd] with the offsets and lengths below
+    const uint32_t* q_offsets;
+    const uint32_t* kv_offsets;
+    const uint32_t* q_lens;
+    const uint32_t* kv_lens;
+    uint32_t* status;
+};
+// kv_rows: rows of the K and V arrays (cache: slots * kv_heads * max_seq_len). 0 when launched, 1 for a call it does not take,
+// < 0 on failure.
+int m40_attention_prefill_tc(M40llmCudaContext* ctx, cudaStream_t s, const M40PrefillTcArgs& a, uint64_t kv_rows);

@@ -116,3 +116,32 @@ def test_build_compressed_from_dense(nat, O, kvh, hd, R, bs, L):
     for kv in (dense, comp, other):
         nat.lib.m40llm_kvcache_destroy(kv)
     nat.free_all()
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("pos,rows,scale", [(0, 65, 1.0), (33, 100, 1.0), (0, 128, 6.0), (127, 129, 6.0), (0, 700, 6.0), (900, 257, 1.0)])
+def test_step_rows_over_cache(nat, pkg, hd, pos, rows, scale):
+    """Prompt attention over the cache at the edges of its 128 x 128 tiles; with scale 6 a row's maximum grows past its reference
+    from tile to tile. Probabilities are f16: an output is off by at most 2^-11 of the largest value."""
+    N = pkg.native
+    rng = np.random.default_rng(hd + rows)
+    qh, kvh, L = 8, 2, pos + rows
+    kv = nat.kv_dense(L + 7, 4, kvh, hd)
+    K, V = (rng.standard_normal((L, kvh, hd)).astype(np.float16) for _ in range(2))
+    nat.kv_fill(kv, 3, K, V)
+    q = (scale * rng.standard_normal((rows, qh, hd))).astype(np.float32)
+    dq, do, ds = nat.buf(q), nat.buf(q.nbytes), nat.buf(np.array([0, rows, 1, pos], np.uint32))
+    r = N.StepRows(rows=rows, segments=1, max_segment_rows=rows, max_len=L, slot_mul=2, slot_add=1, seg=ds.ptr)
+    for _ in range(3):
+        do.upload(np.full(q.shape, 9.0, np.float32))
+        assert nat.lib.m40llm_attention_step_rows_async(nat.ctx, kv, dq.ptr, qh, C.byref(r), do.ptr) == 0
+        nat.sync(1)
+        got = do.download(np.float32, q.shape)
+        for h in range(qh):
+            s = q[:, h].astype(np.float64) @ K[:, h // 4].astype(np.float64).T / np.sqrt(hd)
+            s[np.arange(L)[None, :] > (pos + np.arange(rows))[:, None]] = -np.inf
+            p = np.exp(s - s.max(1, keepdims=True))
+            want = (p / p.sum(1, keepdims=True)) @ V[:, h // 4].astype(np.float64)
+            assert np.abs(got[:, h] - want).max() <= 2.0 ** -11 * float(np.abs(V).max()) + 1e-4
+    nat.lib.m40llm_kvcache_destroy(kv)
+    nat.free_all()
