@@ -68,10 +68,7 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
     // the last q tiles of a sequence see the most keys: they are scheduled first
     const uint32_t b = blockIdx.z, qh = blockIdx.y, r0 = (gridDim.x - 1u - blockIdx.x) * ROWS;
     const M40PrefillCall& pc = a.c;
-    if (CACHE) {
-        pdl_wait();
-        pdl_trigger();
-    }
+    if (CACHE) pdl_wait();
     const uint32_t q_len = CACHE ? pc.seg[4 * b + 1] : a.q_lens[b];
     const uint32_t kv_len = CACHE ? pc.seg[4 * b + 3] + q_len : a.kv_lens[b];
     if (r0 >= q_len || q_len == 0 || kv_len == 0 || q_len > kv_len) return;
@@ -109,6 +106,7 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (CACHE) pdl_trigger();  // only now: see m40_launch_dependent()
     const uint32_t tmem_s = tmem_slot, tmem_o = tmem_s + 2 * KEYS;
     auto wait = [&](uint64_t* bar, uint32_t parity) {
         if (abort_flag) return false;

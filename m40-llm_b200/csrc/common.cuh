@@ -140,6 +140,8 @@ void* m40_ensure_scratch(M40llmCudaContext* ctx, uint32_t kind, size_t bytes, ui
 // on the stream is still running; it must execute pdl_wait() before it reads anything the predecessor wrote and
 // before its own first global write. Kernels call pdl_trigger() early so that their successor's CTAs are placed
 // the moment resources free up. Both are no-ops for plain launches. M40LLM_PDL=0 turns the launch attribute off.
+// A kernel that takes tensor memory takes it before pdl_trigger(): a successor placed beside a CTA that has not yet taken its
+// columns could take them itself and then wait for this grid, which would wait for the columns.
 // ----------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -147,7 +147,8 @@ def test_short_convolution(nat, dim, taps, bias, add):
 
 # -------------------------------------------------------------------------------------------------- latent attention
 class Latent:
-    def __init__(self, nat, H, D, V, R, fp32, sink=True, scale=None, slots=5, max_len=1400, seed=0, sharp=1.0):
+    def __init__(self, nat, H, D, V, R, fp32, sink=True, scale=None, slots=5, max_len=1400, seed=0, sharp=1.0, wdt=N.DT_BF16):
+        self.wdt, pack = wdt, bits if wdt == N.DT_BF16 else (lambda nat, a: nat.buf(np.ascontiguousarray(a, np.float16)).ptr)
         self.nat, self.H, self.D, self.V, self.R, self.eps = nat, H, D, V, R, 1e-4
         rng = np.random.default_rng(seed)
         self.scale = D ** -0.5 if scale is None else scale
@@ -157,7 +158,7 @@ class Latent:
         self.kv = nat.lib.m40llm_kvcache_create_typed(nat.ctx, max_len, slots, 1, R, 0, N.DT_F32 if fp32 else N.DT_F16)
         self.ld = (H * D + R + 7) // 8 * 8
         ukt = self.uk.reshape(H, D, R).transpose(0, 2, 1).reshape(H * R, D)
-        self.dev = [f32(nat, self.cn), bits(nat, self.uk), bits(nat, ukt), bits(nat, self.uv), f32(nat, self.sink) if sink else None]
+        self.dev = [f32(nat, self.cn), pack(nat, self.uk), pack(nat, ukt), pack(nat, self.uv), f32(nat, self.sink) if sink else None]
 
     def oracle(self, q, c):
         """q [T, H * D], c [T, R] of one sequence from position 0 -> [T, H * V]."""
@@ -181,7 +182,7 @@ class Latent:
         packed = np.zeros((rows.n, self.ld), np.float32)
         packed[:, :self.H * self.D], packed[:, self.H * self.D:self.H * self.D + self.R] = q, c
         out = nat.buf(rows.n * self.H * self.V * 4)
-        call = N.LatentAttention(f32(nat, packed), *self.dev, out.ptr, self.ld, self.H, self.D, self.V, N.DT_BF16, self.eps, self.scale)
+        call = N.LatentAttention(f32(nat, packed), *self.dev, out.ptr, self.ld, self.H, self.D, self.V, self.wdt, self.eps, self.scale)
         rc = nat.lib.m40llm_attention_latent_async(nat.ctx, self.kv, C.byref(call), C.byref(rows.c))
         assert rc == 0, rc
         nat.sync(1)
@@ -276,6 +277,22 @@ def test_latent_attention_batch_decode_lengths(nat):
     t.dev[2] = None       # and without the transposed matrix
     got = t.run([(s, n - 1, 1) for s, n in enumerate(lens)], np.array(q), np.array(c), host=False)
     close(got, np.array(want), 3e-3)
+    no_status(nat)
+    t.close()
+
+
+@pytest.mark.parametrize("D,V", [(64, 64), (128, 128), (64, 48)])
+def test_latent_portions_back_to_back(nat, D, V):
+    """f16 weights and whole heads: the prompt kernel of one portion is followed directly by the projection of the next one, and
+    both want tensor memory. Values as exact in f16 as in bf16 (the weights are bf16 values well inside f16's range)."""
+    t = Latent(nat, 40, D, V, 128, 0, slots=9, seed=D + V, wdt=N.DT_F16)
+    rng = np.random.default_rng(7)
+    lens = (300, 129, 65, 200)
+    q, c = ([rng.standard_normal((n, w)).astype(np.float32) for n in lens] for w in (40 * D, 128))
+    want = np.concatenate([t.oracle(a, b) for a, b in zip(q, c)])
+    for _ in range(5):
+        got = t.run([(s, 0, n) for s, n in enumerate(lens)], np.concatenate(q), np.concatenate(c), max_len=max(lens))
+        close(got, want, 3e-3)
     no_status(nat)
     t.close()
 
