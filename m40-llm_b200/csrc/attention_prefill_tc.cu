@@ -1,15 +1,21 @@
 // Prompt attention on the 5th-generation tensor cores: CTA = 128 query rows of one (sequence, q head), keys in tiles of 128.
 //
 //   scores   S[128 q rows][128 keys] = Qhi K^T + Qlo K^T   A = queries (f16 hi and lo, shared memory), B = the key tile, K-major;
-//   softmax  thread = query row = accumulator lane, so a row needs no exchange. A row's reference moves only when its maximum has
-//            grown by 2^8 or more (weights stay in f16 range below that): the accumulated output is rarely rescaled;
-//   values   O[128][HD] += P V                              A = the weights in tensor memory (f16, over the scores they came from),
-//                                                           B = the value tile, MN-major.
+//   softmax  thread = query row = accumulator lane, so a row needs no exchange;
+//   values   O[128][HD + 16] += P [V | 1]                   A = the weights in tensor memory (f16, over the scores they came from),
+//                                                           B = the value tile, MN-major, and behind it a chunk of ones, whose
+//                                                           columns add up the weights that the values were multiplied with.
+//
+// A row's reference is its running maximum, so its strongest key weighs exactly 1, and numerator and denominator share the
+// rounding of all others: relative error 0.96 to 1.01 of what the mma.sync form gives, for queries scaled by 1 to 8. (A reference
+// that moves only with every 2^8 of growth saves most of the rescaling, 264 against 273 us and 203 against 221 us at head size 64,
+// but its strongest weight is rounded: 1.05 times that error for flat scores, 3.3 times for peaked ones. Adding up the rounded
+// weights in the rows' registers took 285 us.)
 //
 // Warps 0..3 are the query rows, warp 4 loads K and V by TMA (two stages each), warp 5 issues the MMAs: S(j + 1) runs while the
-// rows work on S(j). A 128 x 128 tile of HD 128 is 24 MMAs (1536 cycles at the tensor rate) beside 1024 cycles of exponentials per
+// rows work on S(j). A 128 x 128 tile of HD 128 is 24 MMAs (1600 cycles at the tensor rate) beside 1024 cycles of exponentials per
 // scheduler; one set of rows per SM leaves part of either idle. Four packed prompts of 509 to 2048 tokens, 32 / 8 heads of 128:
-// 264 us, against 438 us with mma.sync fragments (attention_prefill.cu), which stay for short segments.
+// 273 us, against 438 us with mma.sync fragments (attention_prefill.cu), which stay for short segments.
 // Rows behind a sequence's last key are whatever the cache holds there; the issuing warp clears them in the value tile, since
 // zero weights do not cancel a NaN.
 //
@@ -36,7 +42,8 @@ constexpr uint32_t IDESC_B_MN = 1u << 16;
 template <int HD>
 struct Smem {
     static constexpr uint32_t CH = HD / 64, TILE = CH * CHUNK;
-    static constexpr uint32_t Q_HI = 0, Q_LO = TILE, K0 = 2 * TILE, V0 = 4 * TILE, END = 6 * TILE;
+    static constexpr uint32_t V_PITCH = TILE + CHUNK;  // a value tile, then 128 rows of ones
+    static constexpr uint32_t Q_HI = 0, Q_LO = TILE, K0 = 2 * TILE, V0 = 4 * TILE, END = V0 + 2 * V_PITCH;
     // staged output: per warp 32 rows of HD + 4 floats, over the dead tiles
     static constexpr uint32_t OUT_ROW = HD + 4;
     static_assert(4 * 32 * OUT_ROW * 4 <= END, "output staging");
@@ -132,7 +139,7 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
                 }
                 mbar_expect_tx(&v_full[s], L::TILE);
                 for (uint32_t c = 0; c < L::CH; ++c)
-                    tma_load_2d(smem + L::V0 + s * L::TILE + c * CHUNK, &tmV, &v_full[s], kv_col + (int)(c * 64u), row);
+                    tma_load_2d(smem + L::V0 + s * L::V_PITCH + c * CHUNK, &tmV, &v_full[s], kv_col + (int)(c * 64u), row);
             }
             if (abort_flag)  // copies in flight land (bounded) before the CTA goes away
                 for (uint32_t i = j > 2 ? j - 2 : 0u; i < j; ++i) {
@@ -143,7 +150,7 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
         __syncwarp();
     } else if (warp == 5) {
         // the warp walks the loop converged (see elect_one()), one lane issues
-        const uint32_t idesc_s = make_idesc(KEYS), idesc_o = make_idesc(HD) | IDESC_B_MN;
+        const uint32_t idesc_s = make_idesc(KEYS), idesc_o = make_idesc(HD + 16) | IDESC_B_MN;
         const uint32_t q_at = smem_u32(smem), k_at = smem_u32(smem + L::K0), v_at = smem_u32(smem + L::V0);
         auto scores = [&](uint32_t j) {
             const uint32_t s = j & 1u;
@@ -174,7 +181,7 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
                 const uint32_t first = kv_end - j * KEYS;
                 for (uint32_t i = first * 8u + lane; i < KEYS * 8u; i += 32u)
                     for (uint32_t c = 0; c < L::CH; ++c)
-                        *reinterpret_cast<uint4*>(smem + L::V0 + s * L::TILE + c * CHUNK + i * 16u) = make_uint4(0u, 0u, 0u, 0u);
+                        *reinterpret_cast<uint4*>(smem + L::V0 + s * L::V_PITCH + c * CHUNK + i * 16u) = make_uint4(0u, 0u, 0u, 0u);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
             }
@@ -184,7 +191,7 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
             if (elect_one()) {
 #pragma unroll
                 for (uint32_t k = 0; k < KEYS / UMMA_K; ++k)
-                    umma_f16_ts(tmem_o, tmem_s + s * KEYS + k * 8u, make_desc_mn(v_at + s * L::TILE + k * 2048u, CHUNK), idesc_o, j | k);
+                    umma_f16_ts(tmem_o, tmem_s + s * KEYS + k * 8u, make_desc_mn(v_at + s * L::V_PITCH + k * 2048u, CHUNK), idesc_o, j | k);
                 umma_commit(&v_empty[s]);
                 umma_commit(&o_done[s]);
             }
@@ -215,11 +222,14 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
                 *reinterpret_cast<uint4*>(dst + L::Q_HI) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
                 *reinterpret_cast<uint4*>(dst + L::Q_LO) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
             }
+            const uint4 ones = make_uint4(0x3c003c00u, 0x3c003c00u, 0x3c003c00u, 0x3c003c00u);
+            for (uint32_t i = tid * 16u; i < CHUNK; i += 128u * 16u)
+                for (uint32_t v = 0; v < 2; ++v) *reinterpret_cast<uint4*>(smem + L::V0 + v * L::V_PITCH + L::TILE + i) = ones;
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             mbar_arrive(&q_ready);
         }
         const uint32_t lim = shift + min(row, q_len - 1u);  // last key this row sees
-        float ref = -INFINITY, l = 0.0f;
+        float ref = -INFINITY, l = 0.0f;  // l: the sink's part of the denominator
         if (CACHE && pc.sink) {  // a sink is a key whose score is known from the start and whose value is zero
             ref = pc.sink[qh] * LOG2E;
             l = 1.0f;
@@ -246,7 +256,7 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
 #pragma unroll
             for (uint32_t i = 4; i < KEYS; ++i) mx[i & 3u] = fmaxf(mx[i & 3u], s[i]);
             const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-            const bool grow = top > ref + 8.0f;  // also a first finite maximum: the reference is -inf
+            const bool grow = top > ref;
             float corr = 1.0f;
             if (grow) {
                 corr = fast_exp2(ref - top);
@@ -257,7 +267,7 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
                 ok = __all_sync(0xffffffffu, wait(&o_done[(j - 1u) & 1u], ((j - 1u) >> 1) & 1u));
                 tc_fence_after();
 #pragma unroll
-                for (uint32_t c = 0; c < HD; c += 16) {
+                for (uint32_t c = 0; c < HD + 16; c += 16) {
                     uint32_t r[16];
                     tmem_ld_x16(tmem_o + lane_addr + c, r);
                     tmem_ld_wait();
@@ -267,19 +277,16 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
                 }
             }
             const float use = ref == -INFINITY ? 0.0f : ref;
-            float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
             for (uint32_t c = 0; c < KEYS / 2; c += 16) {
                 uint32_t p[16];
 #pragma unroll
                 for (uint32_t i = 0; i < 16; ++i) {
                     const float p0 = fast_exp2(s[2 * (c + i)] - use), p1 = fast_exp2(s[2 * (c + i) + 1] - use);
-                    sum[i & 3u] += p0 + p1;
                     p[i] = pack_h2(p0, p1);
                 }
                 tmem_st_x16(s_at + c, p);
             }
-            l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
             tmem_st_wait();
             tc_fence_before();
             mbar_arrive(&p_ready[j & 1u]);
@@ -292,7 +299,10 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
                 uint32_t r[HD];
                 tmem_ld_x64(tmem_o + lane_addr, r);
                 if (HD == 128) tmem_ld_x64(tmem_o + lane_addr + 64u, r + HD - 64);
+                uint32_t weights[4];  // equal columns
+                tmem_ld_x4(tmem_o + lane_addr + HD, weights);
                 tmem_ld_wait();
+                l += __uint_as_float(weights[0]);
 #pragma unroll
                 for (int i = 0; i < HD; ++i) o[i] = __uint_as_float(r[i]);
             }

@@ -145,3 +145,33 @@ def test_step_rows_over_cache(nat, pkg, hd, pos, rows, scale):
             assert np.abs(got[:, h] - want).max() <= 2.0 ** -11 * float(np.abs(V).max()) + 1e-4
     nat.lib.m40llm_kvcache_destroy(kv)
     nat.free_all()
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("pos,rows", [(0, 700), (1000, 129)])
+@pytest.mark.parametrize("scale", [1.0, 2.0, 4.0, 8.0])
+def test_prompt_forms_are_equally_exact(nat, pkg, hd, pos, rows, scale):
+    """Flat to peaked scores: the tcgen05 form rounds weights to f16 relative to the running maximum as the mma.sync form does (which
+    serves queries that lie on 8 bytes only), so their errors are alike; a tenth is left for their different tiles."""
+    rng = np.random.default_rng(hd + rows)
+    qh, kvh, L = 8, 2, pos + rows
+    kv = nat.kv_dense(L, 1, kvh, hd)
+    K, V = (rng.standard_normal((L, kvh, hd)).astype(np.float16) for _ in range(2))
+    nat.kv_fill(kv, 0, K, V)
+    q = (scale * rng.standard_normal((rows, qh, hd))).astype(np.float32)
+    want = np.empty(q.shape)
+    for h in range(qh):
+        s = q[:, h].astype(np.float64) @ K[:, h // 4].astype(np.float64).T / np.sqrt(hd)
+        s[np.arange(L)[None, :] > (pos + np.arange(rows))[:, None]] = -np.inf
+        p = np.exp(s - s.max(1, keepdims=True))
+        want[:, h] = (p / p.sum(1, keepdims=True)) @ V[:, h // 4].astype(np.float64)
+    ds, do, error = nat.buf(np.array([0, rows, 0, pos], np.uint32)), nat.buf(q.nbytes), []
+    r = pkg.native.StepRows(rows=rows, segments=1, max_segment_rows=rows, max_len=L, slot_mul=1, slot_add=0, seg=ds.ptr)
+    for shift in (0, 2):
+        dq = nat.buf(np.concatenate([np.zeros(shift, np.float32), q.ravel()]))
+        assert nat.lib.m40llm_attention_step_rows_async(nat.ctx, kv, dq.ptr + 4 * shift, qh, C.byref(r), do.ptr) == 0
+        nat.sync(1)
+        error.append(np.linalg.norm(do.download(np.float32, q.shape) - want) / np.linalg.norm(want))
+    assert error[0] <= 1.1 * error[1] and error[1] <= 2.0 ** -11, error
+    nat.lib.m40llm_kvcache_destroy(kv)
+    nat.free_all()
