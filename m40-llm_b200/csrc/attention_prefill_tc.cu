@@ -123,29 +123,23 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
         return false;
     };
 
+    uint32_t k_sent = 0, v_sent = 0;  // tiles that the loading thread has requested
     if (warp == 4) {
         if (lane == 0) {
-            uint32_t j = 0;
-            for (; j < n_tiles; ++j) {
+            for (uint32_t j = 0; j < n_tiles; ++j) {
                 const uint32_t s = j & 1u, round = j >> 1;
                 const int row = kv_row + (int)(j * KEYS);
                 if (round > 0 && !wait(&k_empty[s], (round - 1u) & 1u)) break;
                 mbar_expect_tx(&k_full[s], L::TILE);
                 for (uint32_t c = 0; c < L::CH; ++c)
                     tma_load_2d(smem + L::K0 + s * L::TILE + c * CHUNK, &tmK, &k_full[s], kv_col + (int)(c * 64u), row);
-                if (round > 0 && !wait(&v_empty[s], (round - 1u) & 1u)) {
-                    mbar_wait(&k_full[s], round & 1u);
-                    break;
-                }
+                ++k_sent;
+                if (round > 0 && !wait(&v_empty[s], (round - 1u) & 1u)) break;
                 mbar_expect_tx(&v_full[s], L::TILE);
                 for (uint32_t c = 0; c < L::CH; ++c)
                     tma_load_2d(smem + L::V0 + s * L::V_PITCH + c * CHUNK, &tmV, &v_full[s], kv_col + (int)(c * 64u), row);
+                ++v_sent;
             }
-            if (abort_flag)  // copies in flight land (bounded) before the CTA goes away
-                for (uint32_t i = j > 2 ? j - 2 : 0u; i < j; ++i) {
-                    mbar_wait(&k_full[i & 1u], (i >> 1) & 1u);
-                    mbar_wait(&v_full[i & 1u], (i >> 1) & 1u);
-                }
         }
         __syncwarp();
     } else if (warp == 5) {
@@ -320,9 +314,8 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
                 }
             }
             if (CACHE && pc.gate && row < q_len) inv *= m40_sigmoid(pc.gate[(q_row0 + tid) * pc.gate_ld + qh]);
-            // rows leave through shared memory (every tile has been read), whole lines at a time
+            // rows leave through shared memory, whole lines at a time: after the last value product nothing reads or writes a tile
             float* stage = reinterpret_cast<float*>(smem) + warp * 32u * L::OUT_ROW;
-            asm volatile("bar.sync 1, 128;" ::: "memory");
 #pragma unroll
             for (int i = 0; i < HD; i += 4)
                 *reinterpret_cast<float4*>(stage + lane * L::OUT_ROW + i) =
@@ -339,6 +332,11 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
     }
     tc_fence_before();
     __syncthreads();
+    if (abort_flag && warp == 4 && lane == 0)  // copies in flight land (bounded) before the CTA goes away
+        for (uint32_t i = 0; i < 2; ++i) {
+            if (k_sent > i) mbar_wait(&k_full[i], ((k_sent - 1u - i) >> 1) & 1u);
+            if (v_sent > i) mbar_wait(&v_full[i], ((v_sent - 1u - i) >> 1) & 1u);
+        }
     if (warp == 5) {
         tc_fence_after();
         tmem_dealloc(tmem_slot, 512);

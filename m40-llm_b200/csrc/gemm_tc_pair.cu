@@ -18,8 +18,9 @@
 // therefore only SEG k-blocks long; the epilogue warps add them up in registers, rounding, while the MMAs fill the other
 // accumulator.
 //
-// Every wait is bounded: a wait that runs out sets bit 2 of the device status word, the CTAs stop issuing work, wait for their
-// copies in flight, free tensor memory and return.
+// Every wait is bounded: a wait that runs out winds down both CTAs (give_up()): they stop issuing work, raise bit 2 of the
+// device status word, wait for their copies in flight, free tensor memory and return. The barrier of two trading warps
+// (finish_gated()) has no bound of its own, so both come to it equally often whatever their waits gave.
 #include <type_traits>
 
 #include "gemm_tc_pair.cuh"
@@ -184,6 +185,11 @@ __global__ void __launch_bounds__(384, 1) gemm_tc_pair_kernel(const __grid_const
     tc_fence_after();
     const uint32_t tmem_base = tmem_slot;
     pdl_trigger();
+    const auto give_up = [&] {
+        abort_flag = 1;
+        st_cluster(map_to_rank(smem_u32(const_cast<uint32_t*>(&abort_flag)), rank ^ 1u), 1u);
+    };
+    uint32_t it = 0;  // stages that the loading thread has filled
 
     // Registers: launched with 3 x 168 per lane of the three warpgroups; the first keeps 40, the epilogue's two take 232 each.
     if (warp < 4) {
@@ -191,7 +197,7 @@ __global__ void __launch_bounds__(384, 1) gemm_tc_pair_kernel(const __grid_const
         if (warp == 0 && lane == 0) {
             // ---------------- TMA producer of this CTA. The weights of the first ring pass do not depend on the previous
             // kernel; everything else waits for it.
-            uint32_t it = 0, s = 0, round = 0;
+            uint32_t s = 0, round = 0;
             bool waited = false, ok = true;
             for (uint32_t u = pair; u < a.units && ok; u += pairs) {
                 const Unit w = unit_of<PAIRED>(a, u);
@@ -212,7 +218,7 @@ __global__ void __launch_bounds__(384, 1) gemm_tc_pair_kernel(const __grid_const
                 }
                 for (uint32_t i = 0; i < w.n_kb; ++i, ++it) {
                     if (round > 0 && (abort_flag || !mbar_wait(&empty[s], (round - 1) & 1u))) {
-                        abort_flag = 1;
+                        give_up();
                         ok = false;
                         break;
                     }
@@ -229,9 +235,6 @@ __global__ void __launch_bounds__(384, 1) gemm_tc_pair_kernel(const __grid_const
                     if (++s == a.stages) s = 0, ++round;
                 }
             }
-            if (!ok && rank == 0)  // copies of either CTA that are still under way end before the pair leaves
-                for (uint32_t i = it > a.stages ? it - a.stages : 0; i < it; ++i)
-                    mbar_wait_cluster(&full[i % a.stages], (i / a.stages) & 1u);
         } else if (warp == 1 && rank == 0) {
             // ---------------- MMA issuer of the pair: the whole warp walks the loop, so that addresses and descriptors stay in
             // uniform registers; one lane issues
@@ -264,7 +267,7 @@ __global__ void __launch_bounds__(384, 1) gemm_tc_pair_kernel(const __grid_const
                     }
                 }
             }
-            if (!ok) abort_flag = 1;
+            if (!ok) give_up();
         }
         __syncwarp();
     } else {
@@ -278,17 +281,17 @@ __global__ void __launch_bounds__(384, 1) gemm_tc_pair_kernel(const __grid_const
         uint32_t seg = 0, traded = 0;
         bool ok = true;
         pdl_wait();
-        for (uint32_t u = pair; u < a.units && ok; u += pairs) {
+        for (uint32_t u = pair; u < a.units && (PAIRED || ok); u += pairs) {
             const Unit w = unit_of<PAIRED>(a, u);
             const uint32_t m_live = min(a.width, a.M - w.m_base);
             float acc[4][32];
 #pragma unroll
             for (uint32_t e = 0; e < 128; ++e) acc[e / 32][e % 32] = 0.0f;
-            for (uint32_t i = 0; i < w.n_kb; i += SEG, ++seg) {
+            for (uint32_t i = 0; i < w.n_kb && ok; i += SEG, ++seg) {
                 const uint32_t b = seg & 1u;
                 ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[b], (seg >> 1) & 1u));
                 if (!ok) {
-                    abort_flag = 1;
+                    give_up();
                     break;
                 }
                 tc_fence_after();
@@ -306,7 +309,7 @@ __global__ void __launch_bounds__(384, 1) gemm_tc_pair_kernel(const __grid_const
                 __syncwarp();
                 if (lane == 0) mbar_arrive_cluster(b ? empty1 : empty0);
             }
-            if (!ok) break;
+            if (!PAIRED && !ok) break;
             const uint32_t in_tile = rank * BLOCK_N + lane_group * 32u + lane;
             const uint32_t n = PAIRED ? w.row0 + rank * (BLOCK_N / 2) + (lane_group & 1u) * 32u + lane : w.row0 + in_tile;
             const uint32_t pitch = a.tiles * M40_PAIR_ROWS;
@@ -314,7 +317,7 @@ __global__ void __launch_bounds__(384, 1) gemm_tc_pair_kernel(const __grid_const
             for (uint32_t q = 0; q < 4; ++q) {
                 const uint32_t c = q * 64u + half * 32u;
                 if (c >= m_live) continue;
-                const uint32_t live = min(32u, m_live - c);
+                const uint32_t live = ok ? min(32u, m_live - c) : 0u;
                 if (PAIRED) {
                     finish_gated(a, acc[q], w.m_base + c, n, live, lane_group < 2u, 1u + warp_pair,
                                  trade + ((traded++ & 1u) * 4u + warp_pair) * 1024u);
@@ -329,10 +332,17 @@ __global__ void __launch_bounds__(384, 1) gemm_tc_pair_kernel(const __grid_const
             }
         }
     }
-    if (abort_flag && threadIdx.x == 128) atomicOr(a.status, 4u);
     tc_fence_before();
     __syncthreads();
     cluster_sync_all();  // neither CTA leaves while the other's MMAs or barriers still use its memory
+    if (abort_flag) {    // the same in both CTAs by now
+        if (threadIdx.x == 0 && rank == 0) {
+            atomicOr(a.status, 4u);
+            for (uint32_t s = 0; s < a.stages && s < it; ++s)  // copies of either CTA that are still under way land
+                mbar_wait_cluster(&full[s], ((it - 1u - s) / a.stages) & 1u);
+        }
+        cluster_sync_all();
+    }
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, 512);

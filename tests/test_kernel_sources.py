@@ -12,7 +12,7 @@ SOURCES = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
 
 
 def plain(path):
-    """The source without comments and string contents."""
+    """The source without comments."""
     text = re.sub(r"//[^\n]*", "", open(path).read())
     return re.sub(r"/\*.*?\*/", "", text, flags=re.S)
 
@@ -36,3 +36,19 @@ def test_tensor_memory_is_taken_before_successors_may_start(path):
         alloc = re.search(r"\btmem_alloc\w*\(", body)
         for m in re.finditer(r"\bpdl_trigger\(\);", body[:alloc.start()] if alloc else ""):
             assert "return;" in body[m.end():body.index("}", m.end())], name
+
+
+def test_unbounded_barriers_do_not_hang_on_a_wait_that_ran_out():
+    """A warp whose bounded wait ran out must not leave others in a named barrier, which has no bound: the prompt kernel has none,
+    and in the CTA-pair kernel the warps that trade columns walk all units whatever their waits gave. What went wrong is reported
+    once no thread can find out any more, and copies in flight are waited for then, whoever gave up."""
+    (prompt,) = [b for _, b in kernels(plain(os.path.join(CSRC, "attention_prefill_tc.cu")))]
+    assert "bar.sync" not in prompt
+    (pair,) = [b for _, b in kernels(plain(os.path.join(CSRC, "gemm_tc_pair.cu")))]
+    epilogue = pair[pair.index("setmaxnreg.inc"):]
+    units = re.search(r"for \(uint32_t u = pair; u < a\.units([^;]*);", epilogue)
+    assert units.group(1) in ("", " && (PAIRED || ok)") and "if (!ok) break;" not in epilogue
+    for body in (prompt, pair):
+        end = body.rindex("__syncthreads();")
+        assert re.search(r"if \(abort_flag\b", body[end:]) and "_full[i]" in body[end:] or "&full[s]" in body[end:]
+    assert "a.status" not in pair[:pair.rindex("__syncthreads();")]
