@@ -51,4 +51,33 @@ __device__ __forceinline__ void split_h2(float x, float y, uint32_t* hi, uint32_
     *lo = pack_h2(x - __half2float(hx), y - __half2float(hy));
 }
 
+// Zero weights do not cancel an infinity or a NaN: in a tile that a row sees in part, the value product hands the row what later
+// tokens hold. The prompt kernels therefore look at what comes out, and a row with something that is not finite in it gets those
+// dimensions once more from the keys that it sees, in plain f32. One warp; row of q with q_dim values, weights relative to `ref` in
+// base 2, not normalised. Lane l returns dimensions d, d + 1 (x, y) and d + 64, d + 65 (z, w; HD 128) with d = 2 l.
+__device__ __forceinline__ bool is_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+template <int HD>
+__device__ __noinline__ float4 attend_row(const float* q, uint32_t q_dim, float scale, const __half* K, const __half* V, size_t pitch,
+                                          uint32_t n, float ref) {
+    const uint32_t d = 2u * (threadIdx.x & 31u);
+    const auto q_at = [&](uint32_t i) { return i < q_dim ? q[i] * scale : 0.0f; };
+    const float4 x = make_float4(q_at(d), q_at(d + 1u), HD == 128 ? q_at(d + 64u) : 0.0f, HD == 128 ? q_at(d + 65u) : 0.0f);
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+    for (uint32_t t = 0; t < n; ++t, K += pitch, V += pitch) {
+        const float2 k0 = __half22float2(*reinterpret_cast<const __half2*>(K + d)), v0 = __half22float2(*reinterpret_cast<const __half2*>(V + d));
+        float2 k1 = make_float2(0.0f, 0.0f), v1 = k1;
+        if (HD == 128) {
+            k1 = __half22float2(*reinterpret_cast<const __half2*>(K + d + 64));
+            v1 = __half22float2(*reinterpret_cast<const __half2*>(V + d + 64));
+        }
+        float s = x.x * k0.x + x.y * k0.y + x.z * k1.x + x.w * k1.y;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        const float p = fast_exp2(s - ref);
+        acc.x += p * v0.x, acc.y += p * v0.y, acc.z += p * v1.x, acc.w += p * v1.y;
+    }
+    return acc;
+}
+
 }  // namespace attn_mma

@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(128, 2) prefill_varlen_kernel(const float* __r
     const uint32_t kv_end = shift + last_q + 1u;
     const uint32_t n_tiles = (kv_end + PF_TILE - 1) / PF_TILE;
     // K and V rows of a tile: f16 global -> shared by cp.async (rows past the end repeat the last visible row: they are
-    // masked below, and their bytes are finite)
+    // masked below)
     auto load_tile = [&](uint32_t tile, uint32_t buf) {
         const uint32_t base = tile * PF_TILE;
         __half* dK = pf_smem + (size_t)buf * 2 * TILE_ELEMS;
@@ -229,6 +229,30 @@ __global__ void __launch_bounds__(128, 2) prefill_varlen_kernel(const float* __r
                     mma16816(o[2 * nd], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], bb[0], bb[1]);
                     mma16816(o[2 * nd + 1], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], bb[2], bb[3]);
                 }
+            }
+        }
+    }
+    // ---- rows with something that is not finite: see attend_row()
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t row = h == 0 ? row_a : row_b;
+        float nan = 0.0f;
+#pragma unroll
+        for (int n = 0; n < NT; ++n) nan = fmaf(o[n][2 * h], 0.0f, fmaf(o[n][2 * h + 1], 0.0f, nan));
+        uint32_t again = __ballot_sync(0xffffffffu, row < q_len && !is_finite(nan));
+        while (again) {
+            const uint32_t gr = (__ffs(again) - 1u) >> 2, t = warp * 16u + gr + 8u * h;
+            again &= ~(0xfu << (4u * gr));
+            const float from = __shfl_sync(0xffffffffu, m_run[h], 4u * gr);
+            const float4 v = attend_row<HD>(Q + (q_row0 + t) * (CACHE ? pc.q_ld : q_heads * HD) + qh * (CACHE ? pc.q_dim : HD),
+                                            CACHE ? pc.q_dim : HD, inv_sqrt * LOG2E, K + kv_base, V + kv_base, kv_pitch, shift + r0 + t + 1u,
+                                            from == -INFINITY ? 0.0f : from);
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {  // dimensions 8 n + 2 t4 and + 1 come from lane 4 (n % 8) + t4
+                const uint32_t src = 4u * (n & 7) + t4;
+                const float x = __shfl_sync(0xffffffffu, n < 8 ? v.x : v.z, src), y = __shfl_sync(0xffffffffu, n < 8 ? v.y : v.w, src);
+                if (g == gr && !is_finite(o[n][2 * h])) o[n][2 * h] = x;
+                if (g == gr && !is_finite(o[n][2 * h + 1])) o[n][2 * h + 1] = y;
             }
         }
     }

@@ -8,16 +8,17 @@
 //
 // A row's reference is its running maximum, so its strongest key weighs exactly 1, and numerator and denominator share the
 // rounding of all others: relative error 0.96 to 1.01 of what the mma.sync form gives, for queries scaled by 1 to 8. (A reference
-// that moves only with every 2^8 of growth saves most of the rescaling, 264 against 273 us and 203 against 221 us at head size 64,
+// that moves only with every 2^8 of growth saves most of the rescaling, 9 of 273 us and 18 of 221 us at head size 64,
 // but its strongest weight is rounded: 1.05 times that error for flat scores, 3.3 times for peaked ones. Adding up the rounded
-// weights in the rows' registers took 285 us.)
+// weights in the rows' registers took 12 us more.)
 //
 // Warps 0..3 are the query rows, warp 4 loads K and V by TMA (two stages each), warp 5 issues the MMAs: S(j + 1) runs while the
 // rows work on S(j). A 128 x 128 tile of HD 128 is 24 MMAs (1600 cycles at the tensor rate) beside 1024 cycles of exponentials per
 // scheduler; one set of rows per SM leaves part of either idle. Four packed prompts of 509 to 2048 tokens, 32 / 8 heads of 128:
-// 273 us, against 438 us with mma.sync fragments (attention_prefill.cu), which stay for short segments.
+// 280 us, against 438 us with mma.sync fragments (attention_prefill.cu), which stay for short segments.
 // Rows behind a sequence's last key are whatever the cache holds there; the issuing warp clears them in the value tile, since
-// zero weights do not cancel a NaN.
+// zero weights do not cancel a NaN. Values of tokens that only some rows see are dealt with at the end (attend_row()): looking
+// through the one or two tiles in question beforehand, in shared memory or with a warp of its own, cost 8 to 22 us of 273, this 5.
 //
 // Every wait is bounded: a wait that runs out raises status bit 4; nothing waits any more from then on, copies in flight are drained
 // and tensor memory is freed.
@@ -31,7 +32,9 @@
 namespace {
 
 using namespace tc;
+using attn_mma::attend_row;
 using attn_mma::fast_exp2;
+using attn_mma::is_finite;
 using attn_mma::LOG2E;
 using attn_mma::pack_h2;
 using attn_mma::split_h2;
@@ -300,6 +303,32 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
 #pragma unroll
                 for (int i = 0; i < HD; ++i) o[i] = __uint_as_float(r[i]);
             }
+            float* stage = reinterpret_cast<float*>(smem) + warp * 32u * L::OUT_ROW;  // nothing reads or writes a tile any more
+            float* mine = stage + lane * L::OUT_ROW;
+            float nan[4] = {};
+#pragma unroll
+            for (int i = 0; i < HD; ++i) nan[i & 3] = fmaf(o[i], 0.0f, nan[i & 3]);
+            uint32_t again = __ballot_sync(0xffffffffu, row < q_len && !is_finite((nan[0] + nan[1]) + (nan[2] + nan[3])));
+            if (again) {
+#pragma unroll
+                for (int i = 0; i < HD; ++i) mine[i] = o[i];
+                __syncwarp();
+                const size_t pitch = CACHE ? HD : (size_t)pc.kv_heads * HD, at = (size_t)kv_row * pitch + kv_col;
+                for (; again; again &= again - 1u) {
+                    const uint32_t r = __ffs(again) - 1u, t = warp * 32u + r;
+                    const float from = __shfl_sync(0xffffffffu, ref, r);
+                    const float4 v = attend_row<HD>(pc.q + (q_row0 + t) * pc.q_ld + qh * pc.q_dim, pc.q_dim, pc.scale * LOG2E, pc.K + at,
+                                                    pc.V + at, pitch, shift + r0 + t + 1u, from == -INFINITY ? 0.0f : from);
+                    float* d = stage + r * L::OUT_ROW + 2u * lane;
+                    if (!is_finite(d[0])) d[0] = v.x;
+                    if (!is_finite(d[1])) d[1] = v.y;
+                    if (HD == 128 && !is_finite(d[64])) d[64] = v.z;
+                    if (HD == 128 && !is_finite(d[65])) d[65] = v.w;
+                }
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < HD; ++i) o[i] = mine[i];
+            }
             float inv = 1.0f / (l > 0.0f ? l : 1.0f);
             if (CACHE && pc.turn_back) {
                 const float4* t = reinterpret_cast<const float4*>(pc.turn_back + (q_row0 - r0 + min(row, q_len - 1u)) * (HD / 2));
@@ -314,11 +343,10 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
                 }
             }
             if (CACHE && pc.gate && row < q_len) inv *= m40_sigmoid(pc.gate[(q_row0 + tid) * pc.gate_ld + qh]);
-            // rows leave through shared memory, whole lines at a time: after the last value product nothing reads or writes a tile
-            float* stage = reinterpret_cast<float*>(smem) + warp * 32u * L::OUT_ROW;
+            // rows leave through shared memory, whole lines at a time
 #pragma unroll
             for (int i = 0; i < HD; i += 4)
-                *reinterpret_cast<float4*>(stage + lane * L::OUT_ROW + i) =
+                *reinterpret_cast<float4*>(mine + i) =
                     make_float4(o[i] * inv, o[i + 1] * inv, o[i + 2] * inv, o[i + 3] * inv);
             __syncwarp();
             constexpr uint32_t PER = HD / 4;  // float4 per row

@@ -175,3 +175,77 @@ def test_prompt_forms_are_equally_exact(nat, pkg, hd, pos, rows, scale):
     assert error[0] <= 1.1 * error[1] and error[1] <= 2.0 ** -11, error
     nat.lib.m40llm_kvcache_destroy(kv)
     nat.free_all()
+
+
+def poisoned(rng, L, kvh, hd, at):
+    """Values, and the same with infinities and a NaN at tokens at .. at + 5 of head 0; (token, dimension, what a row that sees it gets)."""
+    clean = rng.standard_normal((L, kvh, hd)).astype(np.float16)
+    bad, seen = clean.copy(), []
+    for token, d, value, then in ((at, 3, np.inf, np.inf), (at + 1, hd - 1, -np.inf, -np.inf), (at + 2, 10, np.nan, np.nan), (at + 5, 3, -np.inf, np.nan)):
+        bad[token, 0, d] = value
+        seen.append((token, d, then))
+    return clean, bad, seen
+
+
+def check_poisoned(got, plain, seen, pos, group):
+    """Untouched dimensions keep every bit; the touched ones are computed again for rows before the token, with weights that are not
+    rounded to f16 (2^-11 of a value, the largest of which is about 4)."""
+    want, touched = plain.copy(), sorted({d for _, d, _ in seen})
+    for token, d, then in seen:
+        want[max(token - pos, 0):, :group, d] = then
+    finite = np.isfinite(want)
+    assert np.array_equal(got[~finite], want[~finite], equal_nan=True)
+    assert np.abs(got[finite] - want[finite]).max() <= 4 * 2.0 ** -11
+    untouched = np.ones(want.shape, bool)
+    untouched[:, :group, touched] = False
+    assert np.array_equal(got[untouched], want[untouched])
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("pos,rows,at", [(0, 40, 17), (70, 50, 100), (0, 65, 30), (0, 200, 100), (30, 300, 250), (200, 129, 305)])
+def test_values_that_are_not_finite_stay_with_the_rows_that_see_them(nat, pkg, hd, pos, rows, at):
+    """A token whose value overflowed f16 changes the rows from it on and no earlier one; keys and values behind a sequence's last
+    token and of the neighbouring sequences may be anything."""
+    rng = np.random.default_rng(rows)
+    qh, kvh, L = 8, 2, pos + rows
+    K = rng.standard_normal((L, kvh, hd)).astype(np.float16)
+    clean, bad, seen = poisoned(rng, L, kvh, hd, at)
+    q = rng.standard_normal((rows, qh, hd)).astype(np.float32)
+    dq, do, ds = nat.buf(q), nat.buf(q.nbytes), nat.buf(np.array([0, rows, 1, pos], np.uint32))
+    r = pkg.native.StepRows(rows=rows, segments=1, max_segment_rows=rows, max_len=L, slot_mul=1, slot_add=0, seg=ds.ptr)
+    out = []
+    for values, around in ((clean, 0.0), (clean, np.nan), (bad, np.inf)):
+        kv = nat.kv_dense(L + 150, 3, kvh, hd)
+        junk = np.full((L + 150, kvh, hd), around, np.float16)
+        for slot in range(3):
+            nat.kv_fill(kv, slot, junk, junk)
+        nat.kv_fill(kv, 1, K, values)
+        assert nat.lib.m40llm_attention_step_rows_async(nat.ctx, kv, dq.ptr, qh, C.byref(r), do.ptr) == 0
+        nat.sync(1)
+        out.append(do.download(np.float32, q.shape))
+        nat.lib.m40llm_kvcache_destroy(kv)
+    assert np.isfinite(out[0]).all() and np.array_equal(out[0], out[1])
+    check_poisoned(out[2], out[0], seen, pos, qh // kvh)
+    nat.free_all()
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("pos,rows", [(20, 50), (0, 64), (100, 200)])
+def test_packed_values_beyond_f16_stay_with_the_rows_that_see_them(nat, hd, pos, rows):
+    rng = np.random.default_rng(rows + hd)
+    qh, kvh, lens = 4, 2, (rows, 30)
+    kv_lens, at = (pos + rows, 30), pos + rows // 2
+    q = rng.standard_normal((sum(lens), qh, hd)).astype(np.float32)
+    k = rng.standard_normal((sum(kv_lens), kvh, hd)).astype(np.float32)
+    clean, bad, seen = poisoned(rng, sum(kv_lens), kvh, hd, at)
+    offsets = [nat.buf(np.array(x, np.uint32)).ptr for x in ((0, rows), (0, kv_lens[0]), lens, kv_lens)]
+    out = []
+    for v in (clean, np.where(np.isinf(bad), np.sign(bad) * np.float32(1e6), bad)):
+        do = nat.buf(q.nbytes)
+        rc = nat.lib.m40llm_attention_prefill_f32_gqa_varlen(nat.ctx, nat.buf(q).ptr, nat.buf(k).ptr, nat.buf(v.astype(np.float32)).ptr, *offsets, 2,
+                                                             qh, kvh, hd, do.ptr)
+        assert rc == 0, rc
+        out.append(do.download(np.float32, q.shape))
+    assert np.array_equal(out[1][rows:], out[0][rows:])
+    check_poisoned(out[1][:rows], out[0][:rows], seen, pos, qh // kvh)
+    nat.free_all()
