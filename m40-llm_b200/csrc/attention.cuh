@@ -79,7 +79,8 @@ struct M40PrefillCall {
     const float2* turn_back;  // optional (cos, sin) [rows][hd / 2]: the output turns by the inverse of its value rotation
     const float* gate;        // optional, row pitch gate_ld: the output is multiplied by sigmoid(gate[row][head])
     const float* sink;        // optional [q_heads]: exp(sink) joins the denominator
-    uint32_t segments, max_segment_rows, rows;
+    const uint32_t* seg_host; // seg on the host, or null; max_len: bound of position + rows, or 0: what the kernel is chosen by
+    uint32_t segments, max_segment_rows, rows, max_len;
     uint32_t hd, q_heads, kv_heads, q_ld, q_dim, out_ld, v_dim, gate_ld;
     uint32_t slot_mul, slot_add, slots, max_seq_len;
     float scale;

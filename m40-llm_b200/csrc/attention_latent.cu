@@ -937,6 +937,7 @@ int run_expanded(M40llmCudaContext* ctx, const LatArgs& a, uint32_t w_dtype, con
     p.seg = seg;
     p.sink = a.sink;
     p.segments = 1;
+    p.seg_host = seg_host;
     p.max_segment_rows = seg_host[1];
     p.rows = a.rows;
     p.hd = hd;

@@ -12,7 +12,8 @@
 // accumulation (q split into f16 hi + lo so that the scores keep f32-level accuracy, P rounded to f16), and the
 // softmax is online, base 2, in registers. Every kv row is read once per 64 q rows instead of once per q row.
 //
-// Segments of more than 64 rows take the tcgen05 kernel of attention_prefill_tc.cu where alignment allows; this one serves the rest.
+// Calls with a segment of more than 64 rows may take the tcgen05 kernel of attention_prefill_tc.cu, where alignment allows and
+// prompt_cost.cuh says that it is the faster one; this one serves the rest.
 //
 // The same kernel also reads K and V straight from a dense f16 cache (CACHE): a prompt portion whose rows are already
 // appended attends everything its sequence holds, and the output may be turned back and gated before it is stored.
@@ -20,6 +21,7 @@
 #include "attention_mma.cuh"
 #include "attention_prefill_tc.cuh"
 #include "common.cuh"
+#include "prompt_cost.cuh"
 #include "stack_math.cuh"
 
 namespace {
@@ -306,17 +308,29 @@ bool prefill_configure(int device_id) {
     return true;
 }
 
+M40PromptCost prompt_cost(const M40llmCudaContext* ctx, const M40PrefillCall& c) {
+    M40PromptCost cost(c.hd, c.q_heads, (uint32_t)ctx->sm_count, c.max_segment_rows);
+    if (c.seg_host)
+        for (uint32_t i = 0; i < c.segments; ++i) cost.add(c.seg_host[4 * i + 1], c.seg_host[4 * i + 3]);
+    else
+        cost.add(c.max_segment_rows, c.max_len > c.max_segment_rows ? c.max_len - c.max_segment_rows : 0u, c.segments);
+    return cost;
+}
+
 }  // namespace
 
 int m40_attention_prefill(M40llmCudaContext* ctx, const M40PrefillCall& c) {
     if ((c.hd != 64 && c.hd != 128) || !c.K || !c.V || !c.seg) return 1;
     if (c.q_dim > c.hd || c.v_dim > c.hd || ((c.q_dim | c.v_dim | c.q_ld | c.out_ld) & 1u)) return 1;
     if ((((uintptr_t)c.q) & 7u) != 0u || (((uintptr_t)c.out) & 7u) != 0u) return 1;
-    M40PrefillTcArgs ta = {};
-    ta.c = c;
-    ta.status = ctx->d_status;
-    const int rc = m40_attention_prefill_tc(ctx, ctx->decode_stream, ta, (uint64_t)c.slots * c.kv_heads * c.max_seq_len);
-    if (rc <= 0) return rc;
+    const M40PromptCost cost = prompt_cost(ctx, c);
+    if (cost.tc_us() < cost.mma_us()) {
+        M40PrefillTcArgs ta = {};
+        ta.c = c;
+        ta.status = ctx->d_status;
+        const int rc = m40_attention_prefill_tc(ctx, ctx->decode_stream, ta, (uint64_t)c.slots * c.kv_heads * c.max_seq_len);
+        if (rc <= 0) return rc;
+    }
     if (!prefill_configure(ctx->device_id)) return -4;
     const PrefillCache pc = {c, ctx->d_status};
     const dim3 grid((c.max_segment_rows + PF_TILE - 1) / PF_TILE, c.q_heads, c.segments);
@@ -359,6 +373,8 @@ int m40llm_attention_step_rows_async(M40llmCudaContext* ctx, const M40llmKVCache
     p.slots = kv->max_batch_size;
     p.max_seq_len = kv->max_seq_len;
     p.scale = attn_inv_sqrt(kv->head_dim);
+    p.seg_host = rows->seg_host;
+    p.max_len = rows->max_len;
     return m40_attention_prefill(ctx, p);
 }
 
@@ -397,6 +413,8 @@ int m40llm_attention_prefill_f32_gqa_varlen_async(M40llmCudaContext* ctx, const 
         const uint64_t end = (uint64_t)lens[2 * batch_size + i] + kl;
         if (end > total_kv) total_kv = end;
     }
+    M40PromptCost cost(head_dim, q_heads, (uint32_t)ctx->sm_count, max_q);
+    for (uint32_t i = 0; rc == 0 && i < batch_size; ++i) cost.add(lens[i], lens[batch_size + i] - lens[i]);
     free(lens);
     if (rc != 0) return rc;
     // f16 copies of K and V in the prefill stream's scratch
@@ -428,7 +446,7 @@ int m40llm_attention_prefill_f32_gqa_varlen_async(M40llmCudaContext* ctx, const 
     ta.q_lens = d_q_lens;
     ta.kv_lens = d_kv_lens;
     ta.status = ctx->d_status;
-    rc = m40_attention_prefill_tc(ctx, s, ta, total_kv);
+    rc = cost.tc_us() < cost.mma_us() ? m40_attention_prefill_tc(ctx, s, ta, total_kv) : 1;
     if (rc <= 0) return rc;
     dim3 grid((max_q + PF_TILE - 1) / PF_TILE, q_heads, batch_size);
     const size_t smem = (size_t)2 * 2 * PF_TILE * head_dim * sizeof(__half);

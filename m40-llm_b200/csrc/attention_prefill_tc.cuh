@@ -2,7 +2,8 @@
 #pragma once
 #include "attention.cuh"
 
-// Segments shorter than this stay on the mma.sync kernel: they fill one of its 64-row tiles and half of a 128-row tile here.
+// Calls whose longest segment is shorter than this stay on the mma.sync kernel: it fills one of its 64-row tiles and half of a
+// 128-row tile here.
 constexpr uint32_t M40_PREFILL_TC_MIN_ROWS = 65;
 
 struct M40PrefillTcArgs {

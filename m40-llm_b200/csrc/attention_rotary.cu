@@ -395,6 +395,8 @@ extern "C" int m40llm_attention_rotary_async(M40llmCudaContext* ctx, M40llmKVCac
         p.gate_ld = c->ld;
         p.segments = r->segments;
         p.max_segment_rows = r->max_segment_rows;
+        p.seg_host = r->seg_host;
+        p.max_len = r->max_len;
         p.rows = r->rows;
         p.hd = p.q_dim = p.v_dim = kd;
         p.q_heads = c->q_heads;

@@ -119,7 +119,8 @@ def test_build_compressed_from_dense(nat, O, kvh, hd, R, bs, L):
 
 
 @pytest.mark.parametrize("hd", [64, 128])
-@pytest.mark.parametrize("pos,rows,scale", [(0, 65, 1.0), (33, 100, 1.0), (0, 128, 6.0), (127, 129, 6.0), (0, 700, 6.0), (900, 257, 1.0)])
+@pytest.mark.parametrize("pos,rows,scale", [(0, 65, 1.0), (33, 100, 1.0), (0, 128, 6.0), (127, 129, 6.0), (0, 700, 6.0), (900, 257, 1.0),
+                                            (895, 65, 1.0), (1033, 100, 6.0), (896, 128, 1.0), (1023, 129, 6.0), (1151, 1, 1.0)])
 def test_step_rows_over_cache(nat, pkg, hd, pos, rows, scale):
     """Prompt attention over the cache at the edges of its 128 x 128 tiles; with scale 6 a row's maximum grows past its reference
     from tile to tile. Probabilities are f16: an output is off by at most 2^-11 of the largest value."""
@@ -202,7 +203,8 @@ def check_poisoned(got, plain, seen, pos, group):
 
 
 @pytest.mark.parametrize("hd", [64, 128])
-@pytest.mark.parametrize("pos,rows,at", [(0, 40, 17), (70, 50, 100), (0, 65, 30), (0, 200, 100), (30, 300, 250), (200, 129, 305)])
+@pytest.mark.parametrize("pos,rows,at", [(0, 40, 17), (70, 50, 100), (0, 65, 30), (0, 200, 100), (30, 300, 250), (200, 129, 305),
+                                         (640, 65, 650), (768, 128, 800), (700, 129, 805)])
 def test_values_that_are_not_finite_stay_with_the_rows_that_see_them(nat, pkg, hd, pos, rows, at):
     """A token whose value overflowed f16 changes the rows from it on and no earlier one; keys and values behind a sequence's last
     token and of the neighbouring sequences may be anything."""

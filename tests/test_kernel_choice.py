@@ -1,0 +1,54 @@
+"""Rules that choose among kernels are host arithmetic: they are compiled by the host compiler and held against measured times, so
+that no call is slower than by the kernel that served all of them before. Runs without a GPU."""
+import os
+import subprocess
+
+import pytest
+
+import helpers
+
+CSRC = os.path.join(helpers.PKG_DIR, "csrc")
+
+
+@pytest.fixture(scope="module")
+def ask(tmp_path_factory):
+    """Compiles a body of C++ lines that print one number each, and returns those."""
+    def run(header, lines):
+        folder = tmp_path_factory.mktemp("choice")
+        src = folder / "ask.cpp"
+        src.write_text('#include <cstdio>\n#include "%s"\nint main() {\n%s\n}\n' % (os.path.join(CSRC, header), "\n".join(lines)))
+        exe = str(folder / "ask")
+        subprocess.run(["g++", "-O1", "-std=c++17", "-o", exe, str(src)], check=True)
+        return [float(x) for x in subprocess.run([exe], check=True, capture_output=True, text=True).stdout.split()]
+    return run
+
+
+# head size, q heads, kv heads, segments (rows, position, times), us of the tcgen05 and of the mma.sync kernel
+PROMPTS = [
+    (128, 32, 8, [(65, 0, 1)], 9.5, 7.6),
+    (128, 32, 8, [(65, 2048, 1)], 32.9, 59.0),
+    (128, 32, 8, [(256, 0, 1)], 11.8, 10.9),
+    (128, 32, 8, [(512, 0, 1)], 15.9, 25.7),
+    (128, 32, 8, [(65, 0, 32)], 65.1, 50.4),
+    (128, 32, 8, [(65, 1024, 32)], 153.0, 324.1),
+    (128, 32, 8, [(16, 0, 31), (300, 0, 1)], 72.5, 35.6),
+    (128, 32, 8, [(64, 3600, 31), (300, 3600, 1)], 411.9, 598.0),
+    (128, 8, 2, [(192, 0, 12)], 20.3, 13.2),
+    (128, 8, 2, [(1024, 0, 4)], 37.5, 65.1),
+    (64, 32, 4, [(128, 512, 1)], 13.3, 12.6),
+    (64, 32, 4, [(1024, 0, 2)], 50.0, 60.4),
+    (64, 32, 4, [(192, 256, 12)], 60.5, 46.2),
+    (64, 32, 4, [(192, 2048, 12)], 168.5, 199.7),
+    (64, 32, 4, [(64, 1024, 31), (300, 1024, 1)], 147.3, 113.3),
+]
+
+
+def cost(i, hd, qh, kvh, segs):
+    adds = " ".join(f"c{i}.add({r}, {p}, {n});" for r, p, n in segs)
+    return f"M40PromptCost c{i}({hd}, {qh}, 148, {max(r for r, _, _ in segs)}); {adds}"
+
+
+def test_prompt_kernels_are_chosen_as_measured(ask):
+    got = ask("prompt_cost.cuh", [cost(i, *p[:4]) + f' printf("%d\\n", c{i}.tc_us() < c{i}.mma_us());' for i, p in enumerate(PROMPTS)])
+    for p, tc in zip(PROMPTS, got):
+        assert (p[4] if tc else p[5]) <= min(1.05 * p[5], 1.25 * p[4]), p
