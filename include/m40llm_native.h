@@ -573,7 +573,10 @@ typedef struct {
 
 /* Causal attention of a step's rows over a dense f16 cache (head size 64 or 128) that already holds their keys and values: q and
  * out f32 [rows][q_heads][head_dim], softmax scaled by 1/sqrt(head_dim). For portions of prompts: a segment's rows share every
- * read of the cache. Returns 1 for a cache it does not take, -1 / -2 for bad arguments. Decode stream. */
+ * read of the cache. Returns 1 for a cache it does not take, M40LLM_ERR_UNSUPPORTED for a compressed one, -1 / -2 for bad arguments.
+ * With rows->seg_host it also returns 1, and does nothing, where m40llm_attention_last_token_f32_gqa_batched_async is the form to take:
+ * few rows over a long context, more than 16 q heads per kv head (computed in f32 there), or rows that do not fit the cache (rejected
+ * one by one there). Decode stream. */
 int m40llm_attention_step_rows_async(M40llmCudaContext* ctx, const M40llmKVCache* kv, const void* d_q_f32, uint32_t q_heads,
                                      const M40llmStepRows* rows, void* d_out_f32);
 

@@ -309,7 +309,7 @@ bool prefill_configure(int device_id) {
 }
 
 M40PromptCost prompt_cost(const M40llmCudaContext* ctx, const M40PrefillCall& c) {
-    M40PromptCost cost(c.hd, c.q_heads, (uint32_t)ctx->sm_count, c.max_segment_rows);
+    M40PromptCost cost(c.hd, c.q_heads, c.kv_heads, (uint32_t)ctx->sm_count, c.max_segment_rows);
     if (c.seg_host)
         for (uint32_t i = 0; i < c.segments; ++i) cost.add(c.seg_host[4 * i + 1], c.seg_host[4 * i + 3]);
     else
@@ -353,7 +353,15 @@ int m40llm_attention_step_rows_async(M40llmCudaContext* ctx, const M40llmKVCache
     if (rows->rows == 0 || rows->segments == 0 || rows->max_segment_rows == 0 || q_heads == 0 || kv->num_heads == 0 ||
         q_heads % kv->num_heads != 0)
         return -2;
-    if (kv->compressed || !kv->d_k || !kv->d_v) return 1;
+    if (kv->compressed) return M40LLM_ERR_UNSUPPORTED;
+    if (!kv->d_k || !kv->d_v) return 1;
+    if (rows->seg_host)
+        for (uint32_t i = 0; i < rows->segments; ++i) {
+            const uint32_t* s = rows->seg_host + 4 * i;
+            if ((uint64_t)s[0] + s[1] > rows->rows || (uint64_t)s[3] + s[1] > kv->max_seq_len ||
+                (uint64_t)s[2] * rows->slot_mul + rows->slot_add >= kv->max_batch_size)
+                return 1;
+        }
     if (m40_ensure_device(ctx) != 0) return -1;
     M40PrefillCall p = {};
     p.K = kv->d_k;
@@ -375,6 +383,12 @@ int m40llm_attention_step_rows_async(M40llmCudaContext* ctx, const M40llmKVCache
     p.scale = attn_inv_sqrt(kv->head_dim);
     p.seg_host = rows->seg_host;
     p.max_len = rows->max_len;
+    if (p.seg_host) {
+        // groups of more than 16 q heads decode in plain f32 (attention.cu), weights included
+        if (q_heads / kv->num_heads > 16u) return 1;
+        const M40PromptCost cost = prompt_cost(ctx, p);
+        if (cost.prompt_us() >= cost.decode_us()) return 1;
+    }
     return m40_attention_prefill(ctx, p);
 }
 
@@ -413,7 +427,7 @@ int m40llm_attention_prefill_f32_gqa_varlen_async(M40llmCudaContext* ctx, const 
         const uint64_t end = (uint64_t)lens[2 * batch_size + i] + kl;
         if (end > total_kv) total_kv = end;
     }
-    M40PromptCost cost(head_dim, q_heads, (uint32_t)ctx->sm_count, max_q);
+    M40PromptCost cost(head_dim, q_heads, kv_heads, (uint32_t)ctx->sm_count, max_q);
     for (uint32_t i = 0; rc == 0 && i < batch_size; ++i) cost.add(lens[i], lens[batch_size + i] - lens[i]);
     free(lens);
     if (rc != 0) return rc;

@@ -1,10 +1,7 @@
 // Prompt attention on tcgen05; see attention_prefill_tc.cu.
 #pragma once
 #include "attention.cuh"
-
-// Calls whose longest segment is shorter than this stay on the mma.sync kernel: it fills one of its 64-row tiles and half of a
-// 128-row tile here.
-constexpr uint32_t M40_PREFILL_TC_MIN_ROWS = 65;
+#include "prompt_cost.cuh"
 
 struct M40PrefillTcArgs {
     M40PrefillCall c;  // c.seg null: packed K, V [rows][kv_heads][hd] with the offsets and lengths below

@@ -8,9 +8,10 @@ namespace {
 // Portions from this many rows on compute the delta rule's low-rank decay as a projection of its own; below (and when
 // every row is a token of its own sequence) the mixer kernel does it.
 constexpr uint32_t LOW_RANK_ROWS = 2;
-// Llama layers: portions of a prompt attend in the prompt form (64 rows share a read of the cache) when every segment has this
-// many rows; a lone decode row among them would walk its whole context in one CTA. A prompt of 2000 tokens, 4 layers of 32 / 8
-// heads of 128 in passes of 256 rows: 10.5 ms against 13.1 ms in the decode form (145 us a layer and pass for attention).
+// Llama layers: portions of a prompt may attend in the prompt form (64 or 128 rows share a read of the cache) when every segment
+// has this many rows; a lone decode row among them would walk its whole context in one CTA. Whether they do is decided by
+// m40llm_attention_step_rows_async from rows, contexts and heads. A prompt of 2000 tokens, 4 layers of 32 / 8 heads of 128 in passes
+// of 256 rows: 9.9 ms against 13.1 ms in the decode form.
 constexpr uint32_t PROMPT_SEGMENT_ROWS = 16;
 bool prompt_portions(const M40llmStepRows& r) {
     if (!r.seg_host) return false;

@@ -251,3 +251,32 @@ def test_packed_values_beyond_f16_stay_with_the_rows_that_see_them(nat, hd, pos,
     assert np.array_equal(out[1][rows:], out[0][rows:])
     check_poisoned(out[1][:rows], out[0][:rows], seen, pos, qh // kvh)
     nat.free_all()
+
+
+def test_step_rows_leaves_to_the_decode_form_what_is_its(nat, pkg):
+    """With the segments on the host: few rows over a long context, groups whose decode kernel keeps the weights in f32, and rows that
+    do not fit the cache are handed back before anything is written; a compressed cache is refused."""
+    def call(kv, hd, qh, segs):
+        rows = sum(n for _, n, _ in segs)
+        flat = np.array([x for i, (s, n, p) in enumerate(segs) for x in (sum(m for _, m, _ in segs[:i]), n, s, p)], np.uint32)
+        q, out = nat.buf(np.ones((rows, qh, hd), np.float32)), nat.buf(np.full((rows, qh, hd), 9.0, np.float32))
+        r = pkg.native.StepRows(rows=rows, segments=len(segs), max_segment_rows=max(n for _, n, _ in segs), max_len=max(n + p for _, n, p in segs),
+                                slot_mul=1, slot_add=0, seg=nat.buf(flat).ptr, seg_host=flat.ctypes.data)
+        rc = nat.lib.m40llm_attention_step_rows_async(nat.ctx, kv, q.ptr, qh, C.byref(r), out.ptr)
+        nat.sync(1)
+        return rc, bool((out.download(np.float32, (rows, qh, hd)) == 9.0).all())
+
+    kv = nat.kv_dense(8300, 2, 4, 64)
+    assert call(kv, 64, 32, [(0, 256, 300)]) == (0, False) and call(kv, 64, 32, [(0, 16, 0), (1, 40, 60)]) == (0, False)
+    assert call(kv, 64, 32, [(1, 16, 8000)]) == (1, True)
+    assert call(kv, 64, 32, [(1, 256, 8045)]) == (1, True)
+    assert call(kv, 64, 32, [(0, 64, 0), (2, 64, 0)]) == (1, True)
+    wide = nat.kv_dense(600, 1, 1, 64)
+    assert call(wide, 64, 16, [(0, 256, 0)]) == (0, False) and call(wide, 64, 32, [(0, 256, 0)]) == (1, True)
+    compressed = nat.kv_compressed(600, 1, 4, 64, 64, 16, 4)
+    assert call(compressed, 64, 32, [(0, 256, 0)]) == (pkg.native.ERR_UNSUPPORTED, True)
+    st = np.zeros(1, np.uint32)
+    assert nat.lib.m40llm_context_take_device_status(nat.ctx, st.ctypes.data) == 0 and st[0] == 0
+    for c in (kv, wide, compressed):
+        nat.lib.m40llm_kvcache_destroy(c)
+    nat.free_all()

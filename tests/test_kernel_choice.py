@@ -45,10 +45,38 @@ PROMPTS = [
 
 def cost(i, hd, qh, kvh, segs):
     adds = " ".join(f"c{i}.add({r}, {p}, {n});" for r, p, n in segs)
-    return f"M40PromptCost c{i}({hd}, {qh}, 148, {max(r for r, _, _ in segs)}); {adds}"
+    return f"M40PromptCost c{i}({hd}, {qh}, {kvh}, 148, {max(r for r, _, _ in segs)}); {adds}"
 
 
 def test_prompt_kernels_are_chosen_as_measured(ask):
     got = ask("prompt_cost.cuh", [cost(i, *p[:4]) + f' printf("%d\\n", c{i}.tc_us() < c{i}.mma_us());' for i, p in enumerate(PROMPTS)])
     for p, tc in zip(PROMPTS, got):
         assert (p[4] if tc else p[5]) <= min(1.05 * p[5], 1.25 * p[4]), p
+
+
+# the same, us of the faster prompt kernel and of the decode form (a row reads its own context)
+PORTIONS = [
+    (128, 32, 8, [(16, 0, 1)], 5.7, 10.2),
+    (128, 32, 8, [(16, 1024, 1)], 31.3, 24.5),
+    (128, 32, 8, [(16, 8192, 1)], 209.9, 70.6),
+    (128, 32, 8, [(32, 2048, 2)], 56.8, 80.8),
+    (128, 32, 8, [(64, 8192, 1)], 210.0, 239.3),
+    (128, 32, 8, [(256, 8192, 1)], 106.0, 940.7),
+    (128, 16, 2, [(48, 4096, 1)], 107.8, 38.8),
+    (128, 16, 2, [(65, 8192, 1)], 102.0, 75.3),
+    (128, 16, 2, [(16, 2048, 12)], 88.0, 69.5),
+    (128, 16, 2, [(256, 2048, 2)], 34.7, 168.4),
+    (64, 32, 4, [(16, 8192, 1)], 113.6, 26.3),
+    (64, 32, 4, [(64, 4096, 1)], 58.9, 45.6),
+    (64, 32, 4, [(32, 512, 4)], 11.3, 29.7),
+    (64, 32, 4, [(128, 4096, 4)], 45.5, 288.3),
+    (64, 8, 8, [(24, 8192, 2)], 112.7, 93.7),
+    (64, 8, 8, [(24, 1024, 12)], 18.4, 100.8),
+]
+
+
+def test_portions_of_prompts_take_the_form_that_was_faster(ask):
+    got = ask("prompt_cost.cuh", [cost(i, *p[:4]) + f' printf("%d\\n", c{i}.prompt_us() < c{i}.decode_us());' for i, p in enumerate(PORTIONS)])
+    for p, prompt in zip(PORTIONS, got):
+        assert (p[4] if prompt else p[5]) <= 1.05 * p[5], p
+    assert sum(got) >= 7  # and those that gain much do take the prompt form
