@@ -600,16 +600,15 @@ int m40_gemm_tc_f16(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind
     ks = (a.kblocks_total + a.kblocks_per_split - 1) / a.kblocks_per_split;
     // Many rows go to the CTA-pair kernel, which finishes the result itself unless K is split.
     M40PairPlan plan = {};
-    const bool gate_up_pairs = mode == 1 && problems == 2 && N[0] == N[1];
-    const bool finishes = !rope && (gate_up_pairs || (problems == 1 && mode == 0));
+    const bool gate_up = mode == 1 && problems == 2 && N[0] == N[1], one = !rope && problems == 1 && mode == 0;
     const bool pairs = (uint32_t)M >= PAIR_MIN_ROWS;
-    if (pairs && !m40_pair_plan(ctx, (uint32_t)M, a.kblocks_total, (uint32_t)problems, N, gate_up_pairs, !finishes, &plan)) return -2;
+    if (pairs && !m40_pair_plan(ctx, (uint32_t)M, a.kblocks_total, (uint32_t)problems, N, gate_up, !one, &plan)) return -2;
     if (pairs) {
         ks = plan.k_splits;
         a.n_total = plan.tiles * M40_PAIR_ROWS;
         for (int p = 0; p < 4; ++p) a.tile_begin[p] = plan.tile_begin[p] * (M40_PAIR_ROWS / BLOCK_N);
     }
-    const bool direct = pairs ? finishes && ks == 1 : ext && ks == 1 && !rope && problems == 1 && mode == 0;
+    const bool direct = pairs ? plan.paired || (one && ks == 1) : ext && ks == 1 && one;
 
     // scratch: [hi][lo] activation copies, then the partials
     const size_t act_elems = (size_t)M * K;
@@ -625,7 +624,7 @@ int m40_gemm_tc_f16(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind
     CUtensorMap mW[3], mXh, mXl;
     for (int p = 0; p < 3; ++p) {
         const int q = p < problems ? p : 0;
-        const uint32_t w_box = pairs && gate_up_pairs ? BLOCK_N / 2 : BLOCK_N;
+        const uint32_t w_box = pairs && plan.paired ? BLOCK_N / 2 : BLOCK_N;
         if (!make_map_f16(&mW[p], W[q], (uint64_t)N[q], (uint64_t)K, w_box, bf16)) return -2;
     }
     const uint32_t x_box = pairs ? plan.width / 2 : M_pad;
@@ -684,7 +683,6 @@ int m40_gemm_tc_f16(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind
         c.kblocks = a.kblocks_total;
         c.problems = (uint32_t)problems;
         c.fmt_bits = a.fmt_bits;
-        c.paired = gate_up_pairs ? 1u : 0u;
         c.partial = direct ? nullptr : a.partial;
         c.out = a.out;
         c.n_out = a.n_out;

@@ -10,7 +10,7 @@
 // rows are 64 gate rows over 64 up rows, and the two warps that hold a gate row and its up row trade halves of their columns
 // through shared memory. (Two accumulators of half the width in place of that need no trade, but an MMA of 128 columns takes as
 // long as its weight operand does: 1600 cycles per 64-deep step against 1100.)
-// Work units (weight tile x row tile x K split) are dealt round robin over the resident pairs; m40_pair_plan() picks the
+// Work units (weight tile x row tile x K split) are dealt round robin over the resident pairs; gemm_tc_pair_plan.cuh picks the
 // width and the split.
 //
 // Precision: the tensor core cuts its f32 sums off where f32 multiply-adds round, so that the error grows with the number of
@@ -393,45 +393,9 @@ uint32_t resident_pairs(const M40llmCudaContext* ctx) {
 
 }  // namespace
 
-bool m40_pair_plan(const M40llmCudaContext* ctx, uint32_t M, uint32_t kblocks, uint32_t problems, const int* N, bool paired,
+bool m40_pair_plan(const M40llmCudaContext* ctx, uint32_t M, uint32_t kblocks, uint32_t problems, const int* N, bool gate_up,
                    bool partial_only, M40PairPlan* plan) {
-    const uint32_t pairs = resident_pairs(ctx);
-    if (pairs == 0 || M == 0) return false;
-    uint32_t tiles = 0, n_sum = 0;
-    for (uint32_t p = 0; p < (paired ? 1u : problems); ++p) {
-        plan->tile_begin[p] = tiles;
-        const uint32_t rows = paired ? M40_PAIR_ROWS / 2 : M40_PAIR_ROWS;
-        tiles += ((uint32_t)N[p] + rows - 1) / rows;
-        n_sum += (uint32_t)N[p];
-    }
-    for (uint32_t p = paired ? 1u : problems; p < 4; ++p) plan->tile_begin[p] = tiles;
-    plan->tiles = tiles;
-    // Cycles of a call: full waves of units, each kb_per_split k-blocks long, paced by the MMAs (4 cycles per activation row and
-    // k-block, and at least the 90 cycles per MMA that its weight operand takes) or by L2 (about 50 bytes a cycle and SM); then
-    // the last tile's stores, and, where partial sums are needed, their way to L2 and back.
-    double best = 0.0;
-    for (uint32_t width = 32; width <= 256u; width += 32) {
-        const uint32_t m_tiles = (M + width - 1) / width;
-        if (m_tiles > 1 && ((M + m_tiles - 1) / m_tiles + 31) / 32 * 32 != width) continue;  // a narrower tile gives as few
-        if (m_tiles == 1 && width >= M + 32) continue;
-        const double mma = 4.0 * width > 720.0 ? 4.0 * width : 720.0, load = (A_BYTES + 128.0 * width) / 50.0;
-        for (uint32_t ks = 1; ks <= (paired ? 1u : 16u) && (ks == 1 || kblocks / ks >= 4); ++ks) {
-            const uint32_t per = (kblocks + ks - 1) / ks, real = (kblocks + per - 1) / per;
-            if (real != ks) continue;
-            const uint64_t units = (uint64_t)tiles * m_tiles * ks;
-            const double waves = (double)((units + pairs - 1) / pairs);
-            double cost = waves * per * (mma > load ? mma : load) + 2000.0 + 12.0 * width;
-            if (ks > 1 || partial_only) cost += 5000.0 + (double)ks * M * n_sum * 8.0 / (2.0 * pairs * 25.0);
-            if (best == 0.0 || cost < best) {
-                best = cost;
-                plan->width = width;
-                plan->m_tiles = m_tiles;
-                plan->k_splits = ks;
-                plan->kb_per_split = per;
-            }
-        }
-    }
-    return best > 0.0;
+    return m40_pair_cut_best(resident_pairs(ctx), M, kblocks, problems, N, gate_up, partial_only, plan);
 }
 
 int m40_pair_launch(M40llmCudaContext* ctx, cudaStream_t s, const M40PairCall& c, const M40PairPlan& p) {
@@ -450,7 +414,7 @@ int m40_pair_launch(M40llmCudaContext* ctx, cudaStream_t s, const M40PairCall& c
     a.width = p.width;
     a.tiles = p.tiles;
     for (int i = 0; i < 4; ++i) a.tile_begin[i] = p.tile_begin[i];
-    a.problems = c.paired ? 1u : c.problems;
+    a.problems = p.paired ? 1u : c.problems;
     a.fmt_bits = c.fmt_bits;
     a.partial = c.partial;
     a.out = c.out;
@@ -462,8 +426,8 @@ int m40_pair_launch(M40llmCudaContext* ctx, cudaStream_t s, const M40PairCall& c
     a.act = c.act;
     a.tail = c.tail;
     cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = pair_config(attr, 2u * (a.units < pairs ? a.units : pairs), c.paired != 0u, s);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, c.paired ? gemm_tc_pair_kernel<true> : gemm_tc_pair_kernel<false>, c.w[0], c.w[1],
+    const cudaLaunchConfig_t cfg = pair_config(attr, 2u * (a.units < pairs ? a.units : pairs), p.paired, s);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, p.paired ? gemm_tc_pair_kernel<true> : gemm_tc_pair_kernel<false>, c.w[0], c.w[1],
                                              c.w[2], c.xh, c.xl, a);
     M40_COUNT_LAUNCH(ctx);
     return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -2;

@@ -102,6 +102,21 @@ def test_linear_many_rows(nat, rows, n, k, wdt):
           2 * tol, "gated")
 
 
+@pytest.mark.parametrize("rows,n,k,gated", [(300, 9570, 2120, 0), (257, 5000, 6360, 0), (400, 9570, 1160, 1), (257, 9570, 712, 1), (1030, 1000, 4040, 1),
+                                            (511, 640, 2120, 1)])
+def test_linear_many_units(nat, rows, n, k, gated):
+    """More units of work than CTA pairs, so that a pair carries its ring, accumulators and trades from one unit to the next: whole K
+    (odd numbers of partial sums, a remainder), split K, gate and up in shared tiles and as two problems. Limits as above."""
+    rng = np.random.default_rng(rows + n + k)
+    x, w = rng.standard_normal((rows, k)).astype(np.float32), rounded(rng, N.DT_BF16, n, k)
+    y = x.astype(np.float64) @ w.T.astype(np.float64)
+    if not gated:
+        close(run_linear(nat, x, w, N.DT_BF16, rows), y, 8e-6)
+        return
+    w2 = rounded(rng, N.DT_BF16, n, k)
+    close(run_linear(nat, x, w, N.DT_BF16, rows, w2=w2, act=N.ACT_SILU), y * S.sigmoid(y) * (x.astype(np.float64) @ w2.T.astype(np.float64)), 1.6e-5)
+
+
 @pytest.mark.parametrize("rows", [1, 5, 64, 300])
 def test_linear_row_pitch(nat, rows):
     rng = np.random.default_rng(rows)

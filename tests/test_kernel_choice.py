@@ -80,3 +80,16 @@ def test_portions_of_prompts_take_the_form_that_was_faster(ask):
     for p, prompt in zip(PORTIONS, got):
         assert (p[4] if prompt else p[5]) <= 1.05 * p[5], p
     assert sum(got) >= 7  # and those that gain much do take the prompt form
+
+
+# rows, outputs of gate and of up, K: us of shared tiles, of two problems with K splits
+GATE_UP = [(200, 640, 8192, 73.1, 25.0), (160, 4096, 2048, 28.4, 22.0), (129, 64, 2048, 23.0, 12.3), (512, 1408, 2048, 28.4, 23.7), (300, 2048, 8192, 86.8, 51.4),
+           (256, 8192, 64, 13.8, 27.3), (129, 8192, 256, 12.4, 21.2), (2048, 8192, 64, 59.3, 139.6), (1030, 4096, 2048, 81.9, 86.2)]
+
+
+def test_gate_up_calls_are_cut_as_measured(ask):
+    got = ask("gemm_tc_pair_plan.cuh", ["M40PairPlan p;"] + [
+        f'{{ const int n[2] = {{{n}, {n}}}; m40_pair_cut_best(74, {m}, {(k + 63) // 64}, 2, n, true, false, &p); printf("%d\\n", p.paired); }}'
+        for m, n, k, _, _ in GATE_UP])
+    for case, shared in zip(GATE_UP, got):
+        assert (case[3] if shared else case[4]) == min(case[3:]), case
