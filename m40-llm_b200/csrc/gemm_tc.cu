@@ -18,7 +18,7 @@
 // epilogue (bias, residual, or SiLU(gate)*up).
 //
 // Whenever one problem needs no K split, the epilogue warps apply bias, post norm, residual and soft cap themselves and store
-// the result: no partials, no second kernel. More than 128 rows go to the CTA-pair kernel (gemm_tc_pair.cu).
+// the result: no partials, no second kernel. Most calls of more than 128 rows go to the CTA-pair kernel (gemm_tc_pair.cu).
 //
 // Every wait is bounded: a wait that runs out sets bit 2 of the context's device status word, the
 // CTA stops issuing work, frees its TMEM and returns.
@@ -33,11 +33,15 @@ namespace {
 
 using namespace tc;
 
-// From here on a tile of gemm_tc_f16_kernel cannot stack the hi and lo rows in one MMA, and the CTA-pair kernel is faster
-// (111 against 155 + 21 us with the epilogue kernel at 2 x 14336 x 4096 gate | up weights and 256 rows, 638 against
-// 1005 us at 2048 rows). At 128 rows it is
-// slower: 42 + 7 against 35 + 9 us at 4096 x 14336, 21 + 7 against 18 + 8 at 4096 x 4096.
+// Rows at which gemm_tc_f16_kernel cannot stack the hi and lo rows in one MMA any more. Below, the CTA-pair kernel is slower
+// (128 rows: 42 + 7 against 35 + 9 us at 4096 x 14336, 21 + 7 against 18 + 8 at 4096 x 4096); from here on it is mostly faster
+// (gate | up of 2 x 14336 x 4096: 111 against 155 + 21 us at 256 rows, 638 against 1005 at 2048).
 constexpr uint32_t PAIR_MIN_ROWS = 129;
+// What stays on gemm_tc_f16_kernel beyond: calls whose K it splits (so that hi and lo may share an accumulator: the sums are short),
+// up to 144 rows, where two CTAs fit an SM (129 rows, 8192 x 2048: 19.1 against 21.2 us with the pairs, 1408 x 2048: 12.6 against 14.3),
+// and narrow gate | up calls of up to 208 rows with many splits (2 x 640 x 8192: 22 against 24.5 us at 176 rows, 23.4 against 25 at
+// 200). Of 374 measured calls of 129 to 256 rows, 64 to 8192 outputs and K of 64 to 8192 the choice was at most 19 % off the better one.
+constexpr uint32_t SINGLE_MAX_ROWS = 144, SINGLE_GATED_ROWS = 208, SINGLE_GATED_SPLITS = 6;
 
 struct TcArgs {
     float* partial;            // [k_splits][M][n_total]
@@ -80,10 +84,11 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_f16_kernel(const __grid_consta
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * a.stages + 1);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
-    // hi and lo activation tiles are contiguous rows of one operand: a single MMA of width 2 * M_pad takes the weight tile
-    // against both (the weight operand passes the tensor core once); the two halves of the accumulator are added in the
-    // epilogue.
-    const uint32_t acc_cols = 2u * a.M_pad;
+    // hi and lo activation tiles are contiguous rows of one operand: up to M_pad = 128 a single MMA of width 2 * M_pad takes the
+    // weight tile against both (the weight operand passes the tensor core once); the two halves of the accumulator are added in
+    // the epilogue. Wider tiles add the two products in one accumulator.
+    const bool stacked = a.M_pad <= 128u;
+    const uint32_t acc_cols = stacked ? 2u * a.M_pad : a.M_pad;
     uint32_t tmem_cols = 32;
     while (tmem_cols < acc_cols) tmem_cols <<= 1;
 
@@ -151,8 +156,11 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_f16_kernel(const __grid_consta
             const uint32_t sb = sa + a_bytes;
             if (elect_one()) {
 #pragma unroll
-                for (uint32_t k = 0; k < BLOCK_K / UMMA_K; ++k)
-                    umma_f16(tmem_base, make_desc_sw128(sa + k * UMMA_K * 2), make_desc_sw128(sb + k * UMMA_K * 2), idesc, i | k);
+                for (uint32_t k = 0; k < BLOCK_K / UMMA_K; ++k) {
+                    const uint64_t da = make_desc_sw128(sa + k * UMMA_K * 2);
+                    umma_f16(tmem_base, da, make_desc_sw128(sb + k * UMMA_K * 2), idesc, i | k);
+                    if (!stacked) umma_f16(tmem_base, da, make_desc_sw128(sb + b_bytes + k * UMMA_K * 2), idesc, 1u);
+                }
                 umma_commit(&empty[s]);                 // frees the stage once these MMAs have read it
                 if (i + 1 == n_kb) umma_commit(accum);  // accumulator complete
             }
@@ -182,10 +190,12 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_f16_kernel(const __grid_consta
             float v[8];
             if (ok) {
                 tmem_ld8(tmem_base + ((lane_group * 32u) << 16) + c, v);
-                float w[8];
-                tmem_ld8(tmem_base + ((lane_group * 32u) << 16) + a.M_pad + c, w);
+                if (stacked) {
+                    float w[8];
+                    tmem_ld8(tmem_base + ((lane_group * 32u) << 16) + a.M_pad + c, w);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] += w[j];
+                    for (int j = 0; j < 8; ++j) v[j] += w[j];
+                }
             } else {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) v[j] = 0.0f;
@@ -598,10 +608,11 @@ int m40_gemm_tc_f16(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind
     if (ks > 16) ks = 16;
     a.kblocks_per_split = (a.kblocks_total + ks - 1) / ks;
     ks = (a.kblocks_total + a.kblocks_per_split - 1) / a.kblocks_per_split;
-    // Many rows go to the CTA-pair kernel, which finishes the result itself unless K is split.
+    // Many rows go to the CTA-pair kernel, which finishes the result itself unless K is split (see PAIR_MIN_ROWS).
     M40PairPlan plan = {};
     const bool gate_up = mode == 1 && problems == 2 && N[0] == N[1], one = !rope && problems == 1 && mode == 0;
-    const bool pairs = (uint32_t)M >= PAIR_MIN_ROWS;
+    const bool single = ks > 1 && ((uint32_t)M <= SINGLE_MAX_ROWS || (gate_up && (uint32_t)M <= SINGLE_GATED_ROWS && ks >= SINGLE_GATED_SPLITS));
+    const bool pairs = (uint32_t)M >= PAIR_MIN_ROWS && !single;
     if (pairs && !m40_pair_plan(ctx, (uint32_t)M, a.kblocks_total, (uint32_t)problems, N, gate_up, !one, &plan)) return -2;
     if (pairs) {
         ks = plan.k_splits;

@@ -117,6 +117,19 @@ def test_linear_many_units(nat, rows, n, k, gated):
     close(run_linear(nat, x, w, N.DT_BF16, rows, w2=w2, act=N.ACT_SILU), y * S.sigmoid(y) * (x.astype(np.float64) @ w2.T.astype(np.float64)), 1.6e-5)
 
 
+@pytest.mark.parametrize("rows", [129, 143, 144, 145, 208, 209])
+@pytest.mark.parametrize("n,k,gated", [(640, 4096, 1), (641, 2056, 0), (130, 6000, 1)])
+def test_linear_one_cta_beyond_128_rows(nat, rows, n, k, gated):
+    """Both sides of the rows at which calls with split K pass from one CTA per tile to pairs; limits as above."""
+    rng = np.random.default_rng(rows + n + k)
+    x, w, w2 = rng.standard_normal((rows, k)).astype(np.float32), rounded(rng, N.DT_F16, n, k), rounded(rng, N.DT_F16, n, k)
+    y, bias = x.astype(np.float64) @ w.T.astype(np.float64), rng.standard_normal(n)
+    if gated:
+        close(run_linear(nat, x, w, N.DT_F16, rows, w2=w2, act=N.ACT_SILU), y * S.sigmoid(y) * (x.astype(np.float64) @ w2.T.astype(np.float64)), 4e-6)
+    else:
+        close(run_linear(nat, x, w, N.DT_F16, rows, bias=bias), y + bias, 2e-6)
+
+
 @pytest.mark.parametrize("rows", [1, 5, 64, 300])
 def test_linear_row_pitch(nat, rows):
     rng = np.random.default_rng(rows)
