@@ -338,7 +338,7 @@ int launch(M40llmCudaContext* ctx, const M40LatArgs& a) {
 bool m40_latent_tc_takes(const M40LatArgs& a) {
     const void* w[1] = {a.C};
     return a.rank % 128 == 0 && a.rank <= 512 && (uint64_t)a.slots * a.max_seq_len < 0x7fffff00ull &&
-           m40_gemm_tc_supported(2, (int)a.rank, 1, w);
+           m40_gemm_tc_supported(nullptr, 2, (int)a.rank, 1, w);
 }
 
 int m40_latent_tc(M40llmCudaContext* ctx, const M40LatArgs& a) { return a.heads > 16 ? launch<32>(ctx, a) : launch<16>(ctx, a); }

@@ -22,6 +22,8 @@
 //
 // Every wait is bounded: a wait that runs out raises status bit 4; nothing waits any more from then on, copies in flight are drained
 // and tensor memory is freed.
+#include <atomic>
+
 #include "attention.cuh"
 #include "attention_mma.cuh"
 #include "attention_prefill_tc.cuh"
@@ -373,13 +375,14 @@ __global__ void __launch_bounds__(192, 1) prefill_tc_kernel(const __grid_constan
 
 template <int HD, bool CACHE>
 int launch(M40llmCudaContext* ctx, cudaStream_t s, const CUtensorMap& mk, const CUtensorMap& mv, const M40PrefillTcArgs& a) {
-    static unsigned long long configured = 0ull;
+    // contexts on several threads may set it at the same time: setting it twice is harmless, losing another device's bit is not
+    static std::atomic<unsigned long long> configured{0ull};
     const unsigned long long bit = 1ull << (ctx->device_id & 63);
-    if (!(configured & bit)) {
+    if (!(configured.load(std::memory_order_acquire) & bit)) {
         if (cudaFuncSetAttribute(prefill_tc_kernel<HD, CACHE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem<HD>::BYTES) !=
             cudaSuccess)
             return -4;
-        configured |= bit;
+        configured.fetch_or(bit, std::memory_order_release);
     }
     const dim3 grid((a.c.max_segment_rows + ROWS - 1) / ROWS, a.c.q_heads, a.c.segments);
     cudaError_t e;

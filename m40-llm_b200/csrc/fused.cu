@@ -99,7 +99,7 @@ extern "C" int m40llm_qkv_rmsnorm_rope_append_async(M40llmCudaContext* ctx, M40l
     const void* wp[3] = {d_wq_f16, d_wk_f16, d_wv_f16};
     if (rc == 0) {
         // projections done above
-    } else if ((int)rows >= m40_tc_min_rows() && m40_gemm_tc_supported((int)rows, (int)hidden, 3, wp) && hidden % 4 == 0) {
+    } else if ((int)rows >= m40_tc_min_rows() && m40_gemm_tc_supported(ctx, (int)rows, (int)hidden, 3, wp) && hidden % 4 == 0) {
         // one tensor-core launch over Wq | Wk | Wv; the norm rides on the f16 split of the activations
         const __half* w[3] = {(const __half*)d_wq_f16, (const __half*)d_wk_f16, (const __half*)d_wv_f16};
         const int n[3] = {(int)QD, (int)KD, (int)KD};

@@ -495,7 +495,7 @@ int m40_tc_min_rows() {
 int m40_gemm_dispatch_f16(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind, const float* A,
                           const __half* W, float* C, int M, int N, int K, const float* bias, const float* residual) {
     const void* wp[1] = {W};
-    if (M >= m40_tc_min_rows() && m40_gemm_tc_supported(M, K, 1, wp)) {
+    if (M >= m40_tc_min_rows() && m40_gemm_tc_supported(ctx, M, K, 1, wp)) {
         const __half* w[1] = {W};
         const int n[1] = {N};
         float* o[1] = {C};
@@ -605,7 +605,7 @@ int m40_ffn_swiglu(M40llmCudaContext* ctx, uint32_t stream_kind, const void* d_x
                                      (int)hidden, (int)ffn, (const float*)d_residual);
     }
     const void* wp[2] = {d_wg, d_wu};
-    if ((int)rows >= m40_tc_min_rows() && m40_gemm_tc_supported((int)rows, (int)hidden, 2, wp)) {
+    if ((int)rows >= m40_tc_min_rows() && m40_gemm_tc_supported(ctx, (int)rows, (int)hidden, 2, wp)) {
         const __half* w[2] = {(const __half*)d_wg, (const __half*)d_wu};
         const int n[2] = {(int)ffn, (int)ffn};
         float* o[2] = {(float*)d_hid, nullptr};

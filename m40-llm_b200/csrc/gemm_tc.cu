@@ -40,7 +40,7 @@ constexpr uint32_t PAIR_MIN_ROWS = 129;
 // What stays on gemm_tc_f16_kernel beyond: calls whose K it splits (so that hi and lo may share an accumulator: the sums are short),
 // up to 144 rows, where two CTAs fit an SM (129 rows, 8192 x 2048: 19.1 against 21.2 us with the pairs, 1408 x 2048: 12.6 against 14.3),
 // and narrow gate | up calls of up to 208 rows with many splits (2 x 640 x 8192: 22 against 24.5 us at 176 rows, 23.4 against 25 at
-// 200). Of 374 measured calls of 129 to 256 rows, 64 to 8192 outputs and K of 64 to 8192 the choice was at most 19 % off the better one.
+// 200). Of 544 measured calls of 129 to 256 rows, 64 to 8192 outputs and K of 64 to 8192 the choice was at most 19 % off the better one.
 constexpr uint32_t SINGLE_MAX_ROWS = 144, SINGLE_GATED_ROWS = 208, SINGLE_GATED_SPLITS = 6;
 
 struct TcArgs {
@@ -559,8 +559,9 @@ int m40_split_activations(M40llmCudaContext* ctx, cudaStream_t s, const float* X
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-bool m40_gemm_tc_supported(int M, int K, int problems, const void* const* W) {
+bool m40_gemm_tc_supported(const M40llmCudaContext* ctx, int M, int K, int problems, const void* const* W) {
     if (M < 2 || M > 256 || K % 8 != 0 || K < BLOCK_K || problems < 1 || problems > 3) return false;
+    if ((uint32_t)M >= PAIR_MIN_ROWS && !m40_pair_available(ctx)) return false;
     for (int p = 0; p < problems; ++p)
         if ((((uintptr_t)W[p]) & 15u) != 0u) return false;
     return get_encode() != nullptr;

@@ -23,11 +23,11 @@ struct M40TcRopeAppend {
 // Tensor map of a row-major 16-bit matrix [rows][cols] for 128-byte-swizzled boxes of box_rows x 64, zeros out of bounds.
 bool m40_tc_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, bool bf16);
 
-// True when the tcgen05 path can take this problem set (2 <= M <= 256, K % 8 == 0, 16-byte aligned weights).
-bool m40_gemm_tc_supported(int M, int K, int problems, const void* const* W);
+// True when the tcgen05 path can take this problem set (2 <= M <= 256, K % 8 == 0, 16-byte aligned weights, CTA pairs on the device
+// for more than 128 rows; up to there ctx may be null).
+bool m40_gemm_tc_supported(const M40llmCudaContext* ctx, int M, int K, int problems, const void* const* W);
 
-// What a call does beyond the Llama layer's projections. With it M may exceed 256: the rows are then cut into blocks that
-// share one launch (grid.z).
+// What a call does beyond the Llama layer's projections. With it M may exceed 256.
 struct M40TcExt {
     int bf16;            // weights are bf16 and the activations are split into bf16 hi + lo (both MMA operands share a type)
     int ldx;             // row pitch of X in elements (0: K)

@@ -258,7 +258,7 @@ int launch(M40llmCudaContext* ctx, cudaStream_t s, dim3 grid, size_t smem, const
 
 bool m40_gemm_tc_grouped_supported(const void* w, uint32_t N, uint32_t K, uint32_t ldx, uint32_t group_k) {
     const void* wp[1] = {w};
-    return N > 0 && ldx % 8 == 0 && group_k % 8 == 0 && m40_gemm_tc_supported(2, (int)K, 1, wp);
+    return N > 0 && ldx % 8 == 0 && group_k % 8 == 0 && m40_gemm_tc_supported(nullptr, 2, (int)K, 1, wp);
 }
 
 int m40_gemm_tc_grouped(M40llmCudaContext* ctx, cudaStream_t s, const M40GroupedCall& c) {

@@ -21,6 +21,7 @@
 // Every wait is bounded: a wait that runs out winds down both CTAs (give_up()): they stop issuing work, raise bit 2 of the
 // device status word, wait for their copies in flight, free tensor memory and return. The barrier of two trading warps
 // (finish_gated()) has no bound of its own, so both come to it equally often whatever their waits gave.
+#include <atomic>
 #include <type_traits>
 
 #include "gemm_tc_pair.cuh"
@@ -349,12 +350,6 @@ __global__ void __launch_bounds__(384, 1) gemm_tc_pair_kernel(const __grid_const
     }
 }
 
-struct PairDevice {
-    int state;  // 0: not asked, 1: usable, 2: no pairs here
-    uint32_t pairs;
-};
-PairDevice g_device[64];
-
 cudaLaunchConfig_t pair_config(cudaLaunchAttribute* attr, uint32_t ctas, bool paired, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas);
@@ -372,26 +367,31 @@ cudaLaunchConfig_t pair_config(cudaLaunchAttribute* attr, uint32_t ctas, bool pa
     return cfg;
 }
 
+// CTA pairs that fit the device at once, 0 where it takes none. Contexts on several threads may ask at the same time: each finds out
+// for itself and all store the same. A query that fails is not remembered.
 uint32_t resident_pairs(const M40llmCudaContext* ctx) {
-    PairDevice& d = g_device[ctx->device_id & 63];
-    if (d.state == 0) {
-        int clusters = 0;
-        cudaLaunchAttribute attr[2];
-        cudaLaunchConfig_t cfg = pair_config(attr, 2, true, nullptr);
-        cfg.numAttrs = 1;
-        const bool usable =
-            cudaFuncSetAttribute(gemm_tc_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES + 1024) == cudaSuccess &&
-            cudaFuncSetAttribute(gemm_tc_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 RING_BYTES + 1024 + TRADE_BYTES) == cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&clusters, gemm_tc_pair_kernel<true>, &cfg) == cudaSuccess && clusters > 0;
-        if (!usable) cudaGetLastError();
-        d.pairs = usable ? (uint32_t)clusters : 0u;
-        d.state = usable ? 1 : 2;
+    static std::atomic<uint32_t> known[64];  // pairs + 1, per device
+    std::atomic<uint32_t>& slot = known[ctx->device_id & 63];
+    const uint32_t have = slot.load(std::memory_order_acquire);
+    if (have) return have - 1u;
+    int clusters = 0;
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = pair_config(attr, 2, true, nullptr);
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(gemm_tc_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES + 1024) != cudaSuccess ||
+        cudaFuncSetAttribute(gemm_tc_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES + 1024 + TRADE_BYTES) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, gemm_tc_pair_kernel<true>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
     }
-    return d.pairs;
+    slot.store((uint32_t)clusters + 1u, std::memory_order_release);
+    return (uint32_t)clusters;
 }
 
 }  // namespace
+
+bool m40_pair_available(const M40llmCudaContext* ctx) { return resident_pairs(ctx) > 0; }
 
 bool m40_pair_plan(const M40llmCudaContext* ctx, uint32_t M, uint32_t kblocks, uint32_t problems, const int* N, bool gate_up,
                    bool partial_only, M40PairPlan* plan) {

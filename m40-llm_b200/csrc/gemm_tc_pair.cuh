@@ -22,6 +22,7 @@ struct M40PairCall {
     M40Tail tail;
 };
 
+bool m40_pair_available(const M40llmCudaContext* ctx);
 // m40_pair_cut_best() for this device. `gate_up`: two problems of equal N, out = act(first) * second. False: the device takes no CTA
 // pairs.
 bool m40_pair_plan(const M40llmCudaContext* ctx, uint32_t M, uint32_t kblocks, uint32_t problems, const int* N, bool gate_up,

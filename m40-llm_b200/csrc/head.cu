@@ -172,7 +172,7 @@ int m40llm_logits_head_f32_async(M40llmCudaContext* ctx, const void* d_hidden_f3
         if (rc != 1) return rc;
     }
     const void* wp[1] = {d_lm_head_f16};
-    if ((int)rows >= m40_tc_min_rows() && hidden % 4 == 0 && m40_gemm_tc_supported((int)rows, (int)hidden, 1, wp)) {
+    if ((int)rows >= m40_tc_min_rows() && hidden % 4 == 0 && m40_gemm_tc_supported(ctx, (int)rows, (int)hidden, 1, wp)) {
         const __half* w[1] = {(const __half*)d_lm_head_f16};
         const int n[1] = {(int)vocab};
         float* o[1] = {(float*)d_logits_f32};

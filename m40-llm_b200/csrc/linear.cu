@@ -132,19 +132,19 @@ int launch_f32(M40llmCudaContext* ctx, cudaStream_t s, const F32Args& a) {
 
 bool al16(const void* p) { return (((uintptr_t)p) & 15u) == 0u; }
 
-bool tc_takes(const M40llmLinear& c) {
+bool tc_takes(const M40llmCudaContext* ctx, const M40llmLinear& c) {
     const void* wp[2] = {c.w, c.w2};
     const bool tail_used = c.post.kind != M40LLM_NORM_NONE || c.soft_cap > 0.0f || c.bias || c.residual;
     return c.rows >= 2 && (!c.w2 || !tail_used) && al16(c.x) && c.ldx % 4 == 0 &&
-           m40_gemm_tc_supported(c.rows > 256 ? 256 : (int)c.rows, (int)c.K, c.w2 ? 2 : 1, wp);
+           m40_gemm_tc_supported(ctx, c.rows > 256 ? 256 : (int)c.rows, (int)c.K, c.w2 ? 2 : 1, wp);
 }
 
 // Whether the route the call takes applies its norm of x itself. (The streaming kernel declines a few shapes only when it is
 // called; project() then runs the norm as a pass.)
-bool folds_norm(const M40llmLinear& c) {
+bool folds_norm(const M40llmCudaContext* ctx, const M40llmLinear& c) {
     if (c.exact || c.w_dtype == M40LLM_DT_F32 || (c.pre.kind == M40LLM_NORM_RMS && c.pre.groups > 1)) return false;
     if (c.pre.kind <= M40LLM_NORM_DYT && (!al16(c.pre.w) || !al16(c.pre.b))) return false;
-    return c.rows == 1 ? c.K % 8 == 0 && al16(c.x) : tc_takes(c);
+    return c.rows == 1 ? c.K % 8 == 0 && al16(c.x) : tc_takes(ctx, c);
 }
 
 // The projection itself: pre is NONE or one that the route folds in, post NONE or DYT.
@@ -171,7 +171,7 @@ int project(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind, const 
                                        c.w_dtype == M40LLM_DT_BF16 ? M40_GEMV_BF16 : M40_GEMV_F16, c.w2 ? 1 : 0, 1, &seg, np, &ext);
         if (rc != 1) return rc;
     }
-    if (fast && tc_takes(c)) {
+    if (fast && tc_takes(ctx, c)) {
         M40TcExt ext = {};
         ext.bf16 = c.w_dtype == M40LLM_DT_BF16 ? 1 : 0;
         ext.ldx = (int)c.ldx;
@@ -232,7 +232,7 @@ extern "C" int m40llm_linear_async(M40llmCudaContext* ctx, const M40llmLinear* c
 
     // passes of their own: rows of pre(x), rows of the plain result (level-1 arena: this is a composite call)
     const bool rms_after = c.post.kind == M40LLM_NORM_RMS;
-    const bool norm_first = c.pre.kind != M40LLM_NORM_NONE && !folds_norm(c);
+    const bool norm_first = c.pre.kind != M40LLM_NORM_NONE && !folds_norm(ctx, c);
     const size_t pre_elems = norm_first ? ((size_t)c.rows * c.K + 3) & ~(size_t)3 : 0;
     const size_t post_elems = rms_after ? (size_t)c.rows * c.N : 0;
     float* work = nullptr;
