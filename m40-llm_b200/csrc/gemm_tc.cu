@@ -37,11 +37,12 @@ using namespace tc;
 // (128 rows: 42 + 7 against 35 + 9 us at 4096 x 14336, 21 + 7 against 18 + 8 at 4096 x 4096); from here on it is mostly faster
 // (gate | up of 2 x 14336 x 4096: 111 against 155 + 21 us at 256 rows, 638 against 1005 at 2048).
 constexpr uint32_t PAIR_MIN_ROWS = 129;
-// What stays on gemm_tc_f16_kernel beyond: calls whose K it splits (so that hi and lo may share an accumulator: the sums are short),
+// What stays on gemm_tc_f16_kernel beyond: calls of five weight tiles or more whose K it splits three ways or more (so that hi and lo
+// may share an accumulator: the sums are short),
 // up to 144 rows, where two CTAs fit an SM (129 rows, 8192 x 2048: 19.1 against 21.2 us with the pairs, 1408 x 2048: 12.6 against 14.3),
 // and narrow gate | up calls of up to 208 rows with many splits (2 x 640 x 8192: 22 against 24.5 us at 176 rows, 23.4 against 25 at
-// 200). Of 544 measured calls of 129 to 256 rows, 64 to 8192 outputs and K of 64 to 8192 the choice was at most 19 % off the better one.
-constexpr uint32_t SINGLE_MAX_ROWS = 144, SINGLE_GATED_ROWS = 208, SINGLE_GATED_SPLITS = 6;
+// 200). Of 544 measured calls of 129 to 256 rows, 64 to 8192 outputs and K of 64 to 8192 the choice was at most 9 % off the better one.
+constexpr uint32_t SINGLE_MAX_ROWS = 144, SINGLE_SPLITS = 3, SINGLE_TILES = 5, SINGLE_GATED_ROWS = 208, SINGLE_GATED_SPLITS = 6;
 
 struct TcArgs {
     float* partial;            // [k_splits][M][n_total]
@@ -612,7 +613,8 @@ int m40_gemm_tc_f16(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind
     // Many rows go to the CTA-pair kernel, which finishes the result itself unless K is split (see PAIR_MIN_ROWS).
     M40PairPlan plan = {};
     const bool gate_up = mode == 1 && problems == 2 && N[0] == N[1], one = !rope && problems == 1 && mode == 0;
-    const bool single = ks > 1 && ((uint32_t)M <= SINGLE_MAX_ROWS || (gate_up && (uint32_t)M <= SINGLE_GATED_ROWS && ks >= SINGLE_GATED_SPLITS));
+    const bool single = tiles >= SINGLE_TILES && ((ks >= SINGLE_SPLITS && (uint32_t)M <= SINGLE_MAX_ROWS) ||
+                                                  (ks >= SINGLE_GATED_SPLITS && gate_up && (uint32_t)M <= SINGLE_GATED_ROWS));
     const bool pairs = (uint32_t)M >= PAIR_MIN_ROWS && !single;
     if (pairs && !m40_pair_plan(ctx, (uint32_t)M, a.kblocks_total, (uint32_t)problems, N, gate_up, !one, &plan)) return -2;
     if (pairs) {
