@@ -692,7 +692,7 @@ def prefill_case(nat, ev, reps=10):
         b.free()
     return {"prompt_tokens": total, "sequences": [int(n) for n in lens], "ms_per_call": ms, "prompt_tokens_per_s": total / (ms * 1e-3),
             "algorithmic_tflops": tf, "frac_of_bf16_tensor_peak": tf / peak_tf,
-            "note": "mma.sync (legacy tensor path) flash-attention kernel over f16 copies of K / V made by a pack pass of the same call; "
+            "note": "tcgen05 flash-attention kernel (short prompts: mma.sync) over f16 copies of K / V made by a pack pass of the same call; "
                     "the call also reads the lengths back to the host as the reference does"}
 
 

@@ -37,11 +37,10 @@ using namespace tc;
 // (128 rows: 42 + 7 against 35 + 9 us at 4096 x 14336, 21 + 7 against 18 + 8 at 4096 x 4096); from here on it is mostly faster
 // (gate | up of 2 x 14336 x 4096: 111 against 155 + 21 us at 256 rows, 638 against 1005 at 2048).
 constexpr uint32_t PAIR_MIN_ROWS = 129;
-// What stays on gemm_tc_f16_kernel beyond: calls of five weight tiles or more whose K it splits three ways or more (so that hi and lo
-// may share an accumulator: the sums are short),
-// up to 144 rows, where two CTAs fit an SM (129 rows, 8192 x 2048: 19.1 against 21.2 us with the pairs, 1408 x 2048: 12.6 against 14.3),
-// and narrow gate | up calls of up to 208 rows with many splits (2 x 640 x 8192: 22 against 24.5 us at 176 rows, 23.4 against 25 at
-// 200). Of 544 measured calls of 129 to 256 rows, 64 to 8192 outputs and K of 64 to 8192 the choice was at most 9 % off the better one.
+// What stays on gemm_tc_f16_kernel beyond: calls of five weight tiles or more whose K it splits three ways or more (so that hi and
+// lo may share an accumulator: the sums are short). Up to 144 rows two CTAs fit an SM (129 rows, 8192 x 2048: 19.1 against 21.2 us
+// with the pairs, 1408 x 2048: 12.6 against 14.3); narrow gate | up calls with many splits gain up to 208 rows (2 x 640 x 8192: 22
+// against 24.5 us at 176 rows, 23.4 against 25 at 200). Of 544 measured calls of 129 to 256 rows, 64 to 8192 outputs and K of 64 to 8192 the choice was at most 9 % off the better one.
 constexpr uint32_t SINGLE_MAX_ROWS = 144, SINGLE_SPLITS = 3, SINGLE_TILES = 5, SINGLE_GATED_ROWS = 208, SINGLE_GATED_SPLITS = 6;
 
 struct TcArgs {
