@@ -63,6 +63,8 @@ struct TcArgs {
     M40Tail tail;
 };
 
+// STACKED: hi and lo rows in one MMA, M_pad <= 128.
+template <bool STACKED>
 __global__ void __launch_bounds__(192, 1) gemm_tc_f16_kernel(const __grid_constant__ CUtensorMap tmW0,
                                                              const __grid_constant__ CUtensorMap tmW1,
                                                              const __grid_constant__ CUtensorMap tmW2,
@@ -87,8 +89,7 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_f16_kernel(const __grid_consta
     // hi and lo activation tiles are contiguous rows of one operand: up to M_pad = 128 a single MMA of width 2 * M_pad takes the
     // weight tile against both (the weight operand passes the tensor core once); the two halves of the accumulator are added in
     // the epilogue. Wider tiles add the two products in one accumulator.
-    const bool stacked = a.M_pad <= 128u;
-    const uint32_t acc_cols = stacked ? 2u * a.M_pad : a.M_pad;
+    const uint32_t acc_cols = STACKED ? 2u * a.M_pad : a.M_pad;
     uint32_t tmem_cols = 32;
     while (tmem_cols < acc_cols) tmem_cols <<= 1;
 
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_f16_kernel(const __grid_consta
                 for (uint32_t k = 0; k < BLOCK_K / UMMA_K; ++k) {
                     const uint64_t da = make_desc_sw128(sa + k * UMMA_K * 2);
                     umma_f16(tmem_base, da, make_desc_sw128(sb + k * UMMA_K * 2), idesc, i | k);
-                    if (!stacked) umma_f16(tmem_base, da, make_desc_sw128(sb + b_bytes + k * UMMA_K * 2), idesc, 1u);
+                    if (!STACKED) umma_f16(tmem_base, da, make_desc_sw128(sb + b_bytes + k * UMMA_K * 2), idesc, 1u);
                 }
                 umma_commit(&empty[s]);                 // frees the stage once these MMAs have read it
                 if (i + 1 == n_kb) umma_commit(accum);  // accumulator complete
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_f16_kernel(const __grid_consta
             float v[8];
             if (ok) {
                 tmem_ld8(tmem_base + ((lane_group * 32u) << 16) + c, v);
-                if (stacked) {
+                if (STACKED) {
                     float w[8];
                     tmem_ld8(tmem_base + ((lane_group * 32u) << 16) + a.M_pad + c, w);
 #pragma unroll
@@ -711,12 +712,14 @@ int m40_gemm_tc_f16(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind
         static unsigned long long configured = 0ull;
         const unsigned long long bit = 1ull << (ctx->device_id & 63);
         if (!(configured & bit)) {
-            if (cudaFuncSetAttribute(gemm_tc_f16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
+            if (cudaFuncSetAttribute(gemm_tc_f16_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
+                cudaFuncSetAttribute(gemm_tc_f16_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
                 return -2;
             configured |= bit;
         }
         dim3 grid(tiles, ks);
-        m40_launch_dependent(gemm_tc_f16_kernel, grid, dim3(192), smem, s, mW[0], mW[1], mW[2], mXh, mXl, a);
+        m40_launch_dependent(M_pad <= 128u ? gemm_tc_f16_kernel<true> : gemm_tc_f16_kernel<false>, grid, dim3(192), smem, s, mW[0], mW[1], mW[2],
+                             mXh, mXl, a);
         M40_COUNT_LAUNCH(ctx);
         if (cudaGetLastError() != cudaSuccess) return -2;
         if (direct) return 0;
