@@ -3,24 +3,29 @@
 // with a decay w and a removal rate a per head and key channel, u the unit key. All of it is f32.
 //
 // With k = n u (n the key's length) the update of one value column s of S is
-//   d = u . s,   s_i <- w_i s_i + u_i (n v - a_i d),   o = r . s,
-// so columns are independent and a token costs one dot product, one update and one dot product per column. A column's key
-// dimension is shared by a few lanes (16-byte pieces dealt round-robin) and stays in registers; the only serial chain is d,
-// and the second dot product of a token overlaps the first of the next.
+//   d = u . s,   s_i <- w_i s_i + u_i n v - (a u)_i d,   o = r . s,
+// so columns are independent. A column's key dimension is shared by a few lanes (16-byte pieces dealt round-robin) and stays in
+// registers; the only serial chain is d: a dot product over the lanes, then one multiply-add per element.
 //
 //   portions of several tokens, in passes of rows whose records stay in L2:
-//     delta_prepare_kernel  warp = (row, head): gates, decays, unit key -> one record [w | u | a | r | n v] per (head, row);
-//     delta_scan_kernel     CTA = (32 columns, head, segment) walks the tokens; the records of 32 or 16 tokens arrive by one bulk
-//                           copy (cp.async.bulk + mbarrier) several chunks ahead. Eight lanes share two columns, because
-//                           the limit is shared-memory reads: every vector piece read serves both;
+//     delta_prepare_kernel  warp = (row, head): gates, decays, unit key -> one record [w | u | a u | r | n v | c] per (head, row);
+//     delta_scan_kernel     CTA = (16 or 64 columns, head, segment) walks the tokens in pairs; the records of 16 tokens arrive by
+//                           one bulk copy (cp.async.bulk + mbarrier) several chunks ahead. Reads of the records from shared memory
+//                           are the limit, so a lane holds few keys of several columns and every piece serves all of them;
 //     delta_finish_kernel   the per-head norm and the output gate.
 //   delta_decode_kernel     one token per sequence: CTA = (head, row) does everything, the low-rank decay projection
 //                           included, in one launch; bound by reading and writing the state once.
-// A chunked (matrix-product) form is not used: its products of decays and of removals would have to leave f32, or lose the
-// property that the result does not depend on where a portion was cut.
+//
+// Two tokens share one trip over the lanes. With s1 the column after the first of a pair,
+//   d1 = u1 . s1 = (w0 u1) . s0 + c1 n0 v0 - c2 d0,   c1 = u1 . u0,   c2 = u1 . (a0 u0),
+// so both dot products start from s0, and c1 and c2 are the same for all columns and come with the record. The terms are those of
+// u1 . s1 added up in another order, in f32 like everything here. A longer chunked (matrix-product) form is not used: its products of
+// decays would have to leave f32.
 //
 // The scan's waits are bounded like the tensor-core kernels': a wait that runs out raises status bit 4, the CTA stops,
 // waits (bounded) for its copies in flight and returns.
+#include <atomic>
+
 #include "common.cuh"
 #include "stack_math.cuh"
 #include "state_cache.cuh"
@@ -29,16 +34,14 @@
 namespace {
 
 constexpr int LANES = 4;          // decode: lanes per column
-constexpr int SCAN_LANES = 8;     // scan: lanes per pair of columns
-constexpr int SCAN_COLS = 32;     // columns per scan CTA
-constexpr int SCAN_THREADS = SCAN_COLS / 2 * SCAN_LANES;
+constexpr int SCAN_THREADS = 128;
 constexpr size_t PASS_BYTES = (size_t)96 << 20;  // records of one pass: inside L2
-// Tokens per bulk copy, and copies in flight, for records of 5 * DP floats.
-__host__ __device__ constexpr int scan_chunk(int dp) { return dp <= 128 ? 32 : 16; }
-__host__ __device__ constexpr size_t scan_stage_bytes(int dp) { return (size_t)scan_chunk(dp) * 5 * dp * sizeof(float); }
-__host__ __device__ constexpr uint32_t scan_stages(int dp) {
-    return (size_t)4 * scan_stage_bytes(dp) <= 196608u ? 4u : (uint32_t)(196608u / scan_stage_bytes(dp));
-}
+constexpr int SCAN_CHUNK = 16;    // tokens per bulk copy (even: pairs do not cross chunks)
+constexpr uint32_t SCAN_MAX_STAGES = 8;
+constexpr int SCAN_SMEM = 196608;
+// A record: w | u | a u | r | n v, DP floats each, then c1, c2 and two floats of padding.
+__host__ __device__ constexpr uint32_t rec_floats(int dp) { return 5u * dp + 4u; }
+__host__ __device__ constexpr size_t scan_stage_bytes(int dp) { return (size_t)SCAN_CHUNK * rec_floats(dp) * sizeof(float); }
 
 struct DeltaArgs {
     const float* packed;
@@ -137,7 +140,8 @@ __device__ __forceinline__ float delta_token(const float* vec, uint32_t l4, floa
 }
 
 // Rows [base, base + count) of every segment (relative to its start) -> records. One warp per (row, head); `rec` holds, per
-// head, n_rec records of 5 * DP floats, the record of row r of the step at r - base.
+// head, n_rec records, the record of row r of the step at r - base. c1 and c2 look back at the row before, whatever sequence it
+// belongs to: the scan uses them within a segment only.
 template <int DP>
 __global__ void __launch_bounds__(256) delta_prepare_kernel(DeltaArgs a, float* __restrict__ rec, uint32_t n_rec, uint32_t base,
                                                             uint32_t count) {
@@ -148,7 +152,8 @@ __global__ void __launch_bounds__(256) delta_prepare_kernel(DeltaArgs a, float* 
     if (wid >= count * a.heads) return;
     const uint32_t head = wid % a.heads, row = base + wid / a.heads, D = a.dim, HD = a.heads * D;
     const float* p = a.packed + (size_t)row * a.ld + head * D;
-    float r[CPL], k[CPL], v[CPL], rate[CPL], z[CPL], ss = 0.0f;
+    const float* before = p - (row > 0u ? a.ld : 0u);
+    float r[CPL], k[CPL], v[CPL], rate[CPL], z[CPL], k0[CPL], rate0[CPL], ss = 0.0f, ss0 = 0.0f;
 #pragma unroll
     for (int i = 0; i < CPL; ++i) {
         const uint32_t ch = lane + 32u * i, cc = ch < D ? ch : D - 1u;  // clamped: every load is unconditional
@@ -157,6 +162,8 @@ __global__ void __launch_bounds__(256) delta_prepare_kernel(DeltaArgs a, float* 
         v[i] = p[2 * (size_t)HD + cc];
         rate[i] = p[4 * (size_t)HD + cc] + a.a_bias[head * D + cc];
         z[i] = (a.decay_in ? a.decay_in[(size_t)row * HD + head * D + cc] : 0.0f) + a.w0[head * D + cc];
+        k0[i] = before[HD + cc];
+        rate0[i] = before[4 * (size_t)HD + cc] + a.a_bias[head * D + cc];
     }
     if (!a.decay_in) {
         const float* zp = a.packed + (size_t)row * a.ld + 5 * (size_t)HD;
@@ -169,67 +176,114 @@ __global__ void __launch_bounds__(256) delta_prepare_kernel(DeltaArgs a, float* 
         }
     }
 #pragma unroll
-    for (int i = 0; i < CPL; ++i) ss = lane + 32u * i < D ? fmaf(k[i], k[i], ss) : ss;
+    for (int i = 0; i < CPL; ++i) {
+        ss = lane + 32u * i < D ? fmaf(k[i], k[i], ss) : ss;
+        ss0 = lane + 32u * i < D ? fmaf(k0[i], k0[i], ss0) : ss0;
+    }
     const float len = sqrtf(warp_sum(ss) + a.unit_eps), inv = 1.0f / len;
-    float* dst = rec + ((size_t)head * n_rec + (row - base)) * (5 * DP);
+    const float inv0 = 1.0f / sqrtf(warp_sum(ss0) + a.unit_eps);
+    float* dst = rec + ((size_t)head * n_rec + (row - base)) * rec_floats(DP);
+    float c1 = 0.0f, c2 = 0.0f;
 #pragma unroll
     for (int i = 0; i < CPL; ++i) {
         const uint32_t ch = lane + 32u * i;
         const bool in = ch < D;
+        const float u = k[i] * inv, u0 = k0[i] * inv0;
         dst[ch] = in ? decay_of(a, z[i]) : 0.0f;
-        dst[DP + ch] = in ? k[i] * inv : 0.0f;
-        dst[2 * DP + ch] = in ? m40_sigmoid(rate[i]) : 0.0f;
+        dst[DP + ch] = in ? u : 0.0f;
+        dst[2 * DP + ch] = in ? u * m40_sigmoid(rate[i]) : 0.0f;
         dst[3 * DP + ch] = in ? r[i] : 0.0f;
         dst[4 * DP + ch] = in ? len * v[i] : 0.0f;
+        c1 = in ? fmaf(u, u0, c1) : c1;
+        c2 = in ? fmaf(u, u0 * m40_sigmoid(rate0[i]), c2) : c2;
     }
+    c1 = warp_sum(c1), c2 = warp_sum(c2);
+    if (lane == 0) *reinterpret_cast<float4*>(dst + 5 * DP) = make_float4(c1, c2, 0.0f, 0.0f);
 }
 
-// Four sums over the eight lanes of a column pair at once: the shuffles of one level are independent of each other.
-__device__ __forceinline__ void sum_lanes8(float& a, float& b, float& c, float& d) {
-#pragma unroll
-    for (int o = 1; o < SCAN_LANES; o <<= 1) {
-        const float ta = __shfl_xor_sync(0xffffffffu, a, o), tb = __shfl_xor_sync(0xffffffffu, b, o);
-        const float tc_ = __shfl_xor_sync(0xffffffffu, c, o), td = __shfl_xor_sync(0xffffffffu, d, o);
-        a += ta, b += tb, c += tc_, d += td;
-    }
-}
-// This lane's pieces of one token's record.
-template <int NI>
-struct TokenVec {
-    float4 u[NI], w[NI], a[NI], r[NI];
-    float2 nv;
-    __device__ __forceinline__ void load(const float* rec, uint32_t l, uint32_t col) {
-        constexpr int DP = NI * SCAN_LANES * 4;
-        const float4* v4 = reinterpret_cast<const float4*>(rec) + l;
-#pragma unroll
-        for (int i = 0; i < NI; ++i) {
-            w[i] = v4[SCAN_LANES * i];
-            u[i] = v4[DP / 4 + SCAN_LANES * i];
-            a[i] = v4[2 * (DP / 4) + SCAN_LANES * i];
-            r[i] = v4[3 * (DP / 4) + SCAN_LANES * i];
-        }
-        nv = *reinterpret_cast<const float2*>(rec + 4 * DP + col);
-    }
+// Two f32 in one register pair: one instruction works on both (rounded like the scalar ones).
+struct F2 {
+    unsigned long long v;
 };
-__device__ __forceinline__ float dot4(const float4& x, const float4& y) {
-    return fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, x.w * y.w)));
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
 }
-__device__ __forceinline__ void update4(float4& s, const float4& w, const float4& u, const float4& a, float d, float nv) {
-    s.x = fmaf(u.x, fmaf(-a.x, d, nv), w.x * s.x);
-    s.y = fmaf(u.y, fmaf(-a.y, d, nv), w.y * s.y);
-    s.z = fmaf(u.z, fmaf(-a.z, d, nv), w.z * s.z);
-    s.w = fmaf(u.w, fmaf(-a.w, d, nv), w.w * s.w);
+__device__ __forceinline__ float f2_sum(F2 a) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
+    return lo + hi;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+// This lane's pieces of one vector of a record.
+template <int NI, int LANES>
+__device__ __forceinline__ void load_pieces(const float* vec, uint32_t l, F2 (&x)[2 * NI]) {
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+        const ulonglong2 t = *(reinterpret_cast<const ulonglong2*>(vec) + l + LANES * i);
+        x[2 * i].v = t.x, x[2 * i + 1].v = t.y;
+    }
+}
+// One trip over LANES lanes: every lane gets the sums of d and e, and of the V values o by halving the one of index held_sum<V>(l),
+// in o[0]. The shuffles of a level are independent of each other and stand next to each other: the compiler keeps their order, and
+// one value after the other would pay for each shuffle's latency (16 instead of 4: 300 instead of 241 us for 2048 tokens of 32 x 64).
+template <int COLS, int V, int LANES, int BIT = 1>
+__device__ __forceinline__ void sums_over_lanes(float (&d)[COLS], float (&e)[COLS], float (&o)[V], uint32_t l) {
+    constexpr uint32_t FULL = 0xffffffffu;
+    if constexpr (BIT < LANES) {
+        constexpr int H = V > 1 ? V / 2 : 1;
+        const bool upper = l & BIT;
+        float td[COLS], te[COLS], to[H], half[H];
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) td[c] = __shfl_xor_sync(FULL, d[c], BIT), te[c] = __shfl_xor_sync(FULL, e[c], BIT);
+#pragma unroll
+        for (int i = 0; i < H; ++i) to[i] = __shfl_xor_sync(FULL, V > 1 && !upper ? o[V > 1 ? H + i : 0] : o[i], BIT);
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) d[c] += td[c], e[c] += te[c];
+#pragma unroll
+        for (int i = 0; i < H; ++i) half[i] = (V > 1 && upper ? o[V > 1 ? H + i : 0] : o[i]) + to[i];
+        sums_over_lanes<COLS, H, LANES, BIT * 2>(d, e, half, l);
+        o[0] = half[0];
+    }
+}
+template <int V>
+__device__ __forceinline__ uint32_t held_sum(uint32_t l) {
+    uint32_t at = 0;
+#pragma unroll
+    for (int half = V / 2, bit = 0; half > 0; half /= 2, ++bit) at += (l >> bit & 1u) * half;
+    return at;
 }
 
-// grid (column blocks, heads, segments). Rows [base, base + count) of the segment, counted from its start.
-template <int NI>
+// COLS adjacent values.
+template <int COLS>
+__device__ __forceinline__ void load_values(const float* p, float (&v)[COLS]) {
+    static_assert(COLS == 2 || COLS == 4, "vector loads");
+    if constexpr (COLS == 2)
+        *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(p);
+    else
+        *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
+}
+
+// grid (column blocks, heads, segments). Rows [base, base + count) of the segment, counted from its start. LANES lanes hold COLS
+// columns of LANES * NI * 4 keys. 2048 tokens of one sequence, 32 heads of 64: 241 us (324 a token at a time, 32 columns per CTA), of
+// which a pair's chain of shuffles and multiply-adds takes most; 1500 tokens of 16 sequences, 64 heads: 137 us (238).
+template <int NI, int LANES, int COLS>
 __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a, const float* __restrict__ rec, uint32_t n_rec,
-                                                                  uint32_t rec_base, uint32_t base, uint32_t count) {
-    constexpr int DP = NI * SCAN_LANES * 4, CHUNK = scan_chunk(DP);
-    constexpr uint32_t stages = scan_stages(DP);
-    constexpr uint32_t REC = 5 * DP;
+                                                                  uint32_t rec_base, uint32_t base, uint32_t count, uint32_t stages) {
+    constexpr int DP = NI * LANES * 4;
+    constexpr uint32_t REC = rec_floats(DP), CHUNK = SCAN_CHUNK;
     extern __shared__ __align__(128) float ring[];
-    __shared__ uint64_t full[4];
+    __shared__ uint64_t full[SCAN_MAX_STAGES];
     __shared__ uint32_t stop;
     const uint32_t tid = threadIdx.x;
     if (tid == 0) {
@@ -240,7 +294,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a, c
     __syncthreads();
     pdl_wait();
     pdl_trigger();
-    const uint32_t head = blockIdx.y, col0 = blockIdx.x * SCAN_COLS, D = a.dim, HD = a.heads * D;
+    const uint32_t head = blockIdx.y, col0 = blockIdx.x * (SCAN_THREADS / LANES * COLS), D = a.dim, HD = a.heads * D;
     const uint32_t seg0 = a.seg[4 * blockIdx.z], seg_n = a.seg[4 * blockIdx.z + 1];
     const uint32_t slot = a.seg[4 * blockIdx.z + 2] * a.slot_mul + a.slot_add, pos0 = a.seg[4 * blockIdx.z + 3];
     if (slot >= a.slots || (uint64_t)seg0 + seg_n > a.rows) {
@@ -251,62 +305,114 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a, c
     const uint32_t n = seg_n - base < count ? seg_n - base : count, row0 = seg0 + base;
     const float* src = rec + ((size_t)head * n_rec + (row0 - rec_base)) * REC;
     const uint32_t chunks = (n + CHUNK - 1) / CHUNK;
-    auto request = [&](uint32_t ch) {  // thread 0
-        const uint32_t m = n - ch * CHUNK < CHUNK ? n - ch * CHUNK : CHUNK, bytes = m * REC * 4u, s = ch % stages;
+    auto request = [&](uint32_t ch, uint32_t s) {  // thread 0
+        const uint32_t m = n - ch * CHUNK < CHUNK ? n - ch * CHUNK : CHUNK, bytes = m * REC * 4u;
         tc::mbar_expect_tx(&full[s], bytes);
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                      ::"r"(tc::smem_u32(ring + (size_t)s * CHUNK * REC)), "l"(src + (size_t)ch * CHUNK * REC), "r"(bytes),
                      "r"(tc::smem_u32(&full[s])) : "memory");
     };
     if (tid == 0)
-        for (uint32_t ch = 0; ch < chunks && ch < stages; ++ch) request(ch);
+        for (uint32_t ch = 0; ch < chunks && ch < stages; ++ch) request(ch, ch);
 
-    const uint32_t l = tid % SCAN_LANES, c = tid / SCAN_LANES * 2u, ca = col0 + c, cb = ca + 1u;
+    const uint32_t l = tid % LANES, first = col0 + tid / LANES * COLS;
+    const uint32_t nv_at = 4 * DP + (first < DP ? first : 0u);  // a block may reach beyond the padded columns
     float* state = a.state + ((size_t)slot * a.heads + head) * D * D;
-    float4 sa[NI], sb[NI];
+    F2 s[COLS][2 * NI];
     const bool fresh = pos0 == 0 && base == 0;
-    load_column<NI, SCAN_LANES>(state + (size_t)(ca < D ? ca : 0u) * D, D, l, fresh || ca >= D, sa);
-    load_column<NI, SCAN_LANES>(state + (size_t)(cb < D ? cb : 0u) * D, D, l, fresh || cb >= D, sb);
-    float* out = a.out + (size_t)row0 * HD + head * D + (l == 0 ? ca : cb);
-    const bool store = l == 0 ? ca < D : (l == 1 && cb < D);
+#pragma unroll
+    for (int c = 0; c < COLS; ++c) {
+        float4 t[NI];
+        const uint32_t col = first + c;
+        load_column<NI, LANES>(state + (size_t)(col < D ? col : 0u) * D, D, l, fresh || col >= D, t);
+#pragma unroll
+        for (int i = 0; i < NI; ++i) s[c][2 * i] = f2(t[i].x, t[i].y), s[c][2 * i + 1] = f2(t[i].z, t[i].w);
+    }
+    // lanes 0 .. 2 COLS - 1 store: outputs o[column][token] of a pair
+    constexpr uint32_t V = 2 * COLS;
+    const uint32_t token = held_sum<V>(l) % 2u, mine = first + held_sum<V>(l) / 2u;
+    float* out = a.out + (size_t)(row0 + token) * HD + head * D + (mine < D ? mine : 0u);
+    const bool store = l < V && mine < D;
 
-    // Software pipeline: a token's pieces are read while the previous token is worked on (within a chunk), and the two
-    // outputs of the previous token are summed over the lanes together with this token's two d.
-    float oa = 0.0f, ob = 0.0f;
-    uint32_t ch = 0;
+    const F2 zero = f2(0.0f, 0.0f);
+    float o[V] = {};  // the outputs of the pair before, still spread over the lanes: summed together with this pair's products
+    bool held = false;
+    uint32_t ch = 0, slot_at = 0, phase = 0;
     for (; ch < chunks; ++ch) {
-        const uint32_t s = ch % stages;
-        if (!tc::mbar_wait(&full[s], (ch / stages) & 1u)) stop = 1u;
-        const float* buf = ring + (size_t)s * CHUNK * REC;
+        if (!tc::mbar_wait(&full[slot_at], phase)) stop = 1u;
+        const float* buf = ring + (size_t)slot_at * CHUNK * REC;
         const uint32_t m = n - ch * CHUNK < CHUNK ? n - ch * CHUNK : CHUNK;
-        TokenVec<NI> cur;
-        cur.load(buf, l, col0 + c);
-#pragma unroll 2
-        for (uint32_t t = 0; t < m; ++t) {
-            TokenVec<NI> nxt;
-            nxt.load(buf + (size_t)(t + 1u < m ? t + 1u : t) * REC, l, col0 + c);
-            float da = 0.0f, db = 0.0f;
+        F2 u0[2 * NI], q1[2 * NI], w0[2 * NI];  // of the pair at hand: u0, w0 and w0 u1
+        load_pieces<NI, LANES>(buf, l, w0);
+        load_pieces<NI, LANES>(buf + DP, l, u0);
+        load_pieces<NI, LANES>(buf + (m > 1u ? REC : 0u) + DP, l, q1);
 #pragma unroll
-            for (int i = 0; i < NI; ++i) {
-                da += dot4(cur.u[i], sa[i]);
-                db += dot4(cur.u[i], sb[i]);
-            }
-            sum_lanes8(da, db, oa, ob);
-            const uint32_t row = ch * CHUNK + t;
-            if (store && row > 0u) out[(size_t)(row - 1u) * HD] = l == 0 ? oa : ob;
-            oa = ob = 0.0f;
+        for (int i = 0; i < 2 * NI; ++i) q1[i] = f2_mul(q1[i], w0[i]);
+        for (uint32_t t = 0; t < m; t += 2u) {
+            const float* va = buf + (size_t)t * REC;
+            const bool two = t + 1u < m;
+            const float* vb = va + (two ? REC : 0u);
+            float d[COLS], e[COLS];
 #pragma unroll
-            for (int i = 0; i < NI; ++i) {
-                update4(sa[i], cur.w[i], cur.u[i], cur.a[i], da, cur.nv.x);
-                update4(sb[i], cur.w[i], cur.u[i], cur.a[i], db, cur.nv.y);
-                oa += dot4(cur.r[i], sa[i]);
-                ob += dot4(cur.r[i], sb[i]);
+            for (int c = 0; c < COLS; ++c) {
+                F2 x = f2_mul(u0[0], s[c][0]), y = f2_mul(q1[0], s[c][0]);
+#pragma unroll
+                for (int i = 1; i < 2 * NI; ++i) x = f2_fma(u0[i], s[c][i], x), y = f2_fma(q1[i], s[c][i], y);
+                d[c] = f2_sum(x), e[c] = f2_sum(y);
             }
-            cur = nxt;
+            // the rest of this pair's records and the start of the next pair's are on their way during the shuffles
+            F2 ua[2 * NI], r[2 * NI], u1[2 * NI], w1[2 * NI], ub[2 * NI], r1[2 * NI];
+            load_pieces<NI, LANES>(va + 2 * DP, l, ua);
+            load_pieces<NI, LANES>(va + 3 * DP, l, r);
+            load_pieces<NI, LANES>(vb, l, w1);
+            load_pieces<NI, LANES>(vb + DP, l, u1);
+            load_pieces<NI, LANES>(vb + 2 * DP, l, ub);
+            load_pieces<NI, LANES>(vb + 3 * DP, l, r1);
+            const float2 cc = *reinterpret_cast<const float2*>(vb + 5 * DP);
+            float nv0[COLS], nv1[COLS];
+            load_values<COLS>(va + nv_at, nv0);
+            load_values<COLS>(vb + nv_at, nv1);
+            sums_over_lanes<COLS, V, LANES>(d, e, o, l);
+            if (held) {
+                if (store) out[0] = o[0];
+                out += 2 * (size_t)HD;
+            }
+            held = two;
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) {
+                const F2 n0 = f2(nv0[c], nv0[c]), d0 = f2(-d[c], -d[c]);
+                F2 x = zero;
+#pragma unroll
+                for (int i = 0; i < 2 * NI; ++i) {
+                    s[c][i] = f2_fma(ua[i], d0, f2_fma(w0[i], s[c][i], f2_mul(u0[i], n0)));
+                    x = f2_fma(r[i], s[c][i], x);
+                }
+                o[2 * c] = f2_sum(x);
+            }
+            if (!two) break;  // the last token of the segment
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) {
+                const float d1 = fmaf(-cc.y, d[c], fmaf(cc.x, nv0[c], e[c]));
+                const F2 n1 = f2(nv1[c], nv1[c]), dd = f2(-d1, -d1);
+                F2 x = zero;
+#pragma unroll
+                for (int i = 0; i < 2 * NI; ++i) {
+                    s[c][i] = f2_fma(ub[i], dd, f2_fma(w1[i], s[c][i], f2_mul(u1[i], n1)));
+                    x = f2_fma(r1[i], s[c][i], x);
+                }
+                o[2 * c + 1] = f2_sum(x);
+            }
+            const float* vn = va + (t + 2u < m ? 2u * REC : 0u);
+            load_pieces<NI, LANES>(vn, l, w0);
+            load_pieces<NI, LANES>(vn + DP, l, u0);
+            load_pieces<NI, LANES>(vn + (t + 3u < m ? REC : 0u) + DP, l, q1);
+#pragma unroll
+            for (int i = 0; i < 2 * NI; ++i) q1[i] = f2_mul(q1[i], w0[i]);
         }
         __syncthreads();  // everyone is done with this slot
         if (stop) break;
-        if (tid == 0 && ch + stages < chunks) request(ch + stages);
+        if (tid == 0 && ch + stages < chunks) request(ch + stages, slot_at);
+        if (++slot_at == stages) slot_at = 0, phase ^= 1u;
     }
     if (ch < chunks) {  // a wait ran out: the copies still in flight must land before this CTA's memory goes away
         if (tid == 0) {
@@ -315,11 +421,23 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a, c
         }
         return;
     }
-    float x0 = 0.0f, x1 = 0.0f;
-    sum_lanes8(oa, ob, x0, x1);
-    if (store) out[(size_t)(n - 1u) * HD] = l == 0 ? oa : ob;
-    if (ca < D) store_column<NI, SCAN_LANES>(state + (size_t)ca * D, D, l, sa);
-    if (cb < D) store_column<NI, SCAN_LANES>(state + (size_t)cb * D, D, l, sb);
+    if (!held) {  // an odd number of tokens: the last one has no partner
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) o[2 * c + 1] = 0.0f;
+    }
+    float none[COLS] = {};
+    sums_over_lanes<COLS, V, LANES>(none, none, o, l);
+    if (store && (held || token == 0u)) out[0] = o[0];
+#pragma unroll
+    for (int c = 0; c < COLS; ++c) {
+        float4 t[NI];
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(t[i].x), "=f"(t[i].y) : "l"(s[c][2 * i].v));
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(t[i].z), "=f"(t[i].w) : "l"(s[c][2 * i + 1].v));
+        }
+        if (first + c < D) store_column<NI, LANES>(state + (size_t)(first + c) * D, D, l, t);
+    }
 }
 
 // out <- (out / rms per head) * norm * sigmoid(g). One warp per (row, head).
@@ -445,22 +563,35 @@ int run_decode(M40llmCudaContext* ctx, const DeltaArgs& a) {
     return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -6;
 }
 
-template <int NI>
-int run_scan(M40llmCudaContext* ctx, const DeltaArgs& a, uint32_t segments, uint32_t max_segment_rows) {
-    constexpr int DP = NI * SCAN_LANES * 4;
-    constexpr uint32_t CHUNK = (uint32_t)scan_chunk(DP);
-    cudaStream_t s = ctx->decode_stream;
-    constexpr size_t smem = scan_stages(DP) * scan_stage_bytes(DP);
-    static_assert(scan_stages(DP) >= 2, "the ring needs two slots");
-    static unsigned long long configured = 0ull;
+template <int NI, int LANES, int COLS>
+int launch_scan(M40llmCudaContext* ctx, const DeltaArgs& a, const float* rec, uint32_t n_rec, uint32_t base, uint32_t pass, uint32_t segments,
+                uint32_t stages) {
+    constexpr int DP = NI * LANES * 4, BLOCK_COLS = SCAN_THREADS / LANES * COLS;
+    const size_t smem = stages * scan_stage_bytes(DP);
+    // contexts on several threads may set it at the same time: setting it twice is harmless, losing another device's bit is not
+    static std::atomic<unsigned long long> configured{0ull};
     const unsigned long long bit = 1ull << (ctx->device_id & 63);
-    if (!(configured & bit)) {
-        if (cudaFuncSetAttribute(delta_scan_kernel<NI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (!(configured.load(std::memory_order_acquire) & bit)) {
+        if (cudaFuncSetAttribute(delta_scan_kernel<NI, LANES, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM) != cudaSuccess)
             return -6;
-        configured |= bit;
+        configured.fetch_or(bit, std::memory_order_release);
     }
+    const dim3 grid((a.dim + BLOCK_COLS - 1) / BLOCK_COLS, a.heads, segments);
+    const cudaError_t e = m40_launch_dependent(delta_scan_kernel<NI, LANES, COLS>, grid, dim3(SCAN_THREADS), smem, ctx->decode_stream, a, rec,
+                                               n_rec, base, base, pass, stages);
+    M40_COUNT_LAUNCH(ctx);
+    return e == cudaSuccess ? 0 : -6;
+}
+
+// P: 32-key pieces of a column.
+template <int P>
+int run_scan(M40llmCudaContext* ctx, const DeltaArgs& a, uint32_t segments, uint32_t max_segment_rows) {
+    constexpr int DP = P * 32;
+    constexpr uint32_t CHUNK = SCAN_CHUNK;
+    cudaStream_t s = ctx->decode_stream;
+    static_assert(2 * scan_stage_bytes(DP) <= SCAN_SMEM, "the ring needs two slots");
     // One segment is walked in passes of rows whose records fit PASS_BYTES; several segments take one pass.
-    const size_t per_row = (size_t)a.heads * 5 * DP * sizeof(float);
+    const size_t per_row = (size_t)a.heads * rec_floats(DP) * sizeof(float);
     uint32_t pass = max_segment_rows;
     if (segments == 1) {
         const size_t fit = PASS_BYTES / per_row / CHUNK * CHUNK;
@@ -469,7 +600,14 @@ int run_scan(M40llmCudaContext* ctx, const DeltaArgs& a, uint32_t segments, uint
     const uint32_t n_rec = segments == 1 ? pass : a.rows;
     float* rec = (float*)m40_ensure_scratch(ctx, 1, n_rec * per_row, 1);
     if (!rec) return -5;
-    const dim3 grid((a.dim + SCAN_COLS - 1) / SCAN_COLS, a.heads, segments);
+    // Narrow CTAs, sixteen lanes and two columns per group, where two per SM take all of them; otherwise eight lanes and four columns,
+    // and a ring that lets three CTAs share an SM.
+    constexpr int LANES = P % 2 == 0 ? 16 : 8;
+    constexpr uint32_t NARROW = SCAN_THREADS / LANES * 2;
+    const uint64_t ctas = (uint64_t)((a.dim + NARROW - 1) / NARROW) * a.heads * segments;
+    const bool narrow = ctas <= 2u * (uint64_t)ctx->sm_count;
+    const uint32_t fit = (uint32_t)((!narrow ? SCAN_SMEM / 3 : (ctas <= (uint64_t)ctx->sm_count ? SCAN_SMEM : SCAN_SMEM / 2)) / scan_stage_bytes(DP));
+    const uint32_t stages = fit < 2u ? 2u : (fit > SCAN_MAX_STAGES ? SCAN_MAX_STAGES : fit);
     cudaError_t e;
     for (uint32_t base = 0; base < max_segment_rows; base += pass) {
         // `rows` of the step from `base` on: with one segment the pass's rows, with several all of them
@@ -477,10 +615,9 @@ int run_scan(M40llmCudaContext* ctx, const DeltaArgs& a, uint32_t segments, uint
         e = m40_launch_dependent(delta_prepare_kernel<DP>, dim3((rows * a.heads + 7) / 8), dim3(256), 0, s, a, rec, n_rec, base, rows);
         M40_COUNT_LAUNCH(ctx);
         if (e != cudaSuccess) return -6;
-        e = m40_launch_dependent(delta_scan_kernel<NI>, grid, dim3(SCAN_THREADS), smem, s, a, (const float*)rec, n_rec, base, base,
-                                 pass);
-        M40_COUNT_LAUNCH(ctx);
-        if (e != cudaSuccess) return -6;
+        const int rc = narrow ? launch_scan<DP / (4 * LANES), LANES, 2>(ctx, a, rec, n_rec, base, pass, segments, stages)
+                              : launch_scan<P, 8, P <= 4 ? 4 : 2>(ctx, a, rec, n_rec, base, pass, segments, stages);
+        if (rc != 0) return rc;
     }
     e = m40_launch_dependent(delta_finish_kernel, dim3((a.rows * a.heads + 7) / 8), dim3(256), 0, s, a);
     M40_COUNT_LAUNCH(ctx);

@@ -422,6 +422,23 @@ def test_delta_rule_portions_and_decode(nat, H, D, R):
     d.close()
 
 
+@pytest.mark.parametrize("H,D", [(80, 64), (300, 16), (40, 128), (110, 48), (20, 200), (40, 64), (75, 64)])
+def test_delta_rule_forms_of_the_scan(nat, H, D):
+    """Heads enough for the form that fills the machine, around the border to the narrow one (two CTAs per SM of 148), whole and odd
+    numbers of pairs of tokens."""
+    d = Delta(nat, H, D, 4, seed=H)
+    rng = np.random.default_rng(H + D)
+    p0 = {0: 0, 2: 0}
+    for step in ([(0, 33)], [(2, 2), (0, 16)], [(0, 1)], [(0, 31), (2, 5)]):
+        segs = [(s, p0[s], n) for s, n in step]
+        for s, n in step:
+            p0[s] += n
+        packed = rng.standard_normal((sum(n for _, n in step), d.width())).astype(np.float32)
+        close(d.device(packed, segs), d.oracle(packed, segs), 2e-5, f"{segs}")
+    close(d.state(0), d.S[0], 5e-6, "state")
+    d.close()
+
+
 def test_delta_rule_prompt_equals_tokens_and_slot_reuse(nat):
     d = Delta(nat, 3, 40, 12, seed=5)
     rng = np.random.default_rng(6)
