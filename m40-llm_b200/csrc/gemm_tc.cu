@@ -1,24 +1,21 @@
-// Batched decode projections on the 5th-generation tensor cores (tcgen05 + TMEM + TMA).
+// Projections of several activation rows on the 5th-generation tensor cores (tcgen05 + TMEM + TMA): which kernel takes a call, the
+// kernels around them, and the one for a little more than 128 rows.
 //
-// For M >= 2 activation rows the projection C[m][n] = sum_k X[m][k] W[n][k] is computed "swapped":
-// the streamed weight tile is the MMA's A operand (128 weight rows = the MMA M dimension) and the
-// small activation matrix is the B operand (MMA N = batch rows padded to 16..256), so the tensor core
-// runs at full height however small the batch is and every weight byte is read from HBM exactly once:
+//   up to 32 rows           gemm_tc_rows.cu: one launch, K splits added up inside a cluster
+//   up to 128 rows or so    gemm_tc_f16_kernel below (and SINGLE_*): one CTA per tile, K splits over the grid, sums finished by a second
+//                           kernel. (With the sums inside a cluster, fetched since there is no room to send them, 128 rows of a layer's
+//                           projections took what they take here.)
+//   beyond                  gemm_tc_pair.cu: CTA pairs
+//
+// In all of them the weights are the MMA's A operand and the activations, split into 16-bit hi + lo parts, its B operand:
 //
 //   D[n_tile 128 x M_pad] (f32, in TMEM)  +=  W[128 x 64] (f16, smem, TMA 128B-swizzled)
 //                                            * Xt[64 x M_pad] (f16, smem, TMA 128B-swizzled)
 //
-// f32 activations are split into f16 hi + lo parts (two MMAs per k-step; tensor time is free while the
-// kernel is HBM-bound), so results keep f32-level accuracy for small batches.
-//
-// Roles inside a CTA (6 warps): warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner, warps 2..5 =
-// epilogue (TMEM -> registers -> global partials). Up to three weight matrices that share the
-// activations (Wq|Wk|Wv, Wgate|Wup) are one launch; K is split over grid.y so that about two CTAs per
-// SM are resident. Partials land in scratch and a small second kernel adds the K splits and applies the
-// epilogue (bias, residual, or SiLU(gate)*up).
-//
+// Roles in gemm_tc_f16_kernel (6 warps): warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner, warps 2..5 = epilogue (TMEM ->
+// registers -> global partials). Up to three weight matrices that share the activations (Wq|Wk|Wv, Wgate|Wup) are one launch.
 // Whenever one problem needs no K split, the epilogue warps apply bias, post norm, residual and soft cap themselves and store
-// the result: no partials, no second kernel. Most calls of more than 128 rows go to the CTA-pair kernel (gemm_tc_pair.cu).
+// the result: no partials, no second kernel.
 //
 // Every wait is bounded: a wait that runs out sets bit 2 of the context's device status word, the
 // CTA stops issuing work, frees its TMEM and returns.
@@ -27,6 +24,7 @@
 #include "common.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_tc_pair.cuh"
+#include "gemm_tc_rows.cuh"
 #include "tc_ptx.cuh"
 
 namespace {
@@ -312,7 +310,8 @@ __global__ void __launch_bounds__(256) norm_split_rows_kernel(const float* __res
         split_store4(*reinterpret_cast<const float4*>(xr + k), norm_w4(w, w_f32, k), scale, hr + k, lr + k);
 }
 
-// Rows of any pitch -> hi / lo copies of type T, with an optional dynamic tanh or RMS norm. One CTA per row.
+// Rows of any pitch -> hi / lo copies of type T, with an RMS or polynomial norm. One CTA per row; few rows get wide CTAs, since what counts
+// there is how long one row takes (5632 columns, polynomial norm, 256 threads: 6 us in a chain of 32-row calls).
 template <typename T>
 __device__ __forceinline__ T to_half_type(float v);
 template <>
@@ -331,8 +330,9 @@ struct SplitRowsArgs {
     float eps, alpha;
 };
 template <typename T>
-__global__ void __launch_bounds__(256) split_rows_kernel(SplitRowsArgs a, T* __restrict__ hi, T* __restrict__ lo) {
-    __shared__ float red[8], red2[8], red3[8];
+__global__ void __launch_bounds__(1024) split_rows_kernel(SplitRowsArgs a, T* __restrict__ hi, T* __restrict__ lo) {
+    __shared__ float red[32], red2[32], red3[32];
+    const uint32_t stride = blockDim.x * 4u, warps = blockDim.x / 32u;
     pdl_wait();
     pdl_trigger();
     const float* xr = a.x + (size_t)blockIdx.x * a.ldx;
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(256) split_rows_kernel(SplitRowsArgs a, T* __r
     float scale = 1.0f;
     if (a.kind == (int)M40LLM_NORM_RMS) {
         float ss = 0.0f;
-        for (uint32_t k = threadIdx.x * 4u; k < a.K; k += 1024u) {
+        for (uint32_t k = threadIdx.x * 4u; k < a.K; k += stride) {
             const float4 v = *reinterpret_cast<const float4*>(xr + k);
             ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
         }
@@ -349,15 +349,14 @@ __global__ void __launch_bounds__(256) split_rows_kernel(SplitRowsArgs a, T* __r
         if ((threadIdx.x & 31u) == 0u) red[threadIdx.x >> 5] = ss;
         __syncthreads();
         float tot = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) tot += red[i];
+        for (uint32_t i = 0; i < warps; ++i) tot += red[i];
         scale = rsqrtf(tot / (float)a.K + a.eps);
     }
     const float* wf = reinterpret_cast<const float*>(a.w);
     float4 poly = make_float4(0.f, 0.f, 0.f, 0.f);
     if (a.kind == (int)M40LLM_NORM_POLY) {
         float s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
-        for (uint32_t k = threadIdx.x * 4u; k < a.K; k += 1024u) {
+        for (uint32_t k = threadIdx.x * 4u; k < a.K; k += stride) {
             const float4 v = *reinterpret_cast<const float4*>(xr + k);
             const float z[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -370,26 +369,18 @@ __global__ void __launch_bounds__(256) split_rows_kernel(SplitRowsArgs a, T* __r
         if ((threadIdx.x & 31u) == 0u) red[threadIdx.x >> 5] = s1, red2[threadIdx.x >> 5] = s2, red3[threadIdx.x >> 5] = s3;
         __syncthreads();
         s1 = s2 = s3 = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) s1 += red[i], s2 += red2[i], s3 += red3[i];
+        for (uint32_t i = 0; i < warps; ++i) s1 += red[i], s2 += red2[i], s3 += red3[i];
         poly = m40_poly_scales(wf, s1, s2, s3, (float)a.K, a.eps);
     }
-    for (uint32_t k = threadIdx.x * 4u; k < a.K; k += 1024u) {
+    for (uint32_t k = threadIdx.x * 4u; k < a.K; k += stride) {
         const float4 v = *reinterpret_cast<const float4*>(xr + k);
         float y[4] = {v.x, v.y, v.z, v.w};
-        if (a.kind == (int)M40LLM_NORM_DYT) {
-            const float4 w = m40_vec4_or(wf, k, 1.0f), b = m40_vec4_or(a.b, k, 0.0f);
-            y[0] = tanhf(a.alpha * y[0]) * w.x + b.x, y[1] = tanhf(a.alpha * y[1]) * w.y + b.y;
-            y[2] = tanhf(a.alpha * y[2]) * w.z + b.z, y[3] = tanhf(a.alpha * y[3]) * w.w + b.w;
-        } else if (a.kind == (int)M40LLM_NORM_RMS) {
+        if (a.kind == (int)M40LLM_NORM_RMS) {
             const float4 w = norm_w4(a.w, a.w_f32, k);
             y[0] *= scale * w.x, y[1] *= scale * w.y, y[2] *= scale * w.z, y[3] *= scale * w.w;
         } else if (a.kind == (int)M40LLM_NORM_POLY) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) y[i] = m40_poly(poly, y[i]);
-        } else if (a.kind == (int)M40LLM_NORM_ACT) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) y[i] = m40_act(a.act, y[i]);
         }
         T h[4], l[4];
 #pragma unroll
@@ -400,6 +391,36 @@ __global__ void __launch_bounds__(256) split_rows_kernel(SplitRowsArgs a, T* __r
         *reinterpret_cast<uint2*>(hr + k) = *reinterpret_cast<const uint2*>(h);
         *reinterpret_cast<uint2*>(lr + k) = *reinterpret_cast<const uint2*>(l);
     }
+}
+
+// The same where a value does not depend on its row's others: CTA = 1024 columns of a row, so that one row does not wait for one CTA
+// (16 x 4096 with a dynamic tanh: 6.4 us with a CTA per row).
+template <typename T>
+__global__ void __launch_bounds__(256) split_columns_kernel(SplitRowsArgs a, T* __restrict__ hi, T* __restrict__ lo) {
+    pdl_trigger();
+    const uint32_t k = (blockIdx.y * 256u + threadIdx.x) * 4u, kk = k < a.K ? k : 0u;
+    const float* wf = reinterpret_cast<const float*>(a.w);
+    float4 w = make_float4(1.f, 1.f, 1.f, 1.f), b = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (a.kind == (int)M40LLM_NORM_DYT) w = m40_vec4_or(wf, kk, 1.0f), b = m40_vec4_or(a.b, kk, 0.0f);
+    pdl_wait();
+    const float4 v = *reinterpret_cast<const float4*>(a.x + (size_t)blockIdx.x * a.ldx + kk);
+    float y[4] = {v.x, v.y, v.z, v.w};
+    if (a.kind == (int)M40LLM_NORM_DYT) {
+        y[0] = tanhf(a.alpha * y[0]) * w.x + b.x, y[1] = tanhf(a.alpha * y[1]) * w.y + b.y;
+        y[2] = tanhf(a.alpha * y[2]) * w.z + b.z, y[3] = tanhf(a.alpha * y[3]) * w.w + b.w;
+    } else if (a.kind == (int)M40LLM_NORM_ACT) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y[i] = m40_act(a.act, y[i]);
+    }
+    if (k >= a.K) return;
+    T h[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        h[i] = to_half_type<T>(y[i]);
+        l[i] = to_half_type<T>(y[i] - m40_load_elem(&h[i]));
+    }
+    *reinterpret_cast<uint2*>(hi + (size_t)blockIdx.x * a.K + k) = *reinterpret_cast<const uint2*>(h);
+    *reinterpret_cast<uint2*>(lo + (size_t)blockIdx.x * a.K + k) = *reinterpret_cast<const uint2*>(l);
 }
 
 // Adds the K splits and applies the epilogue. Thread (n, lane of 2) walks 8 activation rows of one problem.
@@ -537,6 +558,112 @@ bool make_map_f16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t co
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// x (with its norm) -> hi and lo copies [M][K] of the weights' type.
+int split_rows(M40llmCudaContext* ctx, cudaStream_t s, const float* X, int M, int K, const M40GemvNorm* norm, const M40TcExt* ext, __half* xh,
+               __half* xl) {
+    if (!ext) return m40_split_activations(ctx, s, X, xh, xl, M, K, norm);
+    SplitRowsArgs sa = {};
+    sa.x = X;
+    sa.K = (uint32_t)K;
+    sa.ldx = ext->ldx ? (uint32_t)ext->ldx : (uint32_t)K;
+    if (K % 4 != 0 || sa.ldx % 4 != 0 || (((uintptr_t)X) & 15u) != 0u) return -2;
+    if (norm && norm->special) {
+        sa.kind = norm->special;
+        sa.act = norm->act;
+        sa.w = norm->w;
+        sa.eps = norm->eps;
+    } else if (norm && norm->dyt) {
+        sa.kind = (int)M40LLM_NORM_DYT;
+        sa.w = norm->w;
+        sa.b = norm->b;
+        sa.alpha = norm->alpha;
+        if (((((uintptr_t)norm->w) | ((uintptr_t)norm->b)) & 15u) != 0u) return -2;
+    } else if (norm && norm->w) {
+        sa.kind = (int)M40LLM_NORM_RMS;
+        sa.w = norm->w;
+        sa.eps = norm->eps;
+        const bool w_vec = (((uintptr_t)norm->w) & (norm->w_is_f32 ? 15u : 7u)) == 0u;
+        sa.w_f32 = (norm->w_is_f32 ? 1 : 0) | (w_vec ? 0 : 2);
+    }
+    cudaError_t es;
+    if (sa.kind != (int)M40LLM_NORM_RMS && sa.kind != (int)M40LLM_NORM_POLY) {
+        const dim3 grid((unsigned)M, ((unsigned)K + 1023) / 1024);
+        es = ext->bf16 ? m40_launch_dependent(split_columns_kernel<__nv_bfloat16>, grid, dim3(256), 0, s, sa, (__nv_bfloat16*)xh, (__nv_bfloat16*)xl)
+                       : m40_launch_dependent(split_columns_kernel<__half>, grid, dim3(256), 0, s, sa, xh, xl);
+    } else {
+        const unsigned quads = ((unsigned)K / 4 + 31) / 32 * 32, threads = M <= 128 && quads > 256 ? (quads < 1024 ? quads : 1024) : 256;
+        es = ext->bf16 ? m40_launch_dependent(split_rows_kernel<__nv_bfloat16>, dim3((unsigned)M), dim3(threads), 0, s, sa, (__nv_bfloat16*)xh,
+                                              (__nv_bfloat16*)xl)
+                       : m40_launch_dependent(split_rows_kernel<__half>, dim3((unsigned)M), dim3(threads), 0, s, sa, xh, xl);
+    }
+    M40_COUNT_LAUNCH(ctx);
+    return es == cudaSuccess ? 0 : -2;
+}
+
+// Whether the rows kernel can split x itself: no norm, vector loads, and no result over x (other CTAs still read it).
+bool splits_inside(const float* X, int M, int K, const M40GemvNorm* norm, const M40TcExt* ext, int problems, const int* N, float* const* out,
+                   int mode) {
+    const size_t ldx = ext && ext->ldx ? (size_t)ext->ldx : (size_t)K;
+    if (ldx % 4 != 0 || (((uintptr_t)X) & 15u) != 0u) return false;
+    if (norm && (norm->w || norm->dyt || norm->special)) return false;
+    const uintptr_t x0 = (uintptr_t)X, x1 = x0 + (((size_t)M - 1) * ldx + K) * sizeof(float);
+    for (int p = 0; p < (mode == 1 ? 1 : problems); ++p) {
+        const uintptr_t o0 = (uintptr_t)out[p], o1 = o0 + (size_t)M * N[p] * sizeof(float);
+        if (out[p] && o0 < x1 && x0 < o1) return false;
+    }
+    return true;
+}
+
+// Up to M40_ROWS_MAX rows.
+int gemm_rows(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind, const float* X, int M, int K, int problems, const __half* const* W,
+              const int* N, float* const* out, const float* const* bias, const float* const* residual, int mode, const M40GemvNorm* norm,
+              const M40TcRopeAppend* rope, const M40TcExt* ext) {
+    const bool bf16 = ext && ext->bf16, inside = splits_inside(X, M, K, norm, ext, problems, N, out, mode);
+    M40RowsArgs a = {};
+    a.M = (uint32_t)M;
+    a.K = (uint32_t)K;
+    a.problems = (uint32_t)problems;
+    a.paired = mode == 1 ? 1u : 0u;
+    a.fmt_bits = bf16 ? idesc_bf16() : 0u;
+    CUtensorMap w[3], xh = {}, xl = {};
+    for (int p = 0; p < 3; ++p) {
+        const int q = p < problems ? p : 0;
+        if (!make_map_f16(&w[p], W[q], (uint64_t)N[q], (uint64_t)K, a.paired ? BLOCK_N / 2 : BLOCK_N, bf16)) return -2;
+        if (p >= problems) continue;
+        a.N[p] = (uint32_t)N[p];
+        a.out[p] = out[p];
+        a.bias[p] = bias ? bias[p] : nullptr;
+        a.residual[p] = residual ? residual[p] : nullptr;
+    }
+    if (inside) {
+        a.x = X;
+        a.ldx = ext && ext->ldx ? (uint32_t)ext->ldx : (uint32_t)K;
+        xh = xl = w[0];  // not used
+    } else {
+        const size_t act_bytes = (((size_t)M * K * 2 + 255) / 256) * 256;
+        unsigned char* scratch = (unsigned char*)m40_ensure_scratch(ctx, stream_kind, 2 * act_bytes);
+        if (!scratch) return -2;
+        const uint32_t box = ((uint32_t)M + 15) / 16 * 16;
+        if (!make_map_f16(&xh, scratch, (uint64_t)M, (uint64_t)K, box, bf16) ||
+            !make_map_f16(&xl, scratch + act_bytes, (uint64_t)M, (uint64_t)K, box, bf16))
+            return -2;
+        if (split_rows(ctx, s, X, M, K, norm, ext, (__half*)scratch, (__half*)(scratch + act_bytes)) != 0) return -2;
+    }
+    if (ext) {
+        a.act = ext->act;
+        if (mode == 0 && problems == 1) {
+            a.tail = ext->tail;
+            a.post_w = ext->post_w;
+            a.post_b = ext->post_b;
+        }
+    }
+    if (rope) {
+        a.rope_on = 1u;
+        a.rope = *rope;
+    }
+    return m40_rows_launch(ctx, s, !inside ? M40_ROWS_SPLIT : (bf16 ? M40_ROWS_BF16 : M40_ROWS_F16), w, xh, xl, a);
+}
+
 }  // namespace
 
 bool m40_tc_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, bool bf16) {
@@ -579,6 +706,7 @@ int m40_gemm_tc_f16(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind
         for (int p = 0; p < 3; ++p)
             if (N[p] % 128 != 0 || N[p] % (int)rope->head_dim != 0) return -2;
     }
+    if ((uint32_t)M <= M40_ROWS_MAX) return gemm_rows(ctx, s, stream_kind, X, M, K, problems, W, N, out, bias, residual, mode, norm, rope, ext);
     const uint32_t M_pad = ((uint32_t)M + 15) / 16 * 16;
     TcArgs a = {};
     a.fmt_bits = bf16 ? idesc_bf16() : 0u;
@@ -645,39 +773,7 @@ int m40_gemm_tc_f16(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind
     if (!make_map_f16(&mXh, xh, (uint64_t)M, (uint64_t)K, x_box, bf16)) return -2;
     if (!make_map_f16(&mXl, xl, (uint64_t)M, (uint64_t)K, x_box, bf16)) return -2;
 
-    if (ext) {
-        SplitRowsArgs sa = {};
-        sa.x = X;
-        sa.K = (uint32_t)K;
-        sa.ldx = ext->ldx ? (uint32_t)ext->ldx : (uint32_t)K;
-        if (K % 4 != 0 || sa.ldx % 4 != 0 || (((uintptr_t)X) & 15u) != 0u) return -2;
-        if (norm && norm->special) {
-            sa.kind = norm->special;
-            sa.act = norm->act;
-            sa.w = norm->w;
-            sa.eps = norm->eps;
-        } else if (norm && norm->dyt) {
-            sa.kind = (int)M40LLM_NORM_DYT;
-            sa.w = norm->w;
-            sa.b = norm->b;
-            sa.alpha = norm->alpha;
-            if (((((uintptr_t)norm->w) | ((uintptr_t)norm->b)) & 15u) != 0u) return -2;
-        } else if (norm && norm->w) {
-            sa.kind = (int)M40LLM_NORM_RMS;
-            sa.w = norm->w;
-            sa.eps = norm->eps;
-            const bool w_vec = (((uintptr_t)norm->w) & (norm->w_is_f32 ? 15u : 7u)) == 0u;
-            sa.w_f32 = (norm->w_is_f32 ? 1 : 0) | (w_vec ? 0 : 2);
-        }
-        const cudaError_t es =
-            bf16 ? m40_launch_dependent(split_rows_kernel<__nv_bfloat16>, dim3((unsigned)M), dim3(256), 0, s, sa,
-                                        (__nv_bfloat16*)xh, (__nv_bfloat16*)xl)
-                 : m40_launch_dependent(split_rows_kernel<__half>, dim3((unsigned)M), dim3(256), 0, s, sa, xh, xl);
-        M40_COUNT_LAUNCH(ctx);
-        if (es != cudaSuccess) return -2;
-    } else if (m40_split_activations(ctx, s, X, xh, xl, M, K, norm) != 0) {
-        return -2;
-    }
+    if (split_rows(ctx, s, X, M, K, norm, ext, xh, xl) != 0) return -2;
     if (ext) a.tail = ext->tail;
     if (direct) {
         a.direct = 1u;

@@ -86,6 +86,56 @@ def test_linear_gated(nat, rows, n, k, act, fn):
         close(got, fn(h @ w.T.astype(np.float64)) * (h @ w2.T.astype(np.float64)), 3e-6 if exact else 6e-5, f"exact={exact}")
 
 
+@pytest.mark.parametrize("rows", [2, 15, 16, 17, 31, 32])
+@pytest.mark.parametrize("n,k", [(130, 2112), (2050, 5640), (6176, 1096), (300, 256), (19200, 72)])
+@pytest.mark.parametrize("wdt", [N.DT_BF16, N.DT_F16])
+def test_linear_few_rows(nat, rows, n, k, wdt):
+    """Tiles that are not full, one to eight K splits of one to twelve rounds of the ring, shares of rows that do not divide. Limits as
+    below for many rows; they grow with the largest of some thousand outputs, which are near 1."""
+    rng = np.random.default_rng(rows + n)
+    x, w = rng.standard_normal((rows, k)).astype(np.float32), rounded(rng, wdt, n, k)
+    res = rng.standard_normal((rows, n))
+    tol = 8e-6 if wdt == N.DT_BF16 else 2e-6
+    y = x.astype(np.float64) @ w.T.astype(np.float64)
+    close(run_linear(nat, x, w, wdt, rows, residual=res), y + res, tol, "plain, residual in place")
+    act = dict(kind=N.NORM_ACT)
+    h = x.astype(np.float64) * S.sigmoid(x.astype(np.float64))
+    close(run_linear(nat, x, w, wdt, rows, pre=act), h @ w.T.astype(np.float64), tol, "activation before")
+    if n % 2 == 0 and n < 10000:
+        y2 = x.astype(np.float64) @ w[n // 2:].T.astype(np.float64)
+        close(run_linear(nat, x, w[:n // 2], wdt, rows, w2=w[n // 2:]), y[:, :n // 2] * S.sigmoid(y[:, :n // 2]) * y2, 4 * tol, "gated")
+
+
+def test_linear_few_rows_chain_and_in_place(nat):
+    """Projections that feed one another, replayed as a graph so that each starts beside the one before; the last one's result lies over
+    its own input."""
+    rng = np.random.default_rng(11)
+    for rows in (16, 32):
+        k, f = 1024, 5632
+        x = rng.standard_normal((rows, k)).astype(np.float32)
+        up, down, sq = (rounded(rng, N.DT_BF16, *shape) for shape in ((f, k), (k, f), (k, k)))
+        d = {n: nat.buf(f32_to_bf16(a)).ptr for n, a in (("up", up), ("down", down), ("sq", sq))}
+        src, hid, y = nat.buf(x), nat.buf(rows * f * 4), nat.buf(rows * k * 4)
+        call = lambda i, w, o, n, kk: N.Linear(i.ptr, d[w], None, o.ptr, None, None, N.Norm(), N.Norm(), rows, kk, n, 0, N.DT_BF16, 0, 0, 0.0)
+        calls = [call(src, "up", hid, f, k), call(hid, "down", y, k, f), call(y, "sq", y, k, k)] * 4
+        step = lambda: [nat.lib.m40llm_linear_async(nat.ctx, C.byref(c), 1) for c in calls]
+        assert not any(step())
+        nat.sync(1)
+        graph = C.c_void_p()
+        assert nat.lib.m40llm_cuda_graph_begin_capture(nat.ctx, 1) == 0
+        assert not any(step())
+        assert nat.lib.m40llm_cuda_graph_end_capture(nat.ctx, 1, C.byref(graph)) == 0
+        for _ in range(3):
+            assert nat.lib.m40llm_cuda_graph_launch(nat.ctx, graph, 1) == 0
+        nat.sync(1)
+        got = y.download(np.float32, (rows, k))
+        nat.lib.m40llm_cuda_graph_destroy(graph)
+        nat.free_all()
+        no_status(nat)
+        want = x.astype(np.float64) @ up.T.astype(np.float64) @ down.T.astype(np.float64) @ sq.T.astype(np.float64)
+        close(got, want, 2.5e-5, f"{rows} rows")  # three roundings of 8e-6
+
+
 @pytest.mark.parametrize("rows", [129, 256, 257, 511, 1030])
 @pytest.mark.parametrize("n,k", [(255, 1000), (257, 64), (640, 2120)])
 @pytest.mark.parametrize("wdt", [N.DT_BF16, N.DT_F16])

@@ -1,6 +1,7 @@
 """Rules of the kernels that cannot be shown by running them without hanging a GPU: read from their sources."""
 import glob
 import os
+import random
 import re
 
 import pytest
@@ -52,3 +53,37 @@ def test_unbounded_barriers_do_not_hang_on_a_wait_that_ran_out():
         end = body.rindex("__syncthreads();")
         assert re.search(r"if \(abort_flag\b", body[end:]) and "_full[i]" in body[end:] or "&full[s]" in body[end:]
     assert "a.status" not in pair[:pair.rindex("__syncthreads();")]
+
+
+def test_ring_of_the_few_rows_kernel():
+    """Four warps write every fourth k-block of the activation operand and wait by parity for the stage's last use only. Any order in
+    which they and the issuing warp may run, on every ring that the launch allows: no stage is overwritten early, none waits for good."""
+    source = plain(os.path.join(CSRC, "gemm_tc_rows.cu"))
+    low, high = (int(re.search(rf"{n} = (\d+)", source).group(1)) for n in ("MIN_STAGES", "MAX_STAGES"))
+    assert "a.stages < MIN_STAGES" in source
+
+    def run(stages, blocks, rng):
+        freed, filled, holds, done = [0] * stages, [0] * stages, {}, 0
+        at = list(range(4))  # each warp's next k-block
+        while done < blocks:
+            ready = [w for w in range(4) if at[w] < blocks and
+                     (at[w] < stages or freed[at[w] % stages] % 2 != (at[w] // stages - 1) % 2)]
+            if filled[done % stages] % 2 != done // stages % 2:
+                ready.append(4)
+            assert ready, (stages, blocks, done)
+            w = rng.choice(ready)
+            if w == 4:
+                assert holds[done % stages] == done
+                freed[done % stages] += 1
+                done += 1
+            else:
+                assert at[w] - stages < done
+                holds[at[w] % stages] = at[w]
+                filled[at[w] % stages] += 1
+                at[w] += 4
+
+    rng = random.Random(1)
+    for stages in range(low, high + 1):
+        for blocks in (1, 2, 3, 4, 5, 7, 11, 13, 28, 56):
+            for _ in range(20):
+                run(stages, blocks, rng)
