@@ -33,6 +33,7 @@ public:
         mma_.add(64, rows, pos, times);
     }
 
+    double tc_tiles() const { return heads_ * tc_.ctas; }
     double tc_us() const {
         return hd_ == 128 ? tc_.us(*this, 8.5, 1.45, 8.5, 1.45, 0.9, false) : tc_.us(*this, 7.3, 1.25, 7.3, 1.25, 0.9, false);
     }

@@ -53,6 +53,19 @@ def test_prefill_shapes(nat, O, qh, kvh, hd, pairs):
     nat.free_all()
 
 
+@pytest.mark.parametrize("qh,kvh,hd,pairs", [
+    (32, 8, 128, [(700, 700), (513, 1500)]),                      # pairs of heads
+    (32, 4, 64, [(1001, 1001), (640, 2000)]),
+    (40, 40, 64, [(769, 800), (640, 640), (1, 50)]),              # one head per group: rows that follow one another, whole and single tiles
+    (33, 11, 128, [(897, 1000), (600, 600)]),                     # three heads per group
+])
+def test_prefill_two_row_tiles(nat, O, qh, kvh, hd, pairs):
+    """More row tiles than SMs: a CTA works on two of them."""
+    got, exp = run_prefill(nat, O, qh, kvh, hd, pairs, qh + hd)
+    assert_close(got, exp, what=f"prefill {qh}/{kvh} d{hd} {pairs}")
+    nat.free_all()
+
+
 def test_prefill_full_length_and_last_row_equals_decode(nat, O):
     """Maximum kv length the reference admits (8192), and the last q row of a prefill equals last-token decode
     attention over the same keys and values (after their f16 rounding by the cache)."""
