@@ -308,6 +308,57 @@ bool prefill_configure(int device_id) {
     return true;
 }
 
+__global__ void __launch_bounds__(256) collect_lengths_kernel(const uint32_t* q_lens, const uint32_t* kv_lens, const uint32_t* kv_offsets,
+                                                              uint32_t n, uint32_t* dst) {
+    for (uint32_t i = threadIdx.x; i < n; i += 256u) {
+        dst[i] = q_lens[i];
+        dst[n + i] = kv_lens[i];
+        dst[2 * n + i] = kv_offsets[i];
+    }
+}
+
+// The lengths of a packed call on the host. One kernel writes them to the context's mapped memory: three copies to pageable memory each
+// wait for the one before, 50 us of a 290 us call. Where another thread has that memory, or a call has more sequences than fit, they are
+// copied all the same.
+class Lengths {
+public:
+    Lengths(M40llmCudaContext* ctx, uint32_t n) : ctx_(ctx), n_(n) {
+        mapped_ = ctx->readback && (uint64_t)n * 3 <= M40_READBACK && __atomic_exchange_n(&ctx->readback_taken, 1, __ATOMIC_ACQUIRE) == 0;
+    }
+    ~Lengths() { release(); }
+    Lengths(const Lengths&) = delete;
+    Lengths& operator=(const Lengths&) = delete;
+    // Waits for the stream. Null: a call failed.
+    const uint32_t* read(cudaStream_t s, const uint32_t* q_lens, const uint32_t* kv_lens, const uint32_t* kv_offsets) {
+        bool ok;
+        if (mapped_) {
+            collect_lengths_kernel<<<1, 256, 0, s>>>(q_lens, kv_lens, kv_offsets, n_, ctx_->d_readback);
+            M40_COUNT_LAUNCH(ctx_);
+            ok = cudaGetLastError() == cudaSuccess;
+        } else {
+            own_ = (uint32_t*)malloc((size_t)n_ * 3 * sizeof(uint32_t));
+            ok = own_ && cudaMemcpyAsync(own_, q_lens, (size_t)n_ * 4, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+                 cudaMemcpyAsync(own_ + n_, kv_lens, (size_t)n_ * 4, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+                 cudaMemcpyAsync(own_ + 2 * (size_t)n_, kv_offsets, (size_t)n_ * 4, cudaMemcpyDeviceToHost, s) == cudaSuccess;
+        }
+        ok = ok && cudaStreamSynchronize(s) == cudaSuccess;
+        if (!ok) cudaGetLastError();
+        return ok ? (mapped_ ? ctx_->readback : own_) : nullptr;
+    }
+    void release() {
+        free(own_);
+        own_ = nullptr;
+        if (mapped_) __atomic_store_n(&ctx_->readback_taken, 0, __ATOMIC_RELEASE);
+        mapped_ = false;
+    }
+
+private:
+    M40llmCudaContext* ctx_;
+    uint32_t n_;
+    bool mapped_;
+    uint32_t* own_ = nullptr;
+};
+
 M40PromptCost prompt_cost(const M40llmCudaContext* ctx, const M40PrefillCall& c) {
     M40PromptCost cost(c.hd, c.q_heads, c.kv_heads, (uint32_t)ctx->sm_count, c.max_segment_rows);
     if (c.seg_host)
@@ -409,18 +460,12 @@ int m40llm_attention_prefill_f32_gqa_varlen_async(M40llmCudaContext* ctx, const 
     cudaStream_t s = ctx->prefill_stream;
     // The grid needs the longest q run, and the reference validates every pair of lengths on the host
     // (kernels.cu:4861-4886): the lengths are read back behind whatever the prefill stream still holds.
-    uint32_t* lens = (uint32_t*)malloc((size_t)batch_size * 3 * sizeof(uint32_t));
+    Lengths lengths(ctx, batch_size);
+    const uint32_t* lens = lengths.read(s, d_q_lens, d_kv_lens, d_kv_offsets);
     if (!lens) return -7;
     int rc = 0;
     uint32_t max_q = 0;
     uint64_t total_kv = 0;  // rows of K / V the sequences reach: the extent of the f16 copies
-    if (cudaMemcpyAsync(lens, d_q_lens, (size_t)batch_size * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemcpyAsync(lens + batch_size, d_kv_lens, (size_t)batch_size * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemcpyAsync(lens + 2 * batch_size, d_kv_offsets, (size_t)batch_size * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess) {
-        cudaGetLastError();
-        rc = -7;
-    }
     for (uint32_t i = 0; rc == 0 && i < batch_size; ++i) {
         const uint32_t ql = lens[i], kl = lens[batch_size + i];
         if (ql == 0 || kl == 0 || ql > kl || kl > 8192) rc = -8;
@@ -430,7 +475,7 @@ int m40llm_attention_prefill_f32_gqa_varlen_async(M40llmCudaContext* ctx, const 
     }
     M40PromptCost cost(head_dim, q_heads, kv_heads, (uint32_t)ctx->sm_count, max_q);
     for (uint32_t i = 0; rc == 0 && i < batch_size; ++i) cost.add(lens[i], lens[batch_size + i] - lens[i]);
-    free(lens);
+    lengths.release();
     if (rc != 0) return rc;
     // f16 copies of K and V in the prefill stream's scratch
     const size_t kv_elems = (size_t)total_kv * kv_heads * head_dim;

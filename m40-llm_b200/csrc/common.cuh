@@ -46,6 +46,10 @@ struct M40llmCudaContext {
     // Device status word (bit 0: a batched-attention row was out of range and skipped).
     uint32_t* d_status;
     unsigned long long launches;
+    // Mapped host memory for lengths that a call reads back, M40_READBACK values, or null; one call at a time has it (readback_taken).
+    uint32_t* readback;
+    uint32_t* d_readback;
+    int readback_taken;
     // Inverse RoPE frequencies per (base, head_dim), made on the host (see m40_rope_inv_freq) and kept on the device.
     float* d_rope_inv_freq[4];
     float rope_table_base[4];
@@ -53,6 +57,8 @@ struct M40llmCudaContext {
     uint32_t rope_tables;
 };
 
+
+constexpr uint32_t M40_READBACK = 3072;
 
 struct M40llmCudaGraphExec {
     cudaGraph_t graph;

@@ -118,6 +118,12 @@ M40llmCudaContext* m40llm_create_context(int device_id) {
                    cudaSuccess;
     ok = ok && cudaMalloc(&ctx->d_selected_scores, (size_t)ctx->selected_capacity_heads * 64 * sizeof(float)) ==
                    cudaSuccess;
+    if (ok && (cudaHostAlloc((void**)&ctx->readback, M40_READBACK * sizeof(uint32_t), cudaHostAllocMapped) != cudaSuccess ||
+               cudaHostGetDevicePointer((void**)&ctx->d_readback, ctx->readback, 0) != cudaSuccess)) {
+        cudaGetLastError();  // calls do without it
+        if (ctx->readback) cudaFreeHost(ctx->readback);
+        ctx->readback = nullptr;
+    }
     if (ok) {
         cudaMemset(ctx->d_selected_blocks, 0xff, (size_t)ctx->selected_capacity_heads * 64 * sizeof(uint32_t));
         cudaMemset(ctx->d_selected_scores, 0, (size_t)ctx->selected_capacity_heads * 64 * sizeof(float));
@@ -149,6 +155,7 @@ void m40llm_destroy_context(M40llmCudaContext* ctx) {
         free(r);
     }
     if (ctx->d_status) cudaFree(ctx->d_status);
+    if (ctx->readback) cudaFreeHost(ctx->readback);
     if (ctx->d_selected_blocks) cudaFree(ctx->d_selected_blocks);
     if (ctx->d_selected_scores) cudaFree(ctx->d_selected_scores);
     if (ctx->prefill_waits_decode_event) cudaEventDestroy(ctx->prefill_waits_decode_event);
