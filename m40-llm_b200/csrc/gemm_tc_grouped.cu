@@ -48,7 +48,8 @@ __device__ __forceinline__ void store_split<__nv_bfloat16>(__nv_bfloat16* hi, __
     lo[at] = __float2bfloat16_rn(v - __bfloat162float(h));
 }
 
-template <int KIND>
+// STEP (with RG): every row is the next token of its own sequence, and the kernel makes the step.
+template <int KIND, bool STEP>
 __global__ void __launch_bounds__(192, 1) gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap tmW,
                                                                  const __grid_constant__ CUtensorMap tmW2,
                                                                  const __grid_constant__ CUtensorMap tmX0,
@@ -150,6 +151,15 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_grouped_kernel(const __grid_co
     } else {
         const uint32_t lane_group = warp & 3u, row_of_tile = lane_group * 32u + lane;  // weight row of the tile
         pdl_wait();
+        // RG: lanes 0..63 hold r sums, 64..127 the i sums of the same channels; each half finishes half of the rows
+        const uint32_t ch = row_of_tile & 63u, half = a.tile_rows / 2u;
+        const bool is_i = row_of_tile >= 64u;
+        const uint32_t mine = is_i ? half : 0u, other = is_i ? 0u : half;
+        const uint32_t chan = PAIRED ? x_col + (n0 + ch < a.N ? n0 + ch : 0u) : 0u;
+        M40RgStep st[8];
+        float u[8];
+        if (STEP && mine < m_live)  // tiles of 16 rows: one round, fetched while the products are made
+            m40_rg_fetch8(a.rg, m_base + mine, m_live - mine, chan, st, u);
         bool ok = mbar_wait(accum, 0);
         if (!ok) *abort_flag = 1;
         ok = __all_sync(0xffffffffu, ok);
@@ -167,12 +177,9 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_grouped_kernel(const __grid_co
             }
         };
         if constexpr (PAIRED) {
-            // lanes 0..63 hold r sums, 64..127 the i sums of the same channels. Each half finishes half of the rows and hands
-            // the other half's sums over through shared memory (the ring is free).
+            // the other half's sums go over through shared memory (the ring is free)
             float* xs = reinterpret_cast<float*>(smem);  // [tile_rows][64]
-            const uint32_t ch = row_of_tile & 63u, n = n0 + ch, half = a.tile_rows / 2u;
-            const bool is_i = row_of_tile >= 64u;
-            const uint32_t mine = is_i ? half : 0u, other = is_i ? 0u : half;
+            const uint32_t n = n0 + ch;
             for (uint32_t c = other; c < other + half; c += 8) {
                 float v[8];
                 sums(c, v);
@@ -182,17 +189,11 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_grouped_kernel(const __grid_co
             asm volatile("bar.sync 1, 128;" ::: "memory");
             const M40RgArgs& g = a.rg;
             const bool n_ok = n < a.N;
-            const uint32_t chan = x_col + (n_ok ? n : 0u);
             const float sp = m40_softplus(g.lam[chan]), rb = g.ra_b[chan], ib = g.ri_b[chan];
             for (uint32_t c = mine; c < mine + half; c += 8) {
-                float v[8], u[8];
+                float v[8];
                 sums(c, v);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) u[j] = g.u[(size_t)(m_base + min(c + j, m_live - 1u)) * g.width + chan];
-                if (g.step) {
-                    M40RgStep st[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) st[j] = m40_rg_fetch(g, m_base + min(c + j, m_live - 1u), chan);
+                if constexpr (STEP) {
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
                         if (!n_ok || c + j >= m_live) continue;
@@ -200,16 +201,18 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_grouped_kernel(const __grid_co
                         m40_rg_store(g, m_base + c + j, chan, st[j],
                                      m40_rg_gated(g, (is_i ? o : v[j]) + rb, (is_i ? v[j] : o) + ib, sp, u[j]));
                     }
-                    continue;
-                }
+                } else {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    if (!n_ok || c + j >= m_live) continue;
-                    const float o = xs[(c + j) * 64u + ch];
-                    const float2 ab = m40_rg_gated(g, (is_i ? o : v[j]) + rb, (is_i ? v[j] : o) + ib, sp, u[j]);
-                    const size_t at = (size_t)(m_base + c + j) * g.width + chan;
-                    g.a[at] = ab.x;
-                    g.b[at] = ab.y;
+                    for (int j = 0; j < 8; ++j) u[j] = g.u[(size_t)(m_base + min(c + j, m_live - 1u)) * g.width + chan];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        if (!n_ok || c + j >= m_live) continue;
+                        const float o = xs[(c + j) * 64u + ch];
+                        const float2 ab = m40_rg_gated(g, (is_i ? o : v[j]) + rb, (is_i ? v[j] : o) + ib, sp, u[j]);
+                        const size_t at = (size_t)(m_base + c + j) * g.width + chan;
+                        g.a[at] = ab.x;
+                        g.b[at] = ab.y;
+                    }
                 }
             }
         } else {
@@ -240,16 +243,16 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_grouped_kernel(const __grid_co
     }
 }
 
-template <int KIND>
+template <int KIND, bool STEP = false>
 int launch(M40llmCudaContext* ctx, cudaStream_t s, dim3 grid, size_t smem, const CUtensorMap* m, const GArgs& a) {
     static unsigned long long configured = 0ull;
     const unsigned long long bit = 1ull << (ctx->device_id & 63);
     if (!(configured & bit)) {
-        if (cudaFuncSetAttribute(gemm_tc_grouped_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
+        if (cudaFuncSetAttribute(gemm_tc_grouped_kernel<KIND, STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
             return -2;
         configured |= bit;
     }
-    const cudaError_t e = m40_launch_dependent(gemm_tc_grouped_kernel<KIND>, grid, dim3(192), smem, s, m[0], m[1], m[2], m[3], m[4], a);
+    const cudaError_t e = m40_launch_dependent(gemm_tc_grouped_kernel<KIND, STEP>, grid, dim3(192), smem, s, m[0], m[1], m[2], m[3], m[4], a);
     M40_COUNT_LAUNCH(ctx);
     return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -262,6 +265,7 @@ bool m40_gemm_tc_grouped_supported(const void* w, uint32_t N, uint32_t K, uint32
 }
 
 int m40_gemm_tc_grouped(M40llmCudaContext* ctx, cudaStream_t s, const M40GroupedCall& c) {
+    if (c.kind == M40_GROUPED_RG && c.rg.step && c.tile_rows != 16) return -2;  // a thread steps eight rows
     if (c.parts < 1 || c.parts > 3 || c.tile_rows * c.parts > 256 || c.tile_rows % 16 != 0 || c.K == 0 || c.x_rows == 0) return -2;
     const bool paired = c.kind == M40_GROUPED_RG;
     CUtensorMap m[5];
@@ -308,6 +312,6 @@ int m40_gemm_tc_grouped(M40llmCudaContext* ctx, cudaStream_t s, const M40Grouped
         case M40_GROUPED_F32: return launch<M40_GROUPED_F32>(ctx, s, grid, smem, m, a);
         case M40_GROUPED_ACT_SPLIT: return launch<M40_GROUPED_ACT_SPLIT>(ctx, s, grid, smem, m, a);
         case M40_GROUPED_HEADS: return launch<M40_GROUPED_HEADS>(ctx, s, grid, smem, m, a);
-        default: return launch<M40_GROUPED_RG>(ctx, s, grid, smem, m, a);
+        default: return c.rg.step ? launch<M40_GROUPED_RG, true>(ctx, s, grid, smem, m, a) : launch<M40_GROUPED_RG>(ctx, s, grid, smem, m, a);
     }
 }

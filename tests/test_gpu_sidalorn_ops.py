@@ -366,6 +366,41 @@ def test_rglru(nat, W, B, taps, exact):
     nat.free_all()
 
 
+@pytest.mark.parametrize("n", [8, 9, 16, 17, 33])
+def test_rglru_steps_of_many_sequences(nat, n):
+    """A step's tiles hold 16 rows, eight to a thread: full and ragged ones, the first token of a sequence among later ones."""
+    W, B, taps, T = 576, 4, 4, 4
+    rng = np.random.default_rng(n)
+    D = W // B
+    w = {"conv": 0.5 * rng.standard_normal((W, taps)), "conv.b": 0.3 * rng.standard_normal(W), "ra.b": rng.standard_normal((B, D)),
+         "ri.b": rng.standard_normal((B, D)), "lam": rng.uniform(-6, 6, W)}
+    w = {k: a.astype(np.float32) for k, a in w.items()}
+    for k in ("ra", "ri"):
+        w[k] = b16(1.5 * rng.standard_normal((B, D, D)) / D ** 0.5)
+    zeros = np.zeros(W)
+    ow = {k: a.astype(np.float64) for k, a in w.items()} | {
+        "y": np.concatenate([np.eye(W), np.zeros((W, W))], 1), "x": np.concatenate([np.zeros((W, W)), np.eye(W)], 1),
+        "y.b": zeros, "x.b": zeros, "o": np.eye(W)}
+    packed = rng.standard_normal((n, T, 2 * W)).astype(np.float32)
+    ref = [S.rglru(p, np.zeros(W), np.zeros((taps - 1, W)), ow, {"blocks": B})[0] for p in packed]
+    state = nat.lib.m40llm_statecache_create_values(nat.ctx, n, W * (1 + taps))
+    dev = [f32(nat, w["conv"]), f32(nat, w["conv.b"]), bits(nat, w["ra"]), f32(nat, w["ra.b"]), bits(nat, w["ri"]), f32(nat, w["ri.b"]),
+           f32(nat, w["lam"])]
+    at = np.zeros(n, int)
+    for step in range(T):
+        live = [s for s in range(n) if step or s % 3]  # every third sequence begins one step later
+        rows = Rows(nat, [(s, at[s], 1) for s in live])
+        out = nat.buf(rows.n * W * 4)
+        c = N.RgLru(f32(nat, np.stack([packed[s, at[s]] for s in live])), *dev, out.ptr, 2 * W, W, B, taps, N.DT_BF16, 0, 8.0)
+        assert nat.lib.m40llm_rglru_async(nat.ctx, state, C.byref(c), C.byref(rows.c)) == 0
+        nat.sync(1)
+        close(out.download(np.float32, (rows.n, W)), np.stack([ref[s][at[s]] for s in live]), 2e-5, str(step))  # as in test_rglru
+        at[live] += 1
+    no_status(nat)
+    nat.lib.m40llm_statecache_destroy(state)
+    nat.free_all()
+
+
 def test_state_caches_do_not_mix(nat):
     st = nat.lib.m40llm_statecache_create_values(nat.ctx, 2, 64)
     out = np.zeros(64, np.float32)
