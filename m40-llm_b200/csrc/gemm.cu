@@ -412,15 +412,24 @@ int m40_gemm_f32xq80_gguf(M40llmCudaContext* ctx, cudaStream_t s, const float* A
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-// Q8_0 projections for batched rows on the tensor cores, 64 rows per pass. Returns 1 when not applicable.
+// Rows per pass: as many as a call takes, unless the scratch for them is not there (an arena does not grow while its stream is captured).
+static int q80_pass_rows(M40llmCudaContext* ctx, uint32_t stream_kind, int M, int K, int problems, const int* N) {
+    if (M <= 64) return 64;
+    size_t act, part;
+    m40_gemm_tc_q80_scratch(ctx, M < M40_Q80_PASS_ROWS ? M : M40_Q80_PASS_ROWS, K, problems, N, &act, &part);
+    return m40_ensure_scratch(ctx, stream_kind, 2 * act + part) ? M40_Q80_PASS_ROWS : 64;
+}
+
+// Q8_0 projections for batched rows on the tensor cores, in passes of up to M40_Q80_PASS_ROWS rows. Returns 1 when not applicable.
 static int q80_tc_rows(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind, const float* A, int M, int K,
                        int problems, const uint8_t* const* W, const int* N, float* const* out, const float* residual,
                        int mode, const M40GemvNorm* norm = nullptr, const M40TcChain* chain = nullptr) {
     const void* wp[3] = {W[0], problems > 1 ? W[1] : W[0], problems > 2 ? W[2] : W[0]};
     if (M < m40_tc_min_rows() || !m40_gemm_tc_q80_supported(M < 64 ? M : 64, K, problems, wp)) return 1;
-    if (norm && norm->w && M % 64 == 1) return 1;  // a single trailing row would need the un-normalised path
-    for (int m0 = 0; m0 < M; m0 += 64) {
-        const int rows = M - m0 < 64 ? M - m0 : 64;
+    const int pass = q80_pass_rows(ctx, stream_kind, M, K, problems, N);
+    if (norm && norm->w && M % pass == 1) return 1;  // a single trailing row would need the un-normalised path
+    for (int m0 = 0; m0 < M; m0 += pass) {
+        const int rows = M - m0 < pass ? M - m0 : pass;
         if (rows < 2) {  // a single trailing row: CUDA-core kernel
             if (mode == 1) {
                 const int rc1 = m40_gate_up_swiglu_q80(ctx, s, A + (size_t)m0 * K, W[0], W[1], out[0] + (size_t)m0 * N[0], 1, N[0], K);
@@ -441,7 +450,7 @@ static int q80_tc_rows(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_k
             r[p] = residual ? residual + (size_t)m0 * N[p] : nullptr;
         }
         const int rc = m40_gemm_tc_q80(ctx, s, stream_kind, A + (size_t)m0 * K, rows, K, problems, W, N, o, r, mode, norm,
-                                       M <= 64 ? chain : nullptr);
+                                       M <= pass ? chain : nullptr);
         if (rc != 0) return rc;
     }
     return 0;
@@ -557,13 +566,13 @@ int m40_ffn_swiglu(M40llmCudaContext* ctx, uint32_t stream_kind, const void* d_x
     const bool want_norm = norm && norm->w;
     int rc;
     if (q80) {
-        // One pass of up to 64 rows on the tensor cores: the SwiGLU epilogue hands the down projection its
+        // One pass on the tensor cores: the SwiGLU epilogue hands the down projection its
         // activations already split into f16 hi | lo (one launch and one pass over hid fewer).
         M40TcChain first = {}, second = {};
         bool chained = false;
         {
             const void* wp[3] = {d_wg, d_wu, d_wd};
-            if ((int)rows >= m40_tc_min_rows() && rows <= 64 && m40_gemm_tc_q80_supported((int)rows, (int)hidden, 2, wp) &&
+            if ((int)rows >= m40_tc_min_rows() && rows <= (uint32_t)M40_Q80_PASS_ROWS && m40_gemm_tc_q80_supported((int)rows, (int)hidden, 2, wp) &&
                 m40_gemm_tc_q80_supported((int)rows, (int)ffn, 1, wp + 2)) {
                 const int n1[2] = {(int)ffn, (int)ffn}, n2[1] = {(int)hidden};
                 size_t act1, part1, act2, part2;
@@ -576,7 +585,7 @@ int m40_ffn_swiglu(M40llmCudaContext* ctx, uint32_t stream_kind, const void* d_x
                 first.act_off = second.act_off = front;
                 first.write_split = 1;
                 second.read_split = 1;
-                chained = true;
+                chained = rows <= 64 || m40_ensure_scratch(ctx, stream_kind, first.scratch_bytes) != nullptr;
             }
         }
         {

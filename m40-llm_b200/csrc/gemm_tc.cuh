@@ -61,7 +61,8 @@ struct M40TcChain {
 void m40_gemm_tc_q80_scratch(const M40llmCudaContext* ctx, int M, int K, int problems, const int* N, size_t* act_bytes,
                              size_t* part_bytes);
 
-// Same over Q8_0 GGUF rows (K % 256 == 0, 2 <= M <= 64 per call). mode 0: out[p] = X.W[p]^T (+ residual[p]);
+constexpr int M40_Q80_PASS_ROWS = 128;
+// Same over Q8_0 GGUF rows (K % 256 == 0, 2 <= M <= M40_Q80_PASS_ROWS per call). mode 0: out[p] = X.W[p]^T (+ residual[p]);
 // mode 1: out[0] = silu(X.Wg^T) * (X.Wu^T).
 bool m40_gemm_tc_q80_supported(int M, int K, int problems, const void* const* W);
 int m40_gemm_tc_q80(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind, const float* X, int M, int K,

@@ -1,5 +1,7 @@
 """GEMV/GEMM entry points against the oracle (tests/gemm_mixed.rs, gemm_f16xf16_f32.rs, proj_wrappers.rs,
 mlp_wrappers.rs of the reference use 1e-3 absolute; here |a-e| <= 1e-3 + 2e-3|e|)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -82,6 +84,22 @@ def test_gemm_q80(nat, O, M, N, K):
     nat.free_all()
 
 
+@pytest.mark.parametrize("N,K", [(128, 256), (300, 512), (4096, 1024), (24, 14336)])
+def test_gemm_q80_forms_by_rows(nat, O, N, K):
+    """The row counts between which the kernel or the width of its tile changes; columns that end inside a tile, spans that end inside one."""
+    rng = np.random.default_rng(N + K)
+    wq = O.q80_quantize((rng.standard_normal((N, K)) * 0.02).astype(np.float32))
+    dw = nat.buf(wq)
+    a = rng.standard_normal((130, K)).astype(np.float32)
+    exp = O.gemm_f32xq80_gguf(a, wq, N)
+    for M in (2, 3, 7, 8, 9, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 130):
+        da, dc = nat.buf(a[:M]), nat.buf(M * N * 4)
+        assert nat.lib.m40llm_gemm_f32xq80_gguf_f32_async(nat.ctx, da.ptr, dw.ptr, dc.ptr, M, N, K, 1) == 0
+        nat.sync(1)
+        assert_close(dc.download(np.float32, (M, N)), exp[:M], what=f"q80 {M}x{N}x{K}")
+    nat.free_all()
+
+
 @pytest.mark.parametrize("rows,H,F,q80", [(1, 256, 384, True), (1, 4096, 14336, True), (4, 1024, 2816, True),
                                            (32, 4096, 14336, True), (8, 256, 512, True), (70, 512, 1024, True), (32, 2048, 5632, False),
                                            (128, 1024, 2816, True), (256, 512, 1024, True), (65, 512, 1024, True),
@@ -152,3 +170,38 @@ def test_one_row_streaming_shapes(nat, O, fmt, N, K):
     st = np.zeros(1, np.uint32)
     assert nat.lib.m40llm_context_take_device_status(nat.ctx, st.ctypes.data) == 0 and st[0] == 0
     nat.free_all()
+
+
+def test_q80_rows_captured_before_the_scratch_has_grown(pkg):
+    """The arena does not grow during capture: rows that one pass would need more scratch for go in two, as a call of that size always did."""
+    import helpers
+
+    rng = np.random.default_rng(3)
+    rows, H, F = 128, 4096, 14336
+
+    def blocks(n, k):
+        w = np.zeros((n, k // 32), np.dtype([("d", np.float16), ("q", np.int8, 32)]))
+        w["d"], w["q"] = 0.0005, rng.integers(-127, 128, w["q"].shape, np.int8)
+        return w.view(np.uint8)
+
+    own = helpers.Native(pkg.native.lib())
+    try:
+        x = rng.standard_normal((rows, H)).astype(np.float32)
+        dx, dg, du, dd = own.buf(x), own.buf(blocks(F, H)), own.buf(blocks(F, H)), own.buf(blocks(H, F))
+        dh, do, graph = own.buf(rows * F * 4), own.buf(rows * H * 4), C.c_void_p()
+        call = lambda: own.lib.m40llm_ffn_swiglu_q80_f32_async(own.ctx, dx.ptr, dg.ptr, du.ptr, dd.ptr, None, dh.ptr, do.ptr, rows, H, F, 1)
+        assert own.lib.m40llm_cuda_graph_begin_capture(own.ctx, 1) == 0
+        rc = call()
+        assert own.lib.m40llm_cuda_graph_end_capture(own.ctx, 1, C.byref(graph)) == 0 and rc == 0
+        assert own.lib.m40llm_cuda_graph_launch(own.ctx, graph, 1) == 0
+        own.sync(1)
+        captured = do.download(np.float32, (rows, H))
+        assert call() == 0
+        own.sync(1)
+        # f32 sums in another order; a pass's truncation leaves up to 4e-6 of the norm
+        eager = do.download(np.float32, (rows, H))
+        assert np.linalg.norm(captured - eager) <= 1e-5 * np.linalg.norm(eager)
+        own.lib.m40llm_cuda_graph_destroy(graph)
+    finally:
+        own.free_all()
+        own.lib.m40llm_destroy_context(own.ctx)
