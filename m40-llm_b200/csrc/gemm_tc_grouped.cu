@@ -100,31 +100,30 @@ __global__ void __launch_bounds__(192, 1) gemm_tc_grouped_kernel(const __grid_co
 
     if (warp == 0) {
         if (lane == 0) {
-            auto load_w = [&](uint32_t i) {
-                unsigned char* st = smem + (i % a.stages) * stage_bytes;
-                uint64_t* bar = &full[i % a.stages];
-                mbar_expect_tx(bar, stage_bytes);
-                tma_load_2d(st, &tmW, bar, (int)(i * BLOCK_K), (int)w_row);
-                if (PAIRED) tma_load_2d(st + a_bytes / 2, &tmW2, bar, (int)(i * BLOCK_K), (int)w_row);
+            auto load_w = [&](uint32_t i, uint32_t slot) {
+                unsigned char* st = smem + slot * stage_bytes;
+                mbar_expect_tx(&full[slot], stage_bytes);
+                tma_load_2d(st, &tmW, &full[slot], (int)(i * BLOCK_K), (int)w_row);
+                if (PAIRED) tma_load_2d(st + a_bytes / 2, &tmW2, &full[slot], (int)(i * BLOCK_K), (int)w_row);
             };
-            auto load_x = [&](uint32_t i) {
-                unsigned char* st = smem + (i % a.stages) * stage_bytes + a_bytes;
-                uint64_t* bar = &full[i % a.stages];
+            auto load_x = [&](uint32_t i, uint32_t slot) {
+                unsigned char* st = smem + slot * stage_bytes + a_bytes;
                 const int kx = (int)(x_col + i * BLOCK_K);
-                tma_load_2d(st, &tmX0, bar, kx, (int)m_base);
-                if (a.parts > 1) tma_load_2d(st + b_bytes, &tmX1, bar, kx, (int)m_base);
-                if (a.parts > 2) tma_load_2d(st + 2 * b_bytes, &tmX2, bar, kx, (int)m_base);
+                tma_load_2d(st, &tmX0, &full[slot], kx, (int)m_base);
+                if (a.parts > 1) tma_load_2d(st + b_bytes, &tmX1, &full[slot], kx, (int)m_base);
+                if (a.parts > 2) tma_load_2d(st + 2 * b_bytes, &tmX2, &full[slot], kx, (int)m_base);
             };
             const uint32_t pre = min(a.kblocks, a.stages);
-            for (uint32_t i = 0; i < pre; ++i) load_w(i);
+            for (uint32_t i = 0; i < pre; ++i) load_w(i, i);
             pdl_wait();
-            for (uint32_t i = 0; i < pre; ++i) load_x(i);
-            uint32_t issued = pre;
+            for (uint32_t i = 0; i < pre; ++i) load_x(i, i);
+            uint32_t issued = pre, slot = 0, phase = 0;  // carried: a division or remainder takes as long as a block's products
             for (; issued < a.kblocks; ++issued) {
-                if (!mbar_wait(&empty[issued % a.stages], (issued / a.stages - 1u) & 1u)) { *abort_flag = 1; break; }
+                if (!mbar_wait(&empty[slot], phase)) { *abort_flag = 1; break; }
                 if (*abort_flag) break;
-                load_w(issued);
-                load_x(issued);
+                load_w(issued, slot);
+                load_x(issued, slot);
+                if (++slot == a.stages) slot = 0, phase ^= 1u;
             }
             if (*abort_flag)  // copies still in flight land (bounded wait) before the CTA goes away
                 for (uint32_t i = issued > a.stages ? issued - a.stages : 0u; i < issued; ++i)
@@ -298,16 +297,19 @@ int m40_gemm_tc_grouped(M40llmCudaContext* ctx, cudaStream_t s, const M40Grouped
     a.head_pitch = c.head_pitch;
     a.rg = c.rg;
     const uint32_t stage = tc::BLOCK_N * tc::BLOCK_K * 2 + c.parts * c.tile_rows * tc::BLOCK_K * 2;
-    // a short ring and three CTAs per SM where the tile allows it: their prologues and epilogues cover one another
-    uint32_t stages = 66u * 1024u / stage;
+    const uint32_t n_tile = paired ? tc::BLOCK_N / 2 : tc::BLOCK_N;
+    const dim3 grid((c.N + n_tile - 1) / n_tile, c.tiles ? c.max_tiles : (c.x_rows + c.tile_rows - 1) / c.tile_rows, c.tiles ? 1 : c.groups);
+    // A short ring and three CTAs per SM where the tile allows it: their prologues and epilogues cover one another. Where every CTA has an
+    // SM to itself, a ring that holds most of its weights before the activations are there: 16 CTAs, 32 rows, K = 512 10.2 us, with two
+    // stages 12.4.
+    const bool alone = (uint64_t)grid.x * grid.y * grid.z <= (uint64_t)ctx->sm_count;
+    uint32_t stages = (alone ? 192u : 66u) * 1024u / stage;
     if (stages < 2) stages = 2;
     if (stages > a.kblocks) stages = a.kblocks;
     // the paired epilogue passes tile_rows * 64 f32 through the ring
     const uint32_t least = paired ? (c.tile_rows * 64u * 4u + stage - 1) / stage : 1u;
     a.stages = stages < least ? least : stages;
     const size_t smem = (size_t)a.stages * stage + (2 * a.stages + 1) * 8 + 16 + 1024;
-    const uint32_t n_tile = paired ? tc::BLOCK_N / 2 : tc::BLOCK_N;
-    const dim3 grid((c.N + n_tile - 1) / n_tile, c.tiles ? c.max_tiles : (c.x_rows + c.tile_rows - 1) / c.tile_rows, c.tiles ? 1 : c.groups);
     switch (c.kind) {
         case M40_GROUPED_F32: return launch<M40_GROUPED_F32>(ctx, s, grid, smem, m, a);
         case M40_GROUPED_ACT_SPLIT: return launch<M40_GROUPED_ACT_SPLIT>(ctx, s, grid, smem, m, a);

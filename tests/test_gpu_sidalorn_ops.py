@@ -366,10 +366,11 @@ def test_rglru(nat, W, B, taps, exact):
     nat.free_all()
 
 
-@pytest.mark.parametrize("n", [8, 9, 16, 17, 33])
-def test_rglru_steps_of_many_sequences(nat, n):
-    """A step's tiles hold 16 rows, eight to a thread: full and ragged ones, the first token of a sequence among later ones."""
-    W, B, taps, T = 576, 4, 4, 4
+@pytest.mark.parametrize("n,W,B", [(8, 576, 4), (9, 576, 4), (16, 576, 4), (17, 576, 4), (33, 576, 4), (17, 1024, 1), (5, 968, 1)])
+def test_rglru_steps_of_many_sequences(nat, n, W, B):
+    """A step's tiles hold 16 rows, eight to a thread: full and ragged ones, the first token of a sequence among later ones; products with
+    fewer blocks of K than the ring of a block that has its SM to itself, and with more."""
+    taps, T = 4, 4
     rng = np.random.default_rng(n)
     D = W // B
     w = {"conv": 0.5 * rng.standard_normal((W, taps)), "conv.b": 0.3 * rng.standard_normal(W), "ra.b": rng.standard_normal((B, D)),
