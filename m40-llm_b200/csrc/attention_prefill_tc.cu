@@ -14,8 +14,9 @@
 //
 // Warps 0..3 are the query rows, warp 4 loads K and V by TMA (two stages each), warp 5 issues the MMAs: S(j + 1) runs while the
 // rows work on S(j). A 128 x 128 tile of HD 128 is 24 MMAs (1600 cycles at the tensor rate) beside 1024 cycles of exponentials per
-// scheduler; one set of rows per SM leaves part of either idle. Four packed prompts of 509 to 2048 tokens, 32 / 8 heads of 128:
-// 279 us, against 438 us with mma.sync fragments (attention_prefill.cu), which stay for short segments.
+// scheduler; one set of rows per SM leaves part of either idle, so that two row tiles share a CTA where there are more tiles than SMs
+// (TILES). Four packed prompts of 509 to 2048 tokens, 32 / 8 heads of 128: 245 us, with one tile 280, against 438 us with mma.sync
+// fragments (attention_prefill.cu), which stay for short segments; 220 since the call no longer copies its lengths back.
 // Rows behind a sequence's last key are whatever the cache holds there; the issuing warp clears them in the value tile, since
 // zero weights do not cancel a NaN. Values of tokens that only some rows see are dealt with at the end (attend_row()): looking
 // through the one or two tiles in question beforehand, in shared memory or with a warp of its own, cost 8 to 22 us of 273, this 5.
