@@ -3,8 +3,8 @@
 // Q8_0 stores 32 weights as {f16 d; int8 q[32]} (34 bytes, cuda/kernels.cu:856-867 of the reference):
 // w = d * q with a different d for every (row, 32-k block).
 //
-//   raw bytes   TMA (plain 2D box of 128 rows x 272 bytes = 8 blocks per row) straight from the GGUF layout, four
-//               stages deep;
+//   raw bytes   TMA (plain 2D box of 128 rows x 272 bytes = 8 blocks per row) straight from the GGUF layout, two
+//               to four stages deep;
 // More than 32 rows (gemm_tc_q80_kernel; up to 32: gemm_tc_q80_exact_kernel, below):
 //   dequant     16 worker warps. Worker group g (4 warps = 128 threads = 128 weight rows) owns the g-th 64-k
 //               sub-block of every raw stage; a thread turns the two blocks of its row into TWO f16 operands,
@@ -20,8 +20,8 @@
 //               committed once per thread to ONE completion barrier that frees both the operand stage and the
 //               activation slot;
 //   epilogue    the worker threads read their row of D back (tcgen05.ld) at the end of a segment.
-// A pass takes up to 128 rows: it reads and converts the weights once. Feed-forward of 4096 x 14336: 128 rows 130 us, in two passes of 64
-// 179; 65 to 72 rows 107 against 132 to 167; 64 rows 86.
+// A pass takes up to 128 rows: it reads and converts the weights once. Feed-forward of 4096 x 14336: 128 rows 130 to 135 us, in two passes of
+// 64 179; 65 to 72 rows 107 to 112 against 132 to 167; 64 rows 86.
 //
 // Work is split stream-K style: the (tile, 256-k unit) space is cut into one contiguous span per CTA (one CTA per
 // SM), so every SM streams the same number of weight bytes. A span that crosses tile boundaries writes one partial
@@ -388,15 +388,15 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) gemm_tc_q80_kernel(const __gri
 // ---------------------------------------------------------------------------------------------------------------------------------
 // 2 to 32 rows: the signed bytes themselves are the operand. They are exact in f16, so a weight passes the tensor core as one operand, not
 // as hi and lo of d * q; a 32-block's product with Xh and Xl gets accumulator columns of its own, which the worker threads fetch, multiply
-// by the block's scale and add up in f32 registers. Sums of 16 f32 products at a time on the tensor core instead of a whole row: the error
-// against 64 bits falls from 3e-6 to 1.6e-7 of the result's norm (4096 x 14336).
+// by the block's scale and add up in f32 registers. The tensor core sums 32 weights at a time instead of a whole row: the error against 64
+// bits falls from 3e-6 to 1.6e-7 of the result's norm (4096 x 14336).
 //
 // The four groups of worker warps own the 64-k sub-blocks (two blocks) of a unit like above. A group converts its sub-block into one of its
 // two operand stages and then collects the products of the unit before, which were made meanwhile. At a segment's end the groups' sums meet
 // in their product buffers, in a fixed order. What bounds it is the path from barrier to barrier around a unit, not its bytes (2000 cycles a
 // unit; its bytes take 1500): two warps issue, and the loading threads count instead of taking remainders (a remainder a sub-block made
-// the activations late: 74 us). Feed-forward of 4096 x 14336: 2 to 16 rows 51 to 54 us, 17 to 32 61 to 63, against 72 to 75 and 75 to 78
-// with hi and lo operands (2048 x 5632: 24 to 26 and 29, against 29 to 30 and 31); the same on mma.sync took 53 to 56 for 2 to 8 rows and 71
+// the activations late: 74 us). Feed-forward of 4096 x 14336: 2 to 16 rows 52 to 55 us, 17 to 32 62 to 65, against 72 to 75 and 75 to 78
+// with hi and lo operands (2048 x 5632: 25 to 27 and 30, against 29 to 30 and 31); the same on mma.sync took 53 to 56 for 2 to 8 rows and 71
 // to 109 for 16 to 32. From 33 rows on the sums do not fit the threads' registers.
 __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
@@ -443,8 +443,8 @@ struct ExactCfg {
     static constexpr uint32_t STAGES = 8;                          // operand stages of 32 columns: two per group
     static constexpr uint32_t A_COL0 = BUFS * 2 * M_PAD;
     static constexpr uint32_t TILE = 2 * M_PAD * BLOCK_K * 2 * 4;  // activations of a unit: hi, then lo, [4][M_PAD][64] each
-    static constexpr uint32_t SLOTS = M_PAD == 32 ? 2 : 4;         // such units in flight
-    static constexpr uint32_t RAWS = 4;
+    static constexpr uint32_t SLOTS = M_PAD == 32 ? 3 : 4;         // such units in flight
+    static constexpr uint32_t RAWS = M_PAD == 32 ? 3 : 4;          // 3 and 3 units: 63.5, 4 of weights and 2 of activations: 64.5 us at 25 rows
     static_assert(A_COL0 + STAGES * 32 <= TMEM_COLS, "tensor memory");
     static constexpr size_t SMEM = RAWS * RAW_BYTES + SLOTS * TILE + (2 * RAWS + 2 * STAGES + 2 * SLOTS + BUFS) * 8 + 16 + 1024;
 };
