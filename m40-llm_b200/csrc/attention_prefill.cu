@@ -17,6 +17,8 @@
 //
 // The same kernel also reads K and V straight from a dense f16 cache (CACHE): a prompt portion whose rows are already
 // appended attends everything its sequence holds, and the output may be turned back and gated before it is stored.
+#include <cuda.h>
+
 #include "attention.cuh"
 #include "attention_mma.cuh"
 #include "attention_prefill_tc.cuh"
@@ -317,9 +319,38 @@ __global__ void __launch_bounds__(256) collect_lengths_kernel(const uint32_t* q_
     }
 }
 
+using PointerAttributesFn = CUresult (*)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
+PointerAttributesFn get_pointer_attributes() {
+    static const PointerAttributesFn fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const bool ok = cudaGetDriverEntryPoint("cuPointerGetAttributes", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
+        if (!ok) cudaGetLastError();
+        return ok ? (PointerAttributesFn)p : nullptr;
+    }();
+    return fn;
+}
+
+// Whether n values at p lie in one allocation of the context's device. A copy from anywhere else may fail and says so; a kernel that reads
+// there takes the context with it.
+bool in_device_memory(const M40llmCudaContext* ctx, const uint32_t* p, uint32_t n) {
+    const PointerAttributesFn attributes = get_pointer_attributes();
+    if (!attributes || ((uintptr_t)p & 3u) != 0u) return false;
+    unsigned int type = 0, managed = 0;
+    int device = -1;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    CUpointer_attribute which[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                   CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* values[] = {&type, &managed, &device, &start, &size};
+    if (attributes(5, which, values, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS) return false;
+    const uint64_t at = (uint64_t)(uintptr_t)p - start, bytes = (uint64_t)n * sizeof(uint32_t);
+    return type == CU_MEMORYTYPE_DEVICE && !managed && device == ctx->device_id && start != 0 && at <= size && bytes <= size - at;
+}
+
 // The lengths of a packed call on the host. One kernel writes them to the context's mapped memory: three copies to pageable memory each
-// wait for the one before, 50 us of a 290 us call. Where another thread has that memory, or a call has more sequences than fit, they are
-// copied all the same.
+// wait for the one before, 50 us of a 290 us call. Where another thread has that memory, a call has more sequences than fit, or an array
+// is not in this device's memory, they are copied all the same.
 class Lengths {
 public:
     Lengths(M40llmCudaContext* ctx, uint32_t n) : ctx_(ctx), n_(n) {
@@ -331,6 +362,7 @@ public:
     // Waits for the stream. Null: a call failed.
     const uint32_t* read(cudaStream_t s, const uint32_t* q_lens, const uint32_t* kv_lens, const uint32_t* kv_offsets) {
         bool ok;
+        if (mapped_ && !(in_device_memory(ctx_, q_lens, n_) && in_device_memory(ctx_, kv_lens, n_) && in_device_memory(ctx_, kv_offsets, n_))) release();
         if (mapped_) {
             collect_lengths_kernel<<<1, 256, 0, s>>>(q_lens, kv_lens, kv_offsets, n_, ctx_->d_readback);
             M40_COUNT_LAUNCH(ctx_);

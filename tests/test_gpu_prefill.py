@@ -89,6 +89,25 @@ def test_prefill_argument_errors(nat):
     nat.free_all()
 
 
+def test_prefill_lengths_outside_device_memory_are_refused(nat, O):
+    """An array of lengths that no kernel may read is copied, as far as that goes, and never read by a kernel: the call answers with an
+    error and the context goes on. The lengths are invalid, so that a machine that can copy them refuses them too."""
+    x = nat.buf(np.zeros(4 * 64 * 8, np.float32))
+    one, zero = nat.buf(np.array([1], np.uint32)), nat.buf(np.array([0], np.uint32))
+    host = np.zeros(4096, np.uint32)
+    for at in range(3):
+        for ptr in (host.ctypes.data, zero.ptr + 2):   # host memory; half a value
+            lens = [zero.ptr, zero.ptr, zero.ptr]      # q_lens, kv_lens, kv_offsets: no length is valid
+            lens[at] = ptr
+            rc = nat.lib.m40llm_attention_prefill_f32_gqa_varlen_async(nat.ctx, x.ptr, x.ptr, x.ptr, zero.ptr, lens[2], lens[0], lens[1], 1, 4, 2,
+                                                                       64, x.ptr)
+            assert rc in (-7, -8), rc
+            nat.sync(0)
+    got, exp = run_prefill(nat, O, 4, 2, 64, [(3, 3), (2, 5)], 1)
+    assert_close(got, exp)
+    nat.free_all()
+
+
 @pytest.mark.parametrize("kvh,hd,R,bs,L", [(2, 64, 8, 4, 21), (2, 128, 16, 8, 100), (8, 128, 512, 64, 1500), (2, 64, 32, 16, 20)])
 def test_build_compressed_from_dense(nat, O, kvh, hd, R, bs, L):
     """Every slot of the compressed cache ends up as token-by-token appends would have left it: bit-exact old K, q4 V
