@@ -106,6 +106,20 @@ def test_linear_few_rows(nat, rows, n, k, wdt):
         close(run_linear(nat, x, w[:n // 2], wdt, rows, w2=w[n // 2:]), y[:, :n // 2] * S.sigmoid(y[:, :n // 2]) * y2, 4 * tol, "gated")
 
 
+@pytest.mark.parametrize("rows", [2, 16, 17, 32])
+@pytest.mark.parametrize("n,k,limit", [(256, 8192, 8e-7), (1024, 4096, 4.4e-7), (6144, 4096, 9.2e-7), (128, 64, 2e-7), (128, 136, 2e-7)])
+def test_linear_few_rows_sums_stay_short(nat, rows, n, k, limit):
+    """The tensor core truncates its sums, so the error grows with how much of K one of them holds. Operands are exact here: f16 weights,
+    activations that are f16. The limits are a third above 16, 16 and 6 sums' errors (6.3e-7, 3.4e-7 and, with 8, 6.2e-7) and below those of
+    sums twice as long (1.2e-6, 6.3e-7, 9.7e-7); the last two have one block of K and two and a part."""
+    rng = np.random.default_rng(rows + k)
+    x, w = rng.standard_normal((rows, k)).astype(np.float16).astype(np.float32), rounded(rng, N.DT_F16, n, k)
+    want = x.astype(np.float64) @ w.T.astype(np.float64)
+    got = run_linear(nat, x, w, N.DT_F16, rows)
+    err = np.linalg.norm(got - want) / np.linalg.norm(want)
+    assert err <= limit, err
+
+
 def test_linear_few_rows_chain_and_in_place(nat):
     """Projections that feed one another, replayed as a graph so that each starts beside the one before; the last one's result lies over
     its own input."""
