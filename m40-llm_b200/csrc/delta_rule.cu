@@ -3,12 +3,14 @@
 // with a decay w and a removal rate a per head and key channel, u the unit key. All of it is f32.
 //
 // With k = n u (n the key's length) the update of one value column s of S is
-//   d = u . s,   s_i <- w_i s_i + u_i n v - (a u)_i d,   o = r . s,
+//   d = u . s,   s_i <- w_i s_i + u_i (n v - a_i d),   o = r . s,
 // so columns are independent. A column's key dimension is shared by a few lanes (16-byte pieces dealt round-robin) and stays in
-// registers; the only serial chain is d: a dot product over the lanes, then one multiply-add per element.
+// registers; the only serial chain is d: a dot product over the lanes, then two multiply-adds per element. (With one, on
+// w_i s_i + u_i n v from before, a state whose keys come back loses twice as much: n v - a d must cancel before it is rounded to the
+// size of either.)
 //
 //   portions of several tokens, in passes of rows whose records stay in L2:
-//     delta_prepare_kernel  warp = (row, head): gates, decays, unit key -> one record [w | u | a u | r | n v | c] per (head, row);
+//     delta_prepare_kernel  warp = (row, head): gates, decays, unit key -> one record [w | u | a | r | n v | c] per (head, row);
 //     delta_scan_kernel     CTA = (16 or 64 columns, head, segment) walks the tokens in pairs; the records of 16 tokens arrive by
 //                           one bulk copy (cp.async.bulk + mbarrier) several chunks ahead. Reads of the records from shared memory
 //                           are the limit, so a lane holds few keys of several columns and every piece serves all of them;
@@ -39,7 +41,7 @@ constexpr size_t PASS_BYTES = (size_t)96 << 20;  // records of one pass: inside 
 constexpr int SCAN_CHUNK = 16;    // tokens per bulk copy (even: pairs do not cross chunks)
 constexpr uint32_t SCAN_MAX_STAGES = 8;
 constexpr int SCAN_SMEM = 196608;
-// A record: w | u | a u | r | n v, DP floats each, then c1, c2 and two floats of padding.
+// A record: w | u | a | r | n v, DP floats each, then c1, c2 and two floats of padding.
 __host__ __device__ constexpr uint32_t rec_floats(int dp) { return 5u * dp + 4u; }
 __host__ __device__ constexpr size_t scan_stage_bytes(int dp) { return (size_t)SCAN_CHUNK * rec_floats(dp) * sizeof(float); }
 
@@ -191,7 +193,7 @@ __global__ void __launch_bounds__(256) delta_prepare_kernel(DeltaArgs a, float* 
         const float u = k[i] * inv, u0 = k0[i] * inv0;
         dst[ch] = in ? decay_of(a, z[i]) : 0.0f;
         dst[DP + ch] = in ? u : 0.0f;
-        dst[2 * DP + ch] = in ? u * m40_sigmoid(rate[i]) : 0.0f;
+        dst[2 * DP + ch] = in ? m40_sigmoid(rate[i]) : 0.0f;
         dst[3 * DP + ch] = in ? r[i] : 0.0f;
         dst[4 * DP + ch] = in ? len * v[i] : 0.0f;
         c1 = in ? fmaf(u, u0, c1) : c1;
@@ -361,12 +363,12 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a, c
                 d[c] = f2_sum(x), e[c] = f2_sum(y);
             }
             // the rest of this pair's records and the start of the next pair's are on their way during the shuffles
-            F2 ua[2 * NI], r[2 * NI], u1[2 * NI], w1[2 * NI], ub[2 * NI], r1[2 * NI];
-            load_pieces<NI, LANES>(va + 2 * DP, l, ua);
+            F2 a0[2 * NI], r[2 * NI], u1[2 * NI], w1[2 * NI], a1[2 * NI], r1[2 * NI];
+            load_pieces<NI, LANES>(va + 2 * DP, l, a0);
             load_pieces<NI, LANES>(va + 3 * DP, l, r);
             load_pieces<NI, LANES>(vb, l, w1);
             load_pieces<NI, LANES>(vb + DP, l, u1);
-            load_pieces<NI, LANES>(vb + 2 * DP, l, ub);
+            load_pieces<NI, LANES>(vb + 2 * DP, l, a1);
             load_pieces<NI, LANES>(vb + 3 * DP, l, r1);
             const float2 cc = *reinterpret_cast<const float2*>(vb + 5 * DP);
             float nv0[COLS], nv1[COLS];
@@ -384,7 +386,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a, c
                 F2 x = zero;
 #pragma unroll
                 for (int i = 0; i < 2 * NI; ++i) {
-                    s[c][i] = f2_fma(ua[i], d0, f2_fma(w0[i], s[c][i], f2_mul(u0[i], n0)));
+                    s[c][i] = f2_fma(u0[i], f2_fma(a0[i], d0, n0), f2_mul(w0[i], s[c][i]));
                     x = f2_fma(r[i], s[c][i], x);
                 }
                 o[2 * c] = f2_sum(x);
@@ -397,7 +399,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a, c
                 F2 x = zero;
 #pragma unroll
                 for (int i = 0; i < 2 * NI; ++i) {
-                    s[c][i] = f2_fma(ub[i], dd, f2_fma(w1[i], s[c][i], f2_mul(u1[i], n1)));
+                    s[c][i] = f2_fma(u1[i], f2_fma(a1[i], dd, n1), f2_mul(w1[i], s[c][i]));
                     x = f2_fma(r1[i], s[c][i], x);
                 }
                 o[2 * c + 1] = f2_sum(x);

@@ -534,6 +534,28 @@ def test_delta_rule_long_memory(nat):
     d.close()
 
 
+@pytest.mark.parametrize("spread,limit", [(0.0, 6.5e-7), (1e-3, 8.1e-7)])
+@pytest.mark.parametrize("H,D,segments", [(8, 64, 1), (60, 64, 1), (8, 64, 3), (6, 48, 1), (4, 128, 1), (2, 256, 1)])
+def test_delta_rule_keys_that_come_back(nat, H, D, segments, spread, limit):
+    """Consecutive keys nearly equal, removal rates near 1 and hardly any decay: every token takes out what the one before wrote, and n v - a d
+    is a small difference. A token at a time in f32 leaves 5.2e-7 of the state's norm with equal keys and 7.5e-7 with nearly equal ones; an
+    update that rounds w s + u n v first leaves 7.7 to 8.4e-7 and 8.7 to 9.7e-7. The limits lie between."""
+    d = Delta(nat, H, D, 4, seed=D)
+    d.w0[:], d.ab[:], d.w2[:] = -14.0, 14.0, 0.0
+    rng = np.random.default_rng(H)
+    T, HD = 201, H * D
+    packed = rng.standard_normal((segments * T, d.width())).astype(np.float32)
+    packed[:, HD:2 * HD] = np.tile(rng.standard_normal((1, HD)), (segments * T, 1)) + spread * packed[:, HD:2 * HD]
+    packed[:, 4 * HD:5 * HD] = 0.0
+    segs = [(s, 0, T) for s in range(segments)]
+    d.device(packed, segs)
+    d.oracle(packed, segs)
+    for s in range(segments):
+        err = np.linalg.norm(d.state(s) - d.S[s]) / np.linalg.norm(d.S[s])
+        assert err <= limit, err
+    d.close()
+
+
 @pytest.mark.parametrize("wdt", [N.DT_F16, N.DT_F32])
 def test_delta_rule_other_weight_types(nat, wdt):
     d = Delta(nat, 2, 32, 10, seed=2, wdt=wdt)
