@@ -11,7 +11,7 @@
 //
 //   portions of several tokens, in passes of rows whose records stay in L2:
 //     delta_prepare_kernel  warp = (row, head): gates, decays, unit key -> one record [w | u | a | r | n v | c] per (head, row);
-//     delta_scan_kernel     CTA = (16 or 64 columns, head, segment) walks the tokens in pairs; the records of 16 tokens arrive by
+//     delta_scan_kernel     CTA = (16 to 64 columns, head, segment) walks the tokens in pairs; the records of 16 tokens arrive by
 //                           one bulk copy (cp.async.bulk + mbarrier) several chunks ahead. Reads of the records from shared memory
 //                           are the limit, so a lane holds few keys of several columns and every piece serves all of them;
 //     delta_finish_kernel   the per-head norm and the output gate.
@@ -29,6 +29,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "delta_scan_plan.cuh"
 #include "stack_math.cuh"
 #include "state_cache.cuh"
 #include "tc_ptx.cuh"
@@ -36,7 +37,7 @@
 namespace {
 
 constexpr int LANES = 4;          // decode: lanes per column
-constexpr int SCAN_THREADS = 128;
+constexpr int SCAN_THREADS = M40_SCAN_THREADS;
 constexpr size_t PASS_BYTES = (size_t)96 << 20;  // records of one pass: inside L2
 constexpr int SCAN_CHUNK = 16;    // tokens per bulk copy (even: pairs do not cross chunks)
 constexpr uint32_t SCAN_MAX_STAGES = 8;
@@ -277,8 +278,9 @@ __device__ __forceinline__ void load_values(const float* p, float (&v)[COLS]) {
 }
 
 // grid (column blocks, heads, segments). Rows [base, base + count) of the segment, counted from its start. LANES lanes hold COLS
-// columns of LANES * NI * 4 keys. 2048 tokens of one sequence, 32 heads of 64: 241 us (324 a token at a time, 32 columns per CTA), of
-// which a pair's chain of shuffles and multiply-adds takes most; 1500 tokens of 16 sequences, 64 heads: 137 us (238).
+// columns of LANES * NI * 4 keys; which of them a call takes: delta_scan_plan.cuh. A pair's chain of shuffles and multiply-adds takes most
+// of the time. The whole call for 2048 tokens of one sequence, 32 heads of 64: 301 us (368 a token at a time, 32 columns per CTA); 1504
+// tokens of 16 sequences, 64 heads: 187 us (300).
 template <int NI, int LANES, int COLS>
 __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a, const float* __restrict__ rec, uint32_t n_rec,
                                                                   uint32_t rec_base, uint32_t base, uint32_t count, uint32_t stages) {
@@ -297,8 +299,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) delta_scan_kernel(DeltaArgs a, c
     pdl_wait();
     pdl_trigger();
     const uint32_t head = blockIdx.y, col0 = blockIdx.x * (SCAN_THREADS / LANES * COLS), D = a.dim, HD = a.heads * D;
-    const uint32_t seg0 = a.seg[4 * blockIdx.z], seg_n = a.seg[4 * blockIdx.z + 1];
-    const uint32_t slot = a.seg[4 * blockIdx.z + 2] * a.slot_mul + a.slot_add, pos0 = a.seg[4 * blockIdx.z + 3];
+    // last segments first: a step has its single tokens before its prompts, whose chains take longest
+    const uint32_t z = gridDim.z - 1u - blockIdx.z;
+    const uint32_t seg0 = a.seg[4 * z], seg_n = a.seg[4 * z + 1];
+    const uint32_t slot = a.seg[4 * z + 2] * a.slot_mul + a.slot_add, pos0 = a.seg[4 * z + 3];
     if (slot >= a.slots || (uint64_t)seg0 + seg_n > a.rows) {
         if (tid == 0 && blockIdx.x == 0 && head == 0) atomicOr(a.status, 2u);
         return;
@@ -585,7 +589,17 @@ int launch_scan(M40llmCudaContext* ctx, const DeltaArgs& a, const float* rec, ui
     return e == cudaSuccess ? 0 : -6;
 }
 
-// P: 32-key pieces of a column.
+// P: 32-key pieces of a column. The forms that delta_scan_plan.cuh chooses from.
+template <int P>
+int launch_planned(M40llmCudaContext* ctx, const DeltaArgs& a, const float* rec, uint32_t n_rec, uint32_t base, uint32_t pass, uint32_t segments,
+                   uint32_t stages, const M40ScanPlan& plan) {
+    if constexpr (P % 2 == 0)
+        if (plan.lanes == 16) return launch_scan<P / 2, 16, 2>(ctx, a, rec, n_rec, base, pass, segments, stages);
+    if constexpr (P <= 4)
+        if (plan.cols == 4) return launch_scan<P, 8, 4>(ctx, a, rec, n_rec, base, pass, segments, stages);
+    return launch_scan<P, 8, 2>(ctx, a, rec, n_rec, base, pass, segments, stages);
+}
+
 template <int P>
 int run_scan(M40llmCudaContext* ctx, const DeltaArgs& a, uint32_t segments, uint32_t max_segment_rows) {
     constexpr int DP = P * 32;
@@ -602,13 +616,8 @@ int run_scan(M40llmCudaContext* ctx, const DeltaArgs& a, uint32_t segments, uint
     const uint32_t n_rec = segments == 1 ? pass : a.rows;
     float* rec = (float*)m40_ensure_scratch(ctx, 1, n_rec * per_row, 1);
     if (!rec) return -5;
-    // Narrow CTAs, sixteen lanes and two columns per group, where two per SM take all of them; otherwise eight lanes and four columns,
-    // and a ring that lets three CTAs share an SM.
-    constexpr int LANES = P % 2 == 0 ? 16 : 8;
-    constexpr uint32_t NARROW = SCAN_THREADS / LANES * 2;
-    const uint64_t ctas = (uint64_t)((a.dim + NARROW - 1) / NARROW) * a.heads * segments;
-    const bool narrow = ctas <= 2u * (uint64_t)ctx->sm_count;
-    const uint32_t fit = (uint32_t)((!narrow ? SCAN_SMEM / 3 : (ctas <= (uint64_t)ctx->sm_count ? SCAN_SMEM : SCAN_SMEM / 2)) / scan_stage_bytes(DP));
+    const M40ScanPlan plan = m40_scan_plan(a.dim, a.heads, segments, segments == 1 ? max_segment_rows : a.rows, max_segment_rows, (uint32_t)ctx->sm_count);
+    const uint32_t fit = (uint32_t)(SCAN_SMEM / plan.per_sm / scan_stage_bytes(DP));
     const uint32_t stages = fit < 2u ? 2u : (fit > SCAN_MAX_STAGES ? SCAN_MAX_STAGES : fit);
     cudaError_t e;
     for (uint32_t base = 0; base < max_segment_rows; base += pass) {
@@ -617,8 +626,7 @@ int run_scan(M40llmCudaContext* ctx, const DeltaArgs& a, uint32_t segments, uint
         e = m40_launch_dependent(delta_prepare_kernel<DP>, dim3((rows * a.heads + 7) / 8), dim3(256), 0, s, a, rec, n_rec, base, rows);
         M40_COUNT_LAUNCH(ctx);
         if (e != cudaSuccess) return -6;
-        const int rc = narrow ? launch_scan<DP / (4 * LANES), LANES, 2>(ctx, a, rec, n_rec, base, pass, segments, stages)
-                              : launch_scan<P, 8, P <= 4 ? 4 : 2>(ctx, a, rec, n_rec, base, pass, segments, stages);
+        const int rc = launch_planned<P>(ctx, a, rec, n_rec, base, pass, segments, stages, plan);
         if (rc != 0) return rc;
     }
     e = m40_launch_dependent(delta_finish_kernel, dim3((a.rows * a.heads + 7) / 8), dim3(256), 0, s, a);

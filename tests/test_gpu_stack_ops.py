@@ -486,14 +486,14 @@ def test_delta_rule_portions_and_decode(nat, H, D, R):
     d.close()
 
 
-@pytest.mark.parametrize("H,D", [(80, 64), (300, 16), (40, 128), (110, 48), (20, 200), (40, 64), (75, 64)])
+@pytest.mark.parametrize("H,D", [(80, 64), (300, 16), (40, 128), (110, 48), (20, 200), (40, 64), (75, 64), (29, 160), (31, 160), (12, 96), (10, 256), (18, 256)])
 def test_delta_rule_forms_of_the_scan(nat, H, D):
-    """Heads enough for the form that fills the machine, around the border to the narrow one (two CTAs per SM of 148), whole and odd
-    numbers of pairs of tokens."""
+    """Heads and segments enough for every form of the scan, with one to three CTAs per SM of 148, whole and odd numbers of pairs of
+    tokens; prompts long enough for the form of 16 lanes."""
     d = Delta(nat, H, D, 4, seed=H)
     rng = np.random.default_rng(H + D)
     p0 = {0: 0, 2: 0}
-    for step in ([(0, 33)], [(2, 2), (0, 16)], [(0, 1)], [(0, 31), (2, 5)]):
+    for step in ([(0, 33)], [(2, 2), (0, 16)], [(0, 1)], [(0, 31), (2, 5)], [(0, 67)]):
         segs = [(s, p0[s], n) for s, n in step]
         for s, n in step:
             p0[s] += n

@@ -93,3 +93,50 @@ def test_gate_up_calls_are_cut_as_measured(ask):
         for m, n, k, _, _ in GATE_UP])
     for case, shared in zip(GATE_UP, got):
         assert (case[3] if shared else case[4]) == min(case[3:]), case
+
+
+# head size, heads, segments, tokens of each; us of the call a token at a time in CTAs of 32 columns, then of the scan in pairs with 16 lanes
+# and 2 columns, 8 and 2, 8 and 4, each with one, two and three CTAs per SM at most
+SCANS = [
+    (64, 32, 1, 2048, 368.3, [[301.1, 382.6, 493.1], [330.1, 493.3, 692.4], [475.5, 758.7, 980.5]]),
+    (64, 16, 3, 200, 42.0, [[61.2, 44.5, 55.4], [39.2, 55.1, 74.7], [53.4, 81.0, 84.4]]),
+    (64, 16, 6, 100, 43.4, [[50.9, 45.6, 34.4], [40.8, 34.0, 44.0], [33.0, 46.9, 62.6]]),
+    (64, 32, 2, 300, 63.4, [[92.0, 67.5, 83.9], [59.6, 83.5, 112.7], [81.1, 122.0, 168.9]]),
+    (64, 32, 4, 300, 126.9, [[182.4, 132.3, 134.3], [117.8, 99.7, 128.9], [97.2, 138.3, 185.2]]),
+    (64, 64, 1, 256, 54.2, [[78.7, 57.7, 71.8], [51.1, 71.5, 96.6], [69.2, 104.6, 113.0]]),
+    (64, 64, 16, 94, 300.1, [[432.9, 306.3, 275.1], [281.9, 227.6, 218.6], [229.7, 193.1, 187.1]]),
+    (64, 75, 1, 300, 113.1, [[131.3, 105.6, 86.4], [103.6, 86.2, 115.5], [83.7, 125.0, 171.7]]),
+    (64, 48, 12, 50, 96.2, [[143.3, 101.3, 91.5], [92.5, 74.4, 71.5], [74.1, 63.2, 61.6]]),
+    (64, 32, 1, 33, 11.6, [[12.1, 12.6, 14.5], [11.4, 14.3, 17.8], [13.7, 18.5, 18.4]]),
+    (32, 32, 12, 50, 32.0, [None, [31.5, 31.5, 25.7], [33.5, 33.5, 30.5]]),
+    (32, 64, 32, 33, 86.7, [None, [86.9, 86.9, 81.3], [98.4, 98.4, 90.2]]),
+    (96, 24, 3, 200, 101.9, [None, [90.0, 79.6, 108.1], [72.3, 108.4, 146.1]]),
+    (96, 24, 24, 33, 123.8, [None, [116.5, 94.0, 90.7], [110.9, 89.8, 85.7]]),
+    (128, 16, 1, 300, 105.6, [[55.1, 80.8], [76.0, 125.4], [114.2, 188.4]]),
+    (128, 36, 1, 300, 110.4, [[104.8, 87.4], [82.8, 132.7], [121.8, 181.5]]),
+    (128, 64, 1, 300, 216.6, [[207.6, 171.5], [164.4, 150.2], [139.2, 213.3]]),
+    (128, 16, 16, 100, 267.3, [[263.9, 207.7], [206.4, 179.9], [189.8, 162.8]]),
+    (160, 8, 1, 300, 146.1, [[64.7], [112.8], None]),
+    (160, 30, 1, 300, 290.5, [[184.5], [225.5], None]),
+    (192, 16, 2, 300, 297.4, [[194.6], [235.2], None]),
+    (192, 16, 24, 33, 303.0, [[288.0], [258.5], None]),
+    (256, 9, 1, 300, 301.7, [[81.9], [146.1], None]),
+    (256, 19, 1, 300, 589.4, [[221.1], [287.0], None]),
+    (256, 16, 24, 33, 759.9, [[442.3], [418.5], None]),
+]
+
+
+def test_delta_scans_take_the_form_that_was_fastest(ask):
+    got = ask("delta_scan_plan.cuh", [f'{{ const M40ScanPlan p = m40_scan_plan({d}, {h}, {s}, {s * n}, {n}, 148); printf("%u %u %u\\n", p.lanes, p.cols, p.per_sm); }}'
+                                      for d, h, s, n, _, _ in SCANS])
+    for case, (lanes, cols, per) in zip(SCANS, zip(*[iter(got)] * 3)):
+        times = case[5][{(16, 2): 0, (8, 2): 1, (8, 4): 2}[lanes, cols]]
+        assert times[int(per) - 1] <= 1.06 * min(t for f in case[5] if f for t in f), case
+        assert times[int(per) - 1] <= case[4], case
+
+
+def test_single_tokens_beside_a_prompt_do_not_choose_its_scan(ask):
+    """A step of 31 decoding sequences and one prompt: the prompt's chain is what takes long."""
+    alone, beside = ask("delta_scan_plan.cuh", [f'{{ const M40ScanPlan p = m40_scan_plan(64, 32, {s}, {r}, 300, 148); printf("%u\\n", p.lanes * 100 + p.cols); }}'
+                                                for s, r in ((1, 300), (32, 331))])
+    assert alone == 1602 and beside == 802
