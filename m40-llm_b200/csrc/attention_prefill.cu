@@ -411,7 +411,7 @@ int m40_attention_prefill(M40llmCudaContext* ctx, const M40PrefillCall& c) {
         M40PrefillTcArgs ta = {};
         ta.c = c;
         ta.status = ctx->d_status;
-        ta.tiles = cost.tc_tiles();
+        ta.two_tiles = cost.tc_two() ? 1u : 0u;
         const int rc = m40_attention_prefill_tc(ctx, ctx->decode_stream, ta, (uint64_t)c.slots * c.kv_heads * c.max_seq_len);
         if (rc <= 0) return rc;
     }
@@ -538,7 +538,7 @@ int m40llm_attention_prefill_f32_gqa_varlen_async(M40llmCudaContext* ctx, const 
     ta.q_lens = d_q_lens;
     ta.kv_lens = d_kv_lens;
     ta.status = ctx->d_status;
-    ta.tiles = cost.tc_tiles();
+    ta.two_tiles = cost.tc_two() ? 1u : 0u;
     rc = cost.tc_us() < cost.mma_us() ? m40_attention_prefill_tc(ctx, s, ta, total_kv) : 1;
     if (rc <= 0) return rc;
     dim3 grid((max_q + PF_TILE - 1) / PF_TILE, q_heads, batch_size);

@@ -468,9 +468,8 @@ int m40_attention_prefill_tc(M40llmCudaContext* ctx, cudaStream_t s, const M40Pr
     CUtensorMap mk, mv;
     const uint64_t cols = cache ? c.hd : (uint64_t)c.kv_heads * c.hd;
     if (!m40_tc_map(&mk, c.K, kv_rows, cols, KEYS, false) || !m40_tc_map(&mv, c.V, kv_rows, cols, KEYS, false)) return 1;
-    // Two row tiles per CTA where one each would not find an SM for every CTA at once.
     a.pair_heads = c.q_heads / c.kv_heads % 2 == 0 ? 1u : 0u;
-    const bool two = a.tiles > (double)ctx->sm_count;
+    const bool two = a.two_tiles != 0u;
     if (c.hd == 128)
         return cache ? (two ? launch<128, true, 2>(ctx, s, mk, mv, a) : launch<128, true, 1>(ctx, s, mk, mv, a))
                      : (two ? launch<128, false, 2>(ctx, s, mk, mv, a) : launch<128, false, 1>(ctx, s, mk, mv, a));

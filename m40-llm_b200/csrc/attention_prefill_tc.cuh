@@ -10,7 +10,7 @@ struct M40PrefillTcArgs {
     const uint32_t* q_lens;
     const uint32_t* kv_lens;
     uint32_t* status;
-    double tiles;         // tiles of 128 rows of one head that have rows: what the form is chosen by
+    uint32_t two_tiles;   // two tiles of 128 rows per CTA (prompt_cost.cuh)
     uint32_t pair_heads;  // filled in by the launch
 };
 // kv_rows: rows of the K and V arrays (cache: slots * kv_heads * max_seq_len). 0 when launched, 1 for a call it does not take,

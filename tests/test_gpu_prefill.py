@@ -5,6 +5,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
+import two_tiles
 from helpers import assert_close
 
 pytestmark = pytest.mark.gpu
@@ -61,6 +62,13 @@ def test_prefill_shapes(nat, O, qh, kvh, hd, pairs):
 ])
 def test_prefill_two_row_tiles(nat, O, qh, kvh, hd, pairs):
     """More row tiles than SMs: a CTA works on two of them."""
+    got, exp = run_prefill(nat, O, qh, kvh, hd, pairs, qh + hd)
+    assert_close(got, exp, what=f"prefill {qh}/{kvh} d{hd} {pairs}")
+    nat.free_all()
+
+
+@pytest.mark.parametrize("qh,kvh,hd,pairs", two_tiles.PACKED)
+def test_prefill_of_long_prompts_two_row_tiles(nat, O, qh, kvh, hd, pairs):
     got, exp = run_prefill(nat, O, qh, kvh, hd, pairs, qh + hd)
     assert_close(got, exp, what=f"prefill {qh}/{kvh} d{hd} {pairs}")
     nat.free_all()
@@ -282,6 +290,66 @@ def test_packed_values_beyond_f16_stay_with_the_rows_that_see_them(nat, hd, pos,
         out.append(do.download(np.float32, q.shape))
     assert np.array_equal(out[1][rows:], out[0][rows:])
     check_poisoned(out[1][:rows], out[0][:rows], seen, pos, qh // kvh)
+    nat.free_all()
+
+
+def over_cache(nat, pkg, kv, slot, q, pos, shift=0):
+    """Rows over a cache's slot; with `shift` 2 the queries lie on 8 bytes only, which the mma.sync kernel serves."""
+    rows, qh, _ = q.shape
+    dq, do = nat.buf(np.concatenate([np.zeros(shift, np.float32), q.ravel()])), nat.buf(np.full(q.shape, 9.0, np.float32))
+    r = pkg.native.StepRows(rows=rows, segments=1, max_segment_rows=rows, max_len=pos + rows, slot_mul=1, slot_add=0,
+                            seg=nat.buf(np.array([0, rows, slot, pos], np.uint32)).ptr)
+    assert nat.lib.m40llm_attention_step_rows_async(nat.ctx, kv, dq.ptr + 4 * shift, qh, C.byref(r), do.ptr) == 0
+    nat.sync(1)
+    return do.download(np.float32, q.shape)
+
+
+@pytest.mark.parametrize("qh,kvh,hd,pos,rows", two_tiles.CACHED)
+@pytest.mark.parametrize("scale", [1.0, 6.0])
+def test_two_row_tiles_over_cache(nat, pkg, qh, kvh, hd, pos, rows, scale):
+    """As test_step_rows_over_cache and test_prompt_forms_are_equally_exact, with two row tiles per CTA."""
+    rng = np.random.default_rng(hd + rows)
+    L = pos + rows
+    kv = nat.kv_dense(L + 7, 2, kvh, hd)
+    K, V = (rng.standard_normal((L, kvh, hd)).astype(np.float16) for _ in range(2))
+    nat.kv_fill(kv, 1, K, V)
+    q = (scale * rng.standard_normal((rows, qh, hd))).astype(np.float32)
+    want = np.empty(q.shape)
+    unseen = np.arange(L)[None, :] > (pos + np.arange(rows))[:, None]
+    for h in range(qh):
+        s = q[:, h].astype(np.float64) @ K[:, h // (qh // kvh)].astype(np.float64).T / np.sqrt(hd)
+        s[unseen] = -np.inf
+        p = np.exp(s - s.max(1, keepdims=True))
+        want[:, h] = (p / p.sum(1, keepdims=True)) @ V[:, h // (qh // kvh)].astype(np.float64)
+    two, plain = (over_cache(nat, pkg, kv, 1, q, pos, shift) for shift in (0, 2))
+    assert np.abs(two - want).max() <= 2.0 ** -11 * float(np.abs(V).max()) + 1e-4
+    error = [np.linalg.norm(x - want) / np.linalg.norm(want) for x in (two, plain)]
+    assert error[0] <= 1.1 * error[1] and error[1] <= 2.0 ** -11, error
+    nat.lib.m40llm_kvcache_destroy(kv)
+    nat.free_all()
+
+
+@pytest.mark.parametrize("qh,kvh,hd,pos,rows", two_tiles.CACHED)
+@pytest.mark.parametrize("at", [3, 1000, 1290])
+def test_two_row_tiles_keep_values_that_are_not_finite_with_the_rows_that_see_them(nat, pkg, qh, kvh, hd, pos, rows, at):
+    """Tokens in the first, a middle and one of the last tiles: where a CTA's tiles are rows that follow one another, the first of them walks
+    keys that only the second one sees."""
+    rng = np.random.default_rng(rows + at)
+    L = pos + rows
+    K = rng.standard_normal((L, kvh, hd)).astype(np.float16)
+    clean, bad, seen = poisoned(rng, L, kvh, hd, pos + at)
+    q = rng.standard_normal((rows, qh, hd)).astype(np.float32)
+    out = []
+    for values, around in ((clean, 0.0), (clean, np.nan), (bad, np.inf)):
+        kv = nat.kv_dense(L + 150, 3, kvh, hd)
+        junk = np.full((L + 150, kvh, hd), around, np.float16)
+        for slot in range(3):
+            nat.kv_fill(kv, slot, junk, junk)
+        nat.kv_fill(kv, 1, K, values)
+        out.append(over_cache(nat, pkg, kv, 1, q, pos))
+        nat.lib.m40llm_kvcache_destroy(kv)
+    assert np.isfinite(out[0]).all() and np.array_equal(out[0], out[1])
+    check_poisoned(out[2], out[0], seen, pos, qh // kvh)
     nat.free_all()
 
 

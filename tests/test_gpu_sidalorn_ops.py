@@ -227,6 +227,19 @@ def test_latent_attention(nat, H, D, V, R, fp32):
     t.close()
 
 
+@pytest.mark.parametrize("sink", [True, False])
+@pytest.mark.parametrize("V", [64, 40])
+def test_latent_attention_of_a_long_prompt(nat, V, sink):
+    """Every head has keys and values of its own: two tiles of rows that follow one another per CTA, with and without a sink."""
+    H, D, R, T = 40, 64, 64, 1410
+    t = Latent(nat, H, D, V, R, 0, sink=sink, seed=V, max_len=T)
+    rng = np.random.default_rng(2)
+    q, c = rng.standard_normal((T, H * D)).astype(np.float32), rng.standard_normal((T, R)).astype(np.float32)
+    close(t.run([(0, 0, T)], q, c, max_len=T), t.oracle(q, c), 3e-3)
+    no_status(nat)
+    t.close()
+
+
 @pytest.mark.parametrize("fp32", [0, 1])
 @pytest.mark.parametrize("H,D,V,R", [(4, 64, 64, 128), (2, 128, 128, 512), (3, 40, 24, 56)])
 def test_latent_attention_finds_one_far_token(nat, H, D, V, R, fp32):

@@ -5,6 +5,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
+import two_tiles
 from helpers import load_package
 
 load_package()
@@ -369,6 +370,14 @@ def test_attention_optional_parts(nat, norms, turn, gate, D, V, f32):
     rng = np.random.default_rng(2)
     for segs in ([(0, 0, 33)], [(0, 33, 1)], [(1, 0, 5), (0, 34, 90)]):
         a.both(rng.standard_normal((sum(s[2] for s in segs), a.width())).astype(np.float32), segs, 3e-6 if f32 else 3e-3, str(segs))
+    a.close()
+
+
+@pytest.mark.parametrize("H,G,D,V,rows", two_tiles.STACKS)
+def test_attention_of_long_prompts_two_row_tiles(nat, H, G, D, V, rows):
+    """Norms, turned values, gate and padded value sizes in a prompt that takes two row tiles per CTA."""
+    a = Attn(nat, H, G, D, V, 32, 0, seed=H, max_len=rows, scaling=YARN)
+    a.both(np.random.default_rng(rows).standard_normal((rows, a.width())).astype(np.float32), [(1, 0, rows)], 3e-3, "prompt")
     a.close()
 
 

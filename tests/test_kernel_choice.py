@@ -6,6 +6,7 @@ import subprocess
 import pytest
 
 import helpers
+import two_tiles
 
 CSRC = os.path.join(helpers.PKG_DIR, "csrc")
 
@@ -52,6 +53,50 @@ def test_prompt_kernels_are_chosen_as_measured(ask):
     got = ask("prompt_cost.cuh", [cost(i, *p[:4]) + f' printf("%d\\n", c{i}.tc_us() < c{i}.mma_us());' for i, p in enumerate(PROMPTS)])
     for p, tc in zip(PROMPTS, got):
         assert (p[4] if tc else p[5]) <= min(1.05 * p[5], 1.25 * p[4]), p
+
+
+# the same, us of the tcgen05 kernel with one and with two row tiles per CTA
+ROW_TILES = [
+    (128, 32, 8, [(640, 0, 1)], 18.3, 26.0),
+    (128, 32, 8, [(1000, 0, 1)], 27.3, 35.4),
+    (128, 32, 8, [(1300, 0, 1)], 44.8, 43.2),
+    (128, 32, 8, [(2048, 0, 1)], 76.0, 68.3),
+    (128, 32, 8, [(640, 1000, 1)], 42.3, 52.2),
+    (128, 32, 8, [(1000, 4000, 1)], 121.8, 137.4),
+    (128, 32, 8, [(500, 0, 4)], 44.7, 36.6),
+    (128, 32, 8, [(700, 0, 3)], 52.4, 44.5),
+    (128, 16, 2, [(1300, 0, 1)], 23.5, 41.8),
+    (128, 16, 2, [(2048, 0, 1)], 37.3, 60.7),
+    (128, 16, 2, [(1024, 0, 4)], 54.4, 46.3),
+    (128, 16, 2, [(1500, 0, 1), (200, 0, 1), (300, 0, 1)], 32.8, 46.6),
+    (64, 32, 4, [(1000, 0, 1)], 22.0, 27.8),
+    (64, 32, 4, [(2048, 0, 1)], 60.7, 53.0),
+    (64, 32, 4, [(1000, 4000, 1)], 104.0, 112.2),
+    (64, 32, 4, [(500, 0, 4)], 34.0, 26.3),
+    (64, 40, 40, [(820, 0, 1)], 21.8, 25.9),
+    (64, 40, 40, [(1500, 0, 1)], 49.5, 46.4),
+    (64, 40, 40, [(1000, 4000, 1)], 154.7, 191.7),
+    (64, 40, 40, [(65, 2000, 16)], 140.0, 250.3),
+    (64, 40, 40, [(1024, 0, 4)], 105.1, 97.5),
+    (128, 33, 11, [(2048, 0, 1)], 78.4, 77.6),
+    (128, 33, 11, [(65, 2000, 16)], 132.4, 239.2),
+    (128, 33, 11, [(1000, 0, 1)], 28.2, 37.7),
+    (128, 8, 2, [(1024, 0, 4)], 27.4, 35.8),
+]
+
+
+def test_row_tiles_per_cta_are_chosen_as_measured(ask):
+    got = ask("prompt_cost.cuh", [cost(i, *p[:4]) + f' printf("%d\\n", c{i}.tc_two());' for i, p in enumerate(ROW_TILES)])
+    for p, two in zip(ROW_TILES, got):
+        assert (p[5] if two else p[4]) <= 1.05 * min(p[4:]), p
+    assert sum(got) >= 8
+
+
+def test_calls_that_test_two_row_tiles_have_them(ask):
+    cases = [(hd, qh, kvh, [(q, kv - q, 1) for q, kv in pairs]) for qh, kvh, hd, pairs in two_tiles.PACKED]
+    cases += [(hd, qh, kvh, [(rows, pos, 1)]) for qh, kvh, hd, pos, rows in two_tiles.CACHED]
+    cases += [(64 if max(d, v) <= 64 else 128, h, g, [(rows, 0, 1)]) for h, g, d, v, rows in two_tiles.STACKS]
+    assert all(ask("prompt_cost.cuh", [cost(i, *p) + f' printf("%d\\n", c{i}.tc_two() && c{i}.tc_us() < c{i}.mma_us());' for i, p in enumerate(cases)]))
 
 
 # the same, us of the faster prompt kernel and of the decode form (a row reads its own context)
