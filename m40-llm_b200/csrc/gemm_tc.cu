@@ -21,6 +21,8 @@
 // CTA stops issuing work, frees its TMEM and returns.
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_tc_pair.cuh"
@@ -310,8 +312,10 @@ __global__ void __launch_bounds__(256) norm_split_rows_kernel(const float* __res
         split_store4(*reinterpret_cast<const float4*>(xr + k), norm_w4(w, w_f32, k), scale, hr + k, lr + k);
 }
 
-// Rows of any pitch -> hi / lo copies of type T, with an RMS or polynomial norm. One CTA per row; few rows get wide CTAs, since what counts
-// there is how long one row takes (5632 columns, polynomial norm, 256 threads: 6 us in a chain of 32-row calls).
+// Rows of any pitch -> hi / lo copies of type T, with an RMS or polynomial norm. One CTA per row. Where two CTAs of 1024 threads per SM hold
+// all rows they are as wide as that (WIDE), since what counts there is how long one row takes (5632 columns, polynomial norm, 256 threads:
+// 6 us in a chain of 32-row calls; the call of 129 rows of 14336 columns into 4096 outputs 59 us, wide 49). 256 threads for more rows; with
+// the block's width a run-time value for both, those took up to 8 % longer.
 template <typename T>
 __device__ __forceinline__ T to_half_type(float v);
 template <>
@@ -329,10 +333,23 @@ struct SplitRowsArgs {
     int w_f32;  // RMS weights: as in norm_split_rows_kernel
     float eps, alpha;
 };
-template <typename T>
-__global__ void __launch_bounds__(1024) split_rows_kernel(SplitRowsArgs a, T* __restrict__ hi, T* __restrict__ lo) {
+// The warps' sums added up by every thread: eight of them one behind the other, up to 32 over the lanes.
+template <bool WIDE>
+__device__ __forceinline__ float sum_of_warps(const float* red, uint32_t warps) {
+    float t = 0.0f;
+    if constexpr (WIDE) {
+        const uint32_t lane = threadIdx.x & 31u;
+        t = warp_sum(lane < warps ? red[lane] : 0.0f);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) t += red[i];
+    }
+    return t;
+}
+template <typename T, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? 1024 : 256) split_rows_kernel(SplitRowsArgs a, T* __restrict__ hi, T* __restrict__ lo) {
     __shared__ float red[32], red2[32], red3[32];
-    const uint32_t stride = blockDim.x * 4u, warps = blockDim.x / 32u;
+    const uint32_t threads = WIDE ? blockDim.x : 256u, stride = threads * 4u, warps = threads / 32u;
     pdl_wait();
     pdl_trigger();
     const float* xr = a.x + (size_t)blockIdx.x * a.ldx;
@@ -348,8 +365,7 @@ __global__ void __launch_bounds__(1024) split_rows_kernel(SplitRowsArgs a, T* __
         ss = warp_sum(ss);
         if ((threadIdx.x & 31u) == 0u) red[threadIdx.x >> 5] = ss;
         __syncthreads();
-        float tot = 0.0f;
-        for (uint32_t i = 0; i < warps; ++i) tot += red[i];
+        const float tot = sum_of_warps<WIDE>(red, warps);
         scale = rsqrtf(tot / (float)a.K + a.eps);
     }
     const float* wf = reinterpret_cast<const float*>(a.w);
@@ -368,8 +384,7 @@ __global__ void __launch_bounds__(1024) split_rows_kernel(SplitRowsArgs a, T* __
         s1 = warp_sum(s1), s2 = warp_sum(s2), s3 = warp_sum(s3);
         if ((threadIdx.x & 31u) == 0u) red[threadIdx.x >> 5] = s1, red2[threadIdx.x >> 5] = s2, red3[threadIdx.x >> 5] = s3;
         __syncthreads();
-        s1 = s2 = s3 = 0.0f;
-        for (uint32_t i = 0; i < warps; ++i) s1 += red[i], s2 += red2[i], s3 += red3[i];
+        s1 = sum_of_warps<WIDE>(red, warps), s2 = sum_of_warps<WIDE>(red2, warps), s3 = sum_of_warps<WIDE>(red3, warps);
         poly = m40_poly_scales(wf, s1, s2, s3, (float)a.K, a.eps);
     }
     for (uint32_t k = threadIdx.x * 4u; k < a.K; k += stride) {
@@ -591,10 +606,13 @@ int split_rows(M40llmCudaContext* ctx, cudaStream_t s, const float* X, int M, in
         es = ext->bf16 ? m40_launch_dependent(split_columns_kernel<__nv_bfloat16>, grid, dim3(256), 0, s, sa, (__nv_bfloat16*)xh, (__nv_bfloat16*)xl)
                        : m40_launch_dependent(split_columns_kernel<__half>, grid, dim3(256), 0, s, sa, xh, xl);
     } else {
-        const unsigned quads = ((unsigned)K / 4 + 31) / 32 * 32, threads = M <= 128 && quads > 256 ? (quads < 1024 ? quads : 1024) : 256;
-        es = ext->bf16 ? m40_launch_dependent(split_rows_kernel<__nv_bfloat16>, dim3((unsigned)M), dim3(threads), 0, s, sa, (__nv_bfloat16*)xh,
-                                              (__nv_bfloat16*)xl)
-                       : m40_launch_dependent(split_rows_kernel<__half>, dim3((unsigned)M), dim3(threads), 0, s, sa, xh, xl);
+        const unsigned quads = ((unsigned)K / 4 + 31) / 32 * 32, wide = M <= 2 * ctx->sm_count && quads > 256 ? (quads < 1024 ? quads : 1024) : 0;
+        const auto launch = [&](auto* h, auto* l) {
+            using T = std::remove_pointer_t<decltype(h)>;
+            return wide ? m40_launch_dependent(split_rows_kernel<T, true>, dim3((unsigned)M), dim3(wide), 0, s, sa, h, l)
+                        : m40_launch_dependent(split_rows_kernel<T, false>, dim3((unsigned)M), dim3(256), 0, s, sa, h, l);
+        };
+        es = ext->bf16 ? launch((__nv_bfloat16*)xh, (__nv_bfloat16*)xl) : launch(xh, xl);
     }
     M40_COUNT_LAUNCH(ctx);
     return es == cudaSuccess ? 0 : -2;

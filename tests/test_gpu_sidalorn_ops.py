@@ -77,6 +77,18 @@ def test_norms_around_a_projection(nat, rows, n, k, groups, exact):
     close(t.run(z, w, rows, pre=t.norm(N.NORM_ACT, act=N.ACT_GELU_ERF), exact=exact), y, tol, "activation before")
 
 
+@pytest.mark.parametrize("rows", [2, 33, 128, 129, 296, 297])
+@pytest.mark.parametrize("k", [1024, 1032, 2200, 5000])
+def test_norms_of_wide_rows(nat, rows, k):
+    """Blocks of 256 threads, of as many as there are fours of columns and of 1024, over rows that are whole trips and not."""
+    rng = np.random.default_rng(rows + k)
+    t = Norms(nat)
+    x, w = rng.standard_normal((rows, k)).astype(np.float32), rounded(rng, N.DT_BF16, 40, k)
+    g, c = 1 + 0.3 * rng.standard_normal(k), np.array([0.5, 0.7, -0.3, 0.2], np.float32)
+    close(t.run(x, w, rows, pre=t.norm(N.NORM_RMS, 1e-4, g)), S.rms_norm(x, g, 1e-4) @ w.T.astype(np.float64), 6e-5, "rms")
+    close(t.run(x, w, rows, pre=t.norm(N.NORM_POLY, 1e-4, c)), S.poly_norm(x, c, 1e-4) @ w.T.astype(np.float64), 1.8e-4, "poly")
+
+
 def n_parts(k, groups):
     return groups if k % groups == 0 else 1
 
