@@ -332,6 +332,7 @@ struct SplitRowsArgs {
     int act;    // M40LLM_NORM_ACT
     int w_f32;  // RMS weights: as in norm_split_rows_kernel
     float eps, alpha;
+    int late;  // split_columns_kernel: the projection may start once this kernel's own wait is over
 };
 // The warps' sums added up by every thread: eight of them one behind the other, up to 32 over the lanes.
 template <bool WIDE>
@@ -412,12 +413,13 @@ __global__ void __launch_bounds__(WIDE ? 1024 : 256) split_rows_kernel(SplitRows
 // (16 x 4096 with a dynamic tanh: 6.4 us with a CTA per row).
 template <typename T>
 __global__ void __launch_bounds__(256) split_columns_kernel(SplitRowsArgs a, T* __restrict__ hi, T* __restrict__ lo) {
-    pdl_trigger();
+    if (!a.late) pdl_trigger();
     const uint32_t k = (blockIdx.y * 256u + threadIdx.x) * 4u, kk = k < a.K ? k : 0u;
     const float* wf = reinterpret_cast<const float*>(a.w);
     float4 w = make_float4(1.f, 1.f, 1.f, 1.f), b = make_float4(0.f, 0.f, 0.f, 0.f);
     if (a.kind == (int)M40LLM_NORM_DYT) w = m40_vec4_or(wf, kk, 1.0f), b = m40_vec4_or(a.b, kk, 0.0f);
     pdl_wait();
+    if (a.late) pdl_trigger();
     const float4 v = *reinterpret_cast<const float4*>(a.x + (size_t)blockIdx.x * a.ldx + kk);
     float y[4] = {v.x, v.y, v.z, v.w};
     if (a.kind == (int)M40LLM_NORM_DYT) {
@@ -601,6 +603,10 @@ int split_rows(M40llmCudaContext* ctx, cudaStream_t s, const float* X, int M, in
         sa.w_f32 = (norm->w_is_f32 ? 1 : 0) | (w_vec ? 0 : 2);
     }
     cudaError_t es;
+    // A projection that starts before this kernel's wait is over asks for its first weights earlier, but its blocks take room beside the call
+    // before, too. It pays but for short sums of 64 rows on, up to where the call is long: 129 x 1024 into 2048: 12.6 us early, 11.4 late;
+    // 64 x 2048: 9.9 and 9.6; 64 x 1024: 8.6 and 8.85, 33 x 5632 11.4 and 12.7, 256 x 2048: 14.1 and 14.4.
+    sa.late = K <= 2048 && (size_t)M * K >= 128 * 1024 && M < 256 ? 1 : 0;
     if (sa.kind != (int)M40LLM_NORM_RMS && sa.kind != (int)M40LLM_NORM_POLY) {
         const dim3 grid((unsigned)M, ((unsigned)K + 1023) / 1024);
         es = ext->bf16 ? m40_launch_dependent(split_columns_kernel<__nv_bfloat16>, grid, dim3(256), 0, s, sa, (__nv_bfloat16*)xh, (__nv_bfloat16*)xl)
