@@ -105,6 +105,24 @@ def test_prompt_portions_match_single_tokens(nat, O, pkg, hd, parts):
     nat.free_all()
 
 
+@pytest.mark.parametrize("n", [1, 2, 1023, 1024, 1025, 4096, 4097, 5120, 16384, 16385, 20480, 20481, 32000, 49153])
+def test_argmax_of_every_length(nat, n):
+    """Lengths between which a thread's loads are grouped differently: the largest value at the start, at the end and twice, none that counts."""
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((6, n)).astype(np.float32)
+    first = [0, n - 1, min(n - 1, n // 2), min(n - 1, 3 * n // 4), 0, 0]
+    for r, i in enumerate(first[:4]):
+        x[r, i] = 9.0
+    x[2, n - 1] = x[3, n - 1] = 9.0
+    x[3, :first[3]] = np.nan
+    x[4], x[5] = np.nan, -np.inf
+    out = nat.buf(6 * 4)
+    assert nat.lib.m40llm_argmax_f32_async(nat.ctx, nat.buf(x).ptr, 6, n, out.ptr) == 0
+    nat.sync(1)
+    assert out.download(np.uint32, 6).tolist() == first
+    nat.free_all()
+
+
 def test_argmax_and_embedding_rules(nat):
     L = nat.lib
     x = np.array([[1.0, 5.0, 5.0, np.nan, -np.inf], [np.nan, np.nan, np.nan, np.nan, np.nan],
