@@ -291,8 +291,11 @@ int run_rows(M40llmCudaContext* ctx, RgArgs g, uint32_t blocks, const M40llmStep
         q.N = q.K = q.group_k = g.bs;
         q.x_rows = g.rows;
         q.ldx = g.width;
-        // Steps: 16, since a row's step takes longer than its products (32 rows, width 1024: 8.0 us; tiles of 32, fetched row by row, 15.9).
-        q.tile_rows = g.step ? 16 : 32;
+        // Steps: 16, since a row's step takes longer than its products (32 rows, width 1024: 8.0 us; tiles of 32, fetched row by row, 15.9). 32
+        // where tiles of 16 would not all be there at once, three to an SM, and those are (256 rows of width 2560 21.3 us, with 16 22.7; 128 of
+        // width 4096 18.5 and 20.7; but 256 of width 4096 35.0 and 33.3).
+        const uint64_t columns = (uint64_t)((g.bs + 63) / 64) * blocks, most = 3u * (uint64_t)ctx->sm_count;
+        q.tile_rows = g.step && (columns * ((g.rows + 15) / 16) <= most || columns * ((g.rows + 31) / 32) > most) ? 16 : 32;
         q.kind = M40_GROUPED_RG;
         q.rg = g;
         if ((rc = m40_gemm_tc_grouped(ctx, s, q)) != 0) return rc;

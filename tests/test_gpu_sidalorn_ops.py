@@ -391,10 +391,12 @@ def test_rglru(nat, W, B, taps, exact):
     nat.free_all()
 
 
-@pytest.mark.parametrize("n,W,B", [(8, 576, 4), (9, 576, 4), (16, 576, 4), (17, 576, 4), (33, 576, 4), (17, 1024, 1), (5, 968, 1)])
+@pytest.mark.parametrize("n,W,B", [(8, 576, 4), (9, 576, 4), (16, 576, 4), (17, 576, 4), (33, 576, 4), (17, 1024, 1), (5, 968, 1), (250, 1280, 20), (370, 1280, 20),
+                                   (730, 1280, 20)])
 def test_rglru_steps_of_many_sequences(nat, n, W, B):
     """A step's tiles hold 16 rows, eight to a thread: full and ragged ones, the first token of a sequence among later ones; products with
-    fewer blocks of K than the ring of a block that has its SM to itself, and with more."""
+    fewer blocks of K than the ring of a block that has its SM to itself, and with more. The last three have more tiles than two per SM, tiles
+    of 32 rows, and more of either than three per SM."""
     taps, T = 4, 4
     rng = np.random.default_rng(n)
     D = W // B
