@@ -642,7 +642,12 @@ bool splits_inside(const float* X, int M, int K, const M40GemvNorm* norm, const 
 int gemm_rows(M40llmCudaContext* ctx, cudaStream_t s, uint32_t stream_kind, const float* X, int M, int K, int problems, const __half* const* W,
               const int* N, float* const* out, const float* const* bias, const float* const* residual, int mode, const M40GemvNorm* norm,
               const M40TcRopeAppend* rope, const M40TcExt* ext) {
-    const bool bf16 = ext && ext->bf16, inside = splits_inside(X, M, K, norm, ext, problems, N, out, mode);
+    // With more tiles than SMs K has no splits, and every CTA would split all of x: from 17 rows on that takes longer than its weights (32000 x
+    // 2048, 17 and 32 rows: 26.1 and 29.0 us, with x split beforehand 24.4 and 26.1; gate | up of 2 x 14336 x 4096 43.4 and 47.2, 41.6 and 42.5).
+    int tiles = 0;
+    for (int p = 0; p < (mode == 1 ? 1 : problems); ++p) tiles += mode == 1 ? (N[p] + BLOCK_N / 2 - 1) / (BLOCK_N / 2) : (N[p] + BLOCK_N - 1) / BLOCK_N;
+    const bool bf16 = ext && ext->bf16, long_split = M > 16 && tiles > ctx->sm_count;
+    const bool inside = !long_split && splits_inside(X, M, K, norm, ext, problems, N, out, mode);
     M40RowsArgs a = {};
     a.M = (uint32_t)M;
     a.K = (uint32_t)K;

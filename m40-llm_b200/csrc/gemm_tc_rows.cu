@@ -20,8 +20,8 @@
 // At this few rows a call is a chain of latencies beside a stream of weights, and the split, the sums and the epilogue as launches of
 // their own cost more than their work: 16 rows of 4096 x 4096 took 12.8 us with them and take 8.8, 4096 x 14336 32.5 and 22.0, 32 rows of
 // 2048 x 2048 9.2 and 6.2. A norm or activation of x is not applied here: every tile's CTA would do it again (a dynamic tanh of
-// 16 x 4096 values in each of 224 CTAs: 87 us against 39 with a split kernel); calls with one and calls whose result lies over x come split
-// already (M40_ROWS_SPLIT).
+// 16 x 4096 values in each of 224 CTAs: 87 us against 39 with a split kernel); calls with one, calls whose result lies over x and calls of more
+// than 16 rows with more tiles than SMs come split already (M40_ROWS_SPLIT).
 //
 // Every wait is bounded: a wait that runs out raises status bit 4; all threads still meet at the barriers, copies in flight land
 // (bounded) and tensor memory is freed.
