@@ -55,19 +55,43 @@ def test_unbounded_barriers_do_not_hang_on_a_wait_that_ran_out():
     assert "a.status" not in pair[:pair.rindex("__syncthreads();")]
 
 
+def expression(text):
+    """A C expression of unsigned names and numbers as a Python one."""
+    return re.sub(r"\b(\d+)u\b", r"\1", text).replace("a.stages", "stages").replace("/", "//").replace("&&", "and")
+
+
+def statements(text):
+    """Comma-separated C assignments and increments as Python ones."""
+    return [re.sub(r"\+\+(\w+)", r"\1 += 1", re.sub(r"^uint32_t ", "", expression(part.strip()))) for part in text.split(",")]
+
+
 def test_ring_of_the_few_rows_kernel():
-    """Four warps write every fourth k-block of the activation operand and wait by parity for the stage's last use only. Any order in
-    which they and the issuing warp may run, on every ring that the launch allows: no stage is overwritten early, none waits for good."""
+    """Four warps write every fourth k-block of the activation operand and wait by parity for the stage's last use only. The first stage, the
+    parity waited for and the way on are taken from the kernel. Any order in which the warps and the issuing one may run, on every ring that the
+    launch allows: no stage is overwritten early, none waits for good."""
     source = plain(os.path.join(CSRC, "gemm_tc_rows.cu"))
     low, high = (int(re.search(rf"{n} = (\d+)", source).group(1)) for n in ("MIN_STAGES", "MAX_STAGES"))
     assert "a.stages < MIN_STAGES" in source
+    maker = source[source.index("void make_operand("):source.index("gemm_tc_rows_kernel(")]
+    start = statements(re.search(r"(uint32_t s = [^;]*, round = [^;]*);", maker).group(1))
+    waits, parity = re.search(r"if \(half == 0 && (.*?)\) ok = __all_sync\(0xffffffffu, !\*abort_flag && mbar_wait\(&empty\[s\], (.*?)\)\);", maker).groups()
+    step, wraps, wrap = re.search(r"if \(lane == 0\) mbar_arrive\(&x_full\[s\]\);\s*(s \+= [^;]*);\s*if \((.*?)\) (s -= [^;]*);", maker).groups()
+    # the k-block that is converted at stage s of the round is w + 4 i: as the columns are fetched and the trips counted
+    assert "(kb0 + w + t / UNITS * 4u) * BLOCK_K" in maker and "(n_kb - w + 3u) / 4u * UNITS" in maker
+    issuer = source[source.index("} else if (warp == 1) {"):]
+    assert re.search(r"uint32_t s = 0, phase = 0;", issuer) and "mbar_wait(&x_full[s], phase)" in issuer
+    assert re.search(r"if \(\+\+s == a\.stages\) s = 0, phase \^= 1u;", issuer)
 
     def run(stages, blocks, rng):
         freed, filled, holds, done = [0] * stages, [0] * stages, {}, 0
+        makers = [{"w": w, "stages": stages} for w in range(4)]
+        for m in makers:
+            for line in start:
+                exec(line, {}, m)
         at = list(range(4))  # each warp's next k-block
         while done < blocks:
-            ready = [w for w in range(4) if at[w] < blocks and
-                     (at[w] < stages or freed[at[w] % stages] % 2 != (at[w] // stages - 1) % 2)]
+            ready = [w for w, m in enumerate(makers) if at[w] < blocks and
+                     (not eval(expression(waits), {}, m) or freed[m["s"]] % 2 != eval(expression(parity), {}, m))]
             if filled[done % stages] % 2 != done // stages % 2:
                 ready.append(4)
             assert ready, (stages, blocks, done)
@@ -77,10 +101,15 @@ def test_ring_of_the_few_rows_kernel():
                 freed[done % stages] += 1
                 done += 1
             else:
-                assert at[w] - stages < done
-                holds[at[w] % stages] = at[w]
-                filled[at[w] % stages] += 1
+                m = makers[w]
+                assert at[w] - stages < done and m["s"] == at[w] % stages
+                holds[m["s"]] = at[w]
+                filled[m["s"]] += 1
                 at[w] += 4
+                exec(expression(step), {}, m)
+                if eval(expression(wraps), {}, m):
+                    for line in statements(wrap):
+                        exec(line, {}, m)
 
     rng = random.Random(1)
     for stages in range(low, high + 1):
