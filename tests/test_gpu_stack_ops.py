@@ -527,6 +527,25 @@ def test_delta_rule_prompt_equals_tokens_and_slot_reuse(nat):
     d.close()
 
 
+@pytest.mark.parametrize("H,D", [(3, 40), (40, 64), (4, 128)])
+def test_delta_rule_cuts_and_company_change_the_rounding_only(nat, H, D):
+    """Tokens go in pairs from a portion's first one on, and what else a step holds may choose another form: the sums of a token are the same
+    terms in another order."""
+    d = Delta(nat, H, D, 4, seed=7)
+    rng = np.random.default_rng(8)
+    packed = rng.standard_normal((131, d.width())).astype(np.float32)
+    whole, state = d.device(packed, [(0, 0, 131)]), d.state(0)
+    for cuts in ([2], [16, 64], [1], [15, 16, 33], [64, 65, 128]):
+        parts = [d.device(packed[a:b], [(1, a, b - a)]) for a, b in zip([0] + cuts, cuts + [131])]
+        close(np.concatenate(parts), whole, 4e-6, f"cut at {cuts}")
+        close(d.state(1), state, 2e-6, f"state, cut at {cuts}")
+    both = d.device(np.concatenate([packed, packed[:70]]), [(1, 0, 131), (2, 0, 70)])
+    close(both[:131], whole, 4e-6, "beside another prompt")
+    close(both[131:], whole[:70], 4e-6, "the other prompt")
+    close(d.state(1), state, 2e-6, "state, beside another prompt")
+    d.close()
+
+
 def test_delta_rule_long_memory(nat):
     """Slow decay and a removal rate near zero: what the first tokens wrote must still be read a thousand tokens later."""
     d = Delta(nat, 1, 48, 4, seed=8)
