@@ -1,4 +1,5 @@
-// Prompt attention on the 5th-generation tensor cores: CTA = 128 query rows of one (sequence, q head), keys in tiles of 128.
+// Prompt attention on the 5th-generation tensor cores: CTA = one or two tiles of 128 query rows of one sequence and kv head, keys in
+// tiles of 128.
 //
 //   scores   S[128 q rows][128 keys] = Qhi K^T + Qlo K^T   A = queries (f16 hi and lo, shared memory), B = the key tile, K-major;
 //   softmax  thread = query row = accumulator lane, so a row needs no exchange;
@@ -12,11 +13,12 @@
 // but its strongest weight is rounded: 1.05 times that error for flat scores, 3.3 times for peaked ones. Adding up the rounded
 // weights in the rows' registers took 12 us more.)
 //
-// Warps 0..3 are the query rows, warp 4 loads K and V by TMA (two stages each), warp 5 issues the MMAs: S(j + 1) runs while the
-// rows work on S(j). A 128 x 128 tile of HD 128 is 24 MMAs (1600 cycles at the tensor rate) beside 1024 cycles of exponentials per
-// scheduler; one set of rows per SM leaves part of either idle, so that two row tiles share a CTA where there are more tiles than SMs
-// (TILES). Four packed prompts of 509 to 2048 tokens, 32 / 8 heads of 128: 245 us, with one tile 280, against 438 us with mma.sync
-// fragments (attention_prefill.cu), which stay for short segments; 220 since the call no longer copies its lengths back.
+// With one tile warps 0..3 are the query rows, warp 4 loads K and V by TMA (a ring of four tiles, three with two row tiles of 128
+// dimensions), warp 5 issues the MMAs: S(j + 1) runs while the rows work on S(j). With two, warps 0..7 are the rows, which add up their rounded
+// weights themselves: there is no chunk of ones. A 128 x 128 tile of HD 128 is 24 MMAs (1600 cycles at the tensor rate) beside 1024
+// cycles of exponentials per scheduler; one set of rows per SM leaves part of either idle, so that two row tiles share a CTA (TILES) where there are enough CTAs to
+// balance (prompt_cost.cuh). Four packed prompts of 509 to 2048 tokens, 32 / 8 heads of 128: 245 us, with one tile 280, against 438 us with
+// mma.sync fragments (attention_prefill.cu), which stay for short segments; 220 since the call no longer copies its lengths back.
 // Rows behind a sequence's last key are whatever the cache holds there; the issuing warp clears them in the value tile, since
 // zero weights do not cancel a NaN. Values of tokens that only some rows see are dealt with at the end (attend_row()): looking
 // through the one or two tiles in question beforehand, in shared memory or with a warp of its own, cost 8 to 22 us of 273, this 5.

@@ -351,11 +351,10 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) gemm_tc_q80_kernel(const __gri
     } else if (warp == 1 || warp == 3) {
         // ---------------- MMA issuers: one accumulator per tile segment. Warp 1 issues
         // hi against [Xh | Xl] (the two activation tiles are contiguous rows of one operand); the lo.Xh products go
-        // to warp 3 and their own accumulator columns (dual issue) or follow from warp 1 into the first half.
+        // to warp 3 and their own accumulator columns (dual issue) or follow from warp 1 into the second half, to the other small products.
         // The two roles are separate instantiations: with both products under a run-time condition in one loop the
         // compiler predicated them, and a predicated-off tcgen05.mma still costs its ~70-90 cycles in the issue slot.
-        // Converged warps with an elected lane in place of "lane == 0" threads: layer step of 6 rows 143 -> 132 us, of 32 rows
-        // 233 -> 227, of 128 rows 626 -> 612.
+        // Converged warps with an elected lane in place of "lane == 0" threads: layer step of 128 rows, then two passes of 64, 626 -> 612 us.
         Q80Smem sm = {s_raw, raw_full, raw_empty, a_full, done, t_full, t_empty, abort_flag};
         if (!dual_issue(M_PAD)) {
             if (warp == 1) q80_issuer<M_PAD, 0>(a, sm, tmem_base, smem_u32(s_b), u0, u1);
